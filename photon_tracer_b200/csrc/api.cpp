@@ -266,7 +266,7 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     if (!s) return fail(PT_ERR_OUT_OF_MEMORY, "pt_scene_create: out of host memory");
     s->device = device;
     s->sms = sms;
-    const size_t bytes = align256(A.nodes.size() * 4) + align256(A.slots.size() * 4) + align256(A.islots.size() * 4) +
+    const size_t bytes = 2 * align256(A.nodes.size() * 4) + align256(A.slots.size() * 4) + align256(A.islots.size() * 4) +
                          align256(A.large.size() * sizeof(float4)) + align256(A.large_mat.size() * 4) +
                          align256(A.sph.size() * sizeof(PtShadeSphere)) + align256(A.tri.size() * sizeof(PtShadeTri)) +
                          align256(A.inst.size() * sizeof(PtShadeInst)) + align256(A.mat.size() * sizeof(PtMaterial)) +
@@ -298,7 +298,12 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     D.tri_uv = upload(base, off, A.tri_uv, err);
     D.tex = upload(base, off, A.tex, err);
     D.texels = upload(base, off, A.texels, err);
+    D.qnodes = reinterpret_cast<const float4*>(base + off);
+    if (err == cudaSuccess)
+        err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(A.nodes.size() / 32), nullptr);
+    off += align256(A.nodes.size() * 4);
     D.has_textures = A.has_textures;
+    D.words = A.use_bvh && stack_words(A.nodes);
     D.ordered_boxes = ordered_boxes(A.nodes);
     D.stack_pack8 = stack_pack8(A.nodes);
     D.tree_kib = tree_kib(A.nodes, A.slots);
@@ -309,6 +314,7 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     s->rays = reinterpret_cast<unsigned long long*>(base + off);
     off += 256;
     if (err == cudaSuccess) err = cudaMemset(s->status, 0, 3 * 256);
+    if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (err != cudaSuccess) {
         cudaFree(s->arena);

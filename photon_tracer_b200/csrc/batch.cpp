@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "batch.h"
+#include "kernels.h"
 #include "scene_host.hpp"
 
 namespace pt {
@@ -402,7 +403,7 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->total_items = items_total;
     b->out_floats = out_floats;
     all.n_flat_slots = 0;
-    const size_t bytes = align256(all.nodes.size() * 4) + align256(all.slots.size() * 4) + align256(all.islots.size() * 4) +
+    const size_t bytes = 2 * align256(all.nodes.size() * 4) + align256(all.slots.size() * 4) + align256(all.islots.size() * 4) +
                          align256(all.large.size() * sizeof(float4)) + align256(all.large_mat.size() * 4) +
                          align256(all.sph.size() * sizeof(PtShadeSphere)) + align256(all.tri.size() * sizeof(PtShadeTri)) +
                          align256(all.inst.size() * sizeof(PtShadeInst)) + align256(all.mat.size() * sizeof(PtMaterial)) +
@@ -430,7 +431,11 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     D.tri_uv = upload(base, off, all.tri_uv, err);
     D.tex = upload(base, off, all.tex, err);
     D.texels = upload(base, off, all.texels, err);
+    D.qnodes = reinterpret_cast<const float4*>(base + off);
+    if (!err) err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(all.nodes.size() / 32), nullptr);
+    off += align256(all.nodes.size() * 4);
     D.has_textures = all.has_textures;
+    D.words = stack_words(all.nodes);
     D.ordered_boxes = ordered_boxes(all.nodes);
     D.stack_pack8 = stack_pack8(all.nodes);
     D.tree_kib = tree_kib(all.nodes, all.slots);
@@ -448,6 +453,7 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->d_rays = reinterpret_cast<unsigned long long*>(base + off + 512);
     b->d_status = reinterpret_cast<unsigned int*>(base + off + 768);
     if (!err) err = cudaMemset(base + off, 0, 4 * 256);
+    if (!err) err = cudaStreamSynchronize(nullptr);
     if (!err) err = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
     if (!err) err = cudaEventCreate(&b->start_event);
     if (!err) err = cudaEventCreateWithFlags(&b->done_event, cudaEventDisableTiming);

@@ -51,6 +51,9 @@ cudaError_t pt_launch_trace_count(const PtSceneDev& scene, const float* rays, si
 cudaError_t pt_launch_primary_depth(const PtSceneDev& scene, const PtCamDev& cam, int width, int height, float* depth,
                                     cudaStream_t stream);
 
+// Fills qnodes (PtSceneDev) from nodes, n nodes of 128 bytes each.
+cudaError_t pt_build_qnodes(const float4* nodes, float4* qnodes, uint32_t n, cudaStream_t stream);
+
 // Blocks of `threads` threads (and dyn_smem bytes of dynamic shared memory)
 // of kernel fn that fit on one SM at once, from the device's limits and the
 // kernel's registers and static shared memory.

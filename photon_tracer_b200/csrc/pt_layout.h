@@ -115,6 +115,7 @@ PT_HD float pt_triangle_light_power(float lum, float area) {
 // Everything a kernel needs, passed by value.
 struct PtSceneDev {
     const float4* nodes;      // 8 float4 per node
+    const float4* qnodes;     // the same nodes, plane 6 the children's stack words (stream.cuh), plane 7 zero
     const float4* slots;      // 3 float4 per slot
     const float4* islots;     // 4 float4 per instance slot
     const float4* large;      // center, radius
@@ -144,5 +145,6 @@ struct PtSceneDev {
     int ordered_boxes;        // every node child box has lo <= hi on each axis (no NaN)
     int stack_pack8;          // every leaf holds <= 15 entries from below slot 2^26 and every
                               // node index is below 2^31: flat-tree stack entries fit 8 bytes
+    int words;                // use_bvh, and every tree's entries fit the stack words of stream.cuh
     uint32_t tree_kib;        // nodes and leaf slots of every tree, KiB (saturating)
 };

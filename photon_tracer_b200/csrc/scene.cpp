@@ -406,7 +406,7 @@ uint32_t tree_kib(const std::vector<float>& nodes, const std::vector<float>& slo
 
 // Checked over every tree of the arena (conservative: the packed entries are
 // only used by walks of a flat tree, which push flat-tree entries alone).
-int stack_pack8(const std::vector<float>& nodes) {
+static int entries_fit(const std::vector<float>& nodes, uint32_t first_bits) {
     if (nodes.size() / 32 >= (size_t(1) << 31)) return 0;
     for (size_t k = 0; k + 32 <= nodes.size(); k += 32)
         for (int c = 0; c < 4; ++c) {
@@ -415,11 +415,14 @@ int stack_pack8(const std::vector<float>& nodes) {
             std::memcpy(&count, &nodes[k + 28 + c], 4);
             if (count == 0) {
                 if (first >= 0x80000000u) return 0;
-            } else if ((count & PT_COUNT_MASK) > 15u || first >= (1u << 26)) {
+            } else if ((count & PT_COUNT_MASK) > 15u || first >= (1u << first_bits)) {
                 return 0;
             }
         }
     return 1;
 }
+
+int stack_pack8(const std::vector<float>& nodes) { return entries_fit(nodes, 26); }
+int stack_words(const std::vector<float>& nodes) { return entries_fit(nodes, 25); }
 
 }  // namespace pt

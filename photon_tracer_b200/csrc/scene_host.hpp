@@ -45,6 +45,9 @@ int ordered_boxes(const std::vector<float>& nodes);
 // (PtSceneDev::stack_pack8): leaves of at most 15 primitives from below slot
 // 2^26, node indices below 2^31.
 int stack_pack8(const std::vector<float>& nodes);
+// 1 when every entry of the scene's trees fits a stack word of stream.cuh:
+// leaves of at most 15 entries from below 2^25, node indices below 2^31.
+int stack_words(const std::vector<float>& nodes);
 // KiB of nodes and leaf slots (PtSceneDev::tree_kib), saturating.
 uint32_t tree_kib(const std::vector<float>& nodes, const std::vector<float>& slots);
 

@@ -3,6 +3,7 @@
 // the work the algorithmic-bytes roofline is defined on.
 #include "../../include/photon_cuda.h"
 #include "kernels.h"
+#include "stream.cuh"
 #include "tracer.cuh"
 
 using namespace ptd;
@@ -78,6 +79,78 @@ __global__ void __launch_bounds__(128) trace_any_kernel(PtSceneDev S, const floa
     if (overflow) atomicOr(S.status, PT_DEV_ERR_STACK);
 }
 
+// The same queries as streaming walks (stream.cuh): a warp owns every
+// (warps)-th run of 32 rays, and its lanes take their next rays as they
+// finish. Issue- and latency-bound: 1M random rays in the room scene take 106
+// warp instructions per ray at 14.5 threads each, the lock-step kernel above
+// 199 at 5.6. On one B200 (identical hits): 4M such rays 1,087 -> 630 us, 1M
+// rays among instances 335 -> 204 us, 1M rays among 488 spheres 93 -> 84 us.
+// Six resident blocks per SM, one wave of them (5: 686 us, four waves of
+// short-lived warps: 703 us); refills at 8 idle lanes and node phases while
+// 12 lanes stand at nodes are flat optima (4..16 lanes: within 2%).
+constexpr int kStreamBlocks = 6, kStreamFetch = 8, kStreamNodes = 12;
+template <bool INST, bool ANY>
+__global__ void __launch_bounds__(128, kStreamBlocks)
+    trace_stream_kernel(PtSceneDev S, const float* __restrict__ rays, size_t n, float tmin, float tmax,
+                        pt_hit* __restrict__ hits, uint8_t* __restrict__ occ) {
+    PT_WORD_STACK(stack, 128, PT_STREAM_STACK);
+    const int lane = threadIdx.x & 31;
+    const size_t warps = size_t(gridDim.x) * 4, warp = blockIdx.x * size_t(4) + (threadIdx.x >> 5);
+    constexpr unsigned ALL = 0xffffffffu;
+    Walk<INST> w;
+    w.top = 0;
+    int state = WALK_DONE;
+    size_t ray = n;      // the lane's ray; n: none
+    size_t next = 0;     // rays of the warp handed out so far
+    bool more = true, overflow = false;
+    while (true) {
+        const unsigned idle = __ballot_sync(ALL, state == WALK_DONE);
+        if ((more && __popc(idle) >= kStreamFetch) || idle == ALL) {
+            if (state == WALK_DONE) {
+                if (ray < n) {
+                    if (ANY) {
+                        occ[ray] = w.h.kind != PT_HIT_NONE ? 1 : 0;
+                    } else {
+                        uint32_t index, sub;
+                        resolve(S, w.h, index, sub);
+                        pt_hit out;
+                        out.kind = w.h.kind;
+                        out.index = w.h.kind == PT_HIT_NONE ? 0u : index;
+                        out.sub = sub;
+                        out.t = w.t_max;
+                        out.u = w.h.u;
+                        out.v = w.h.v;
+                        hits[ray] = out;
+                    }
+                }
+                const size_t k = next + __popc(idle & ((1u << lane) - 1u));
+                ray = ((k >> 5) * warps + warp) * 32 + (k & 31);
+                if (ray < n) {
+                    V o, d;
+                    load_ray(rays, ray, o, d);
+                    state = w.begin(S, o, d, tmin, tmax, ANY, stack);
+                } else {
+                    ray = n;
+                }
+            }
+            next += __popc(idle);
+            more = ((next >> 5) * warps + warp) * 32 < n;
+            if (__all_sync(ALL, state == WALK_DONE && ray >= n)) break;
+        }
+        while (true) {
+            const unsigned nodes = __ballot_sync(ALL, state == AT_NODE);
+            if (!nodes) break;
+            if (__popc(nodes) < kStreamNodes) {
+                const unsigned done = __ballot_sync(ALL, state == WALK_DONE);
+                if ((nodes | done) != ALL || (more && __popc(done) >= kStreamFetch)) break;
+            }
+            if (state == AT_NODE) state = w.expand(S, tmin, stack, overflow);
+        }
+        if (state == AT_LEAF) state = w.leaf(S, tmin, ANY, stack, overflow);
+    }
+    if (__any_sync(ALL, overflow) && lane == 0) atomicOr(S.status, PT_DEV_ERR_STACK);
+}
+
 __global__ void __launch_bounds__(128) trace_count_kernel(PtSceneDev S, const float* __restrict__ rays, size_t n,
                                                            float tmin, float tmax,
                                                            unsigned long long* __restrict__ counts) {
@@ -131,13 +204,35 @@ __global__ void __launch_bounds__(128) primary_depth_kernel(PtSceneDev S, PtCamD
 
 bool flat_scene(const PtSceneDev& S) { return S.inst_root == PT_NONE && S.n_instances == 0; }
 
-int grid_for(size_t n, int threads) {
+int sm_count() {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+int grid_for(size_t n, int threads) {
     const size_t want = (n + threads - 1) / threads;
-    const size_t cap = size_t(sms) * 16;
+    const size_t cap = size_t(sm_count()) * 16;
     return int(want < cap ? (want ? want : 1) : cap);
+}
+
+// Streaming pays once lanes get several rays each. Below two rays per
+// resident lane a walk's own latency is what counts, and the lock-step kernels
+// with their shorter steps are as fast or faster (room scene, closest hits:
+// 30,000 rays 76 against 87 us, 100,000 rays 95 against 106, 300,000 rays 137
+// against 130).
+bool stream_rays(const PtSceneDev& S, size_t n) { return S.words && n > size_t(sm_count()) * kStreamBlocks * 128 * 2; }
+
+template <bool ANY>
+cudaError_t launch_stream(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax, pt_hit* hits,
+                          uint8_t* occ, cudaStream_t stream) {
+    const int blocks = sm_count() * kStreamBlocks;
+    if (flat_scene(S))
+        trace_stream_kernel<false, ANY><<<blocks, 128, 0, stream>>>(S, rays, n, tmin, tmax, hits, occ);
+    else
+        trace_stream_kernel<true, ANY><<<blocks, 128, 0, stream>>>(S, rays, n, tmin, tmax, hits, occ);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -145,6 +240,7 @@ int grid_for(size_t n, int threads) {
 cudaError_t pt_launch_trace_closest(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax,
                                     void* hits, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
+    if (stream_rays(S, n)) return launch_stream<false>(S, rays, n, tmin, tmax, static_cast<pt_hit*>(hits), nullptr, stream);
     if (flat_scene(S))
         trace_closest_kernel<true><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, static_cast<pt_hit*>(hits));
     else
@@ -155,6 +251,7 @@ cudaError_t pt_launch_trace_closest(const PtSceneDev& S, const float* rays, size
 cudaError_t pt_launch_trace_any(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax,
                                 uint8_t* occ, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
+    if (stream_rays(S, n)) return launch_stream<true>(S, rays, n, tmin, tmax, nullptr, occ, stream);
     if (flat_scene(S))
         trace_any_kernel<true><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, occ);
     else
