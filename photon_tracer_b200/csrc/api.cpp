@@ -69,7 +69,7 @@ struct pt_scene {
     unsigned int* work = nullptr;      // megakernel work counter
     unsigned long long* rays = nullptr;
     cudaStream_t stream = nullptr;
-    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum;
+    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum, samples;
     uint32_t* host_counts = nullptr;  // pinned, for the wavefront queue read-back
     int blocks_per_sm[6] = {0, 0, 0, 0, 0, 0};  // megakernel forms: aux, snapshot; extended light sampling
     uint32_t wave_slots = 0;                   // wavefront path-queue capacity; 0: kMaxWaveSlots
@@ -156,6 +156,49 @@ PtRenderParams make_params(const pt_camera* cam, const pt_settings* st) {
 // Paths the wavefront keeps in flight: one per pixel up to 2^20.
 constexpr uint32_t kMaxWaveSlots = 1u << 20;
 
+// Whether a frame renders with the streaming megakernel. It gains from
+// samples in flight; where a lane per pixel already is one per sample, the
+// lock-step form is as fast or faster: with one sample per pixel up to about a
+// million pixels (room, 360,000 pixels: 0.66 against 0.77 ms; 1.44 million:
+// 2.05 against 1.72), and, in scenes of a few nodes, whose walks are short,
+// with up to three (488 spheres, 1.44 million pixels, 2 samples: 1.90 against
+// 2.01 ms; 3: 2.92 against 2.94).
+bool streams(const pt_scene* s, const PtRenderParams& p) {
+    if (!s->dev.words || p.depth < 1 || p.depth > PT_SAMPLES_MAX_DEPTH) return false;
+    if (p.spp == 1) return s->dev.tree_kib > 64 && int64_t(p.width) * p.rows >= (1 << 20);
+    return p.spp > 3 || s->dev.tree_kib > 64;
+}
+
+// Samples per pixel of one streaming launch, as many as the scene's sample
+// buffer of at most kSampleBytes holds (more launches each wait for their last
+// paths: a 1024x1024 frame of 64 samples takes 4); 0 when the frame has to be
+// rendered without a buffer: under stream capture, where a graph would keep
+// its address, or when there is no memory for it.
+constexpr size_t kSampleBytes = size_t(256) << 20;
+
+int samples_per_launch(pt_scene* s, const PtRenderParams& p, cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return 0;
+    }
+    const size_t one = pt_sample_bytes(p);
+    const size_t most = std::max<size_t>(1, kSampleBytes / one);
+    const int launches = int((size_t(p.spp) + most - 1) / most);
+    const int count = (p.spp + launches - 1) / launches;
+    // growing the buffer must not disturb a capture on another stream
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool ok = one <= 4 * kSampleBytes && s->samples.ensure(one * size_t(count), "samples") == PT_OK;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (!ok) {
+        clear_error();
+        cudaGetLastError();
+        return 0;
+    }
+    return count;
+}
+
 pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t stream) {
     if (mode == PT_MODE_WAVEFRONT) {
         const uint64_t px = uint64_t(p.width) * uint64_t(p.rows);
@@ -168,6 +211,18 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
             return cuda_fail(e, "wavefront");
         return PT_OK;
     }
+    p.work = s->work;
+    if (streams(s, p)) {
+        const int count = samples_per_launch(s, p, stream);
+        for (int first = 0; count > 0 && first < p.spp; first += count) {
+            cudaError_t e = cudaMemsetAsync(s->work, 0, sizeof(unsigned int), stream);
+            if (!e)
+                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first),
+                                      static_cast<float*>(s->samples.ptr), s->sms, stream);
+            if (e) return cuda_fail(e, "megakernel launch");
+        }
+        if (count > 0) return PT_OK;
+    }
     if (cudaError_t e = cudaMemsetAsync(s->work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
     const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
     PtLaunchShape shape;
@@ -176,7 +231,6 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
         s->blocks_per_sm[variant] = pt_megakernel_blocks_per_sm(s->dev, shape.threads, p.aux != nullptr,
                                                                 p.rng_mode == PT_RNG_SNAPSHOT, p.nee_ext != 0);
     shape.blocks = s->sms * s->blocks_per_sm[variant];
-    p.work = s->work;
     if (cudaError_t e = pt_launch_megakernel(s->dev, p, shape, stream)) return cuda_fail(e, "megakernel launch");
     return PT_OK;
 }
@@ -357,6 +411,7 @@ pt_status pt_scene_destroy(pt_scene* s) {
     s->out_hits.release();
     s->counts.release();
     s->wave.release();
+    s->samples.release();
     if (s->host_counts) cudaFreeHost(s->host_counts);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->arena) cudaFree(s->arena);

@@ -37,6 +37,16 @@ cudaError_t pt_launch_megakernel(const PtSceneDev& scene, const PtRenderParams& 
                                  cudaStream_t stream);
 int pt_megakernel_blocks_per_sm(const PtSceneDev& scene, int threads, bool aux, bool snapshot, bool ext);
 
+#define PT_SAMPLES_MAX_DEPTH 0xffff  // bounces a streaming path counts
+// The megakernel's streaming form (scenes with PtSceneDev::words, depth in 1..PT_SAMPLES_MAX_DEPTH):
+// samples [first, first + count) of every pixel as paths of their own, each
+// sample's radiance into `buffer`, then added to the pixels' running sums in
+// p.out / p.aux in sample order (scaled after the last one). buffer holds
+// count * pt_sample_bytes(p) bytes, at most 2^32 - 1 samples. p.work zeroed.
+size_t pt_sample_bytes(const PtRenderParams& p);
+cudaError_t pt_launch_samples(const PtSceneDev& scene, const PtRenderParams& p, int first, int count, float* buffer,
+                              int sms, cudaStream_t stream);
+
 // Ray queries: closest hit (pt_hit records), any hit (bytes), and traversal
 // work counters (5 x u64, added to).
 cudaError_t pt_launch_trace_closest(const PtSceneDev& scene, const float* rays, size_t n, float tmin, float tmax,

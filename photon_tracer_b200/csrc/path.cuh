@@ -102,12 +102,11 @@ __device__ __forceinline__ uint32_t pick_light_ext(const PtSceneDev& S, float u)
 // The extended light sample from the surface rec: a light picked by the
 // power-weighted list, a direction toward it (a light sphere's cone as
 // direct_light samples it, :41-80; a triangle uniformly over its area), and
-// the shadow ray. METAL = false is the matte estimate (albedo / pi times the
-// cosine, the albedo applied by the caller); METAL = true the rough-metal one
+// the shadow ray. metal = false is the matte estimate (albedo / pi times the
+// cosine, the albedo applied by the caller); metal = true the rough-metal one
 // (the lobe density at the direction, weighted against the metal's own
 // scattered ray by the power heuristic). False when no shadow ray is needed.
-template <bool METAL>
-__device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec& rec, V mirror, float fuzz,
+__device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec& rec, bool metal, V mirror, float fuzz,
                                                  const Sampler& smp, Rng& rng, Shadow& sh,
                                                  unsigned long long& rays) {
     const uint32_t k = pick_light_ext(S, rng.real());
@@ -169,7 +168,7 @@ __device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec&
     const float pdf = (S.pick_uniform + S.pick_power * power) * pdf_solid;
     if (!(pdf > 0) || !(pdf < 3.0e38f)) return false;
     float f;
-    if (METAL) {
+    if (metal) {
         const float pb = metal_lobe_pdf(mirror, fuzz, dir);
         const float q = pb / pdf;
         f = q * (1 / (1 + q * q));  // lobe density / light pdf, times the power-heuristic weight
@@ -262,23 +261,24 @@ __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, con
     if (EXT) {
         const bool can = S.sample_lights && S.n_lights + S.n_tri_lights > 0 && p.bounce + 1 < depth;
         const float fuzz = mat.emission_fuzz.w;
+        // Rough metal samples a light whether or not the scatter itself is
+        // absorbed, so the light estimate does not depend on the scatter's
+        // outcome; a matte surface when it scatters. One copy of the sample
+        // for both (a second one made the kernel 15% larger, and it is
+        // instruction fetch that bounds it).
+        const bool metal = type == PT_MAT_METAL && fuzz > 1e-3f && can;
+        V mirror = mk(0, 0, 0);
         p.mis_pdf = 0;
-        if (type == PT_MAT_METAL && fuzz > 1e-3f && can) {
-            // sampled whether or not the scatter itself is absorbed, so the
-            // light estimate does not depend on the scatter's outcome
-            const V mirror = reflect(normalize(p.d), rec.normal);
-            if (direct_light_ext<true>(S, rec, mirror, fuzz, smp, rng, sh, rays)) {
-                nee = true;
-                sh.value = (p.tp * att) * sh.value;
-            }
+        if (metal) {
+            mirror = reflect(normalize(p.d), rec.normal);
             if (scatters) p.mis_pdf = metal_lobe_pdf(mirror, fuzz, normalize(dir));
         }
-        if (!scatters) return STEP_DONE;
-        p.sampled = (flags & PT_MF_DIFFUSE) && can;
-        if (p.sampled && direct_light_ext<false>(S, rec, mk(0, 0, 0), 0.0f, smp, rng, sh, rays)) {
+        p.sampled = scatters && (flags & PT_MF_DIFFUSE) && can;
+        if ((metal || p.sampled) && direct_light_ext(S, rec, metal, mirror, fuzz, smp, rng, sh, rays)) {
             nee = true;
             sh.value = (p.tp * att) * sh.value;
         }
+        if (!scatters) return STEP_DONE;
     } else {
         if (!scatters) return STEP_DONE;
         p.sampled = (flags & PT_MF_DIFFUSE) && S.sample_lights && S.n_lights > 0 && p.bounce + 1 < depth;

@@ -32,14 +32,14 @@ enum : uint32_t {
 };
 __device__ __forceinline__ uint32_t q_count(uint32_t w) { return (w & PT_Q_COUNT) >> 25; }
 
-// A lane's state. Above AT_NODE the walk goes on.
+// A lane's state between the phases.
 enum WalkState : int { WALK_DONE = 0, AT_NODE = 1, AT_LEAF = 2 };
 
-// Stack entries in shared memory, per lane ([depth][thread], 8 bytes each);
-// deeper ones in a local array.
-#ifndef PT_STREAM_STACK
-#define PT_STREAM_STACK 8
-#endif
+// The traversal stack in 8-byte entries: the first SH of each lane in shared
+// memory ([depth][thread]), deeper ones in a local array. The ray-query
+// kernel keeps 8 in shared memory (none: 2% slower); the megakernel, whose
+// paths fill shared memory, none.
+constexpr int kWalkStack = 8;
 
 template <int SH, int NT>
 struct WordStack {
@@ -126,6 +126,7 @@ struct Walk {
         h.u = 0;
         h.v = 0;
         top = 0;
+#pragma unroll 1
         for (uint32_t i = 0; i < S.n_large; ++i)
             if (sphere_hit_double(__ldg(S.large + i), o_, d_, t_min, t_max)) {
                 h.kind = PT_HIT_LARGE;
@@ -236,6 +237,7 @@ struct Walk {
             return AT_NODE;
         }
         const bool spheres = (cur & PT_Q_SPHERE) != 0;
+#pragma unroll 1
         for (uint32_t q = first; q < first + n; ++q) {
             const float4* sl = S.slots + 3 * size_t(q);
             const float4 c = __ldg(sl + 2);

@@ -93,7 +93,7 @@ template <bool INST, bool ANY>
 __global__ void __launch_bounds__(128, kStreamBlocks)
     trace_stream_kernel(PtSceneDev S, const float* __restrict__ rays, size_t n, float tmin, float tmax,
                         pt_hit* __restrict__ hits, uint8_t* __restrict__ occ) {
-    PT_WORD_STACK(stack, 128, PT_STREAM_STACK);
+    PT_WORD_STACK(stack, 128, kWalkStack);
     const int lane = threadIdx.x & 31;
     const size_t warps = size_t(gridDim.x) * 4, warp = blockIdx.x * size_t(4) + (threadIdx.x >> 5);
     constexpr unsigned ALL = 0xffffffffu;

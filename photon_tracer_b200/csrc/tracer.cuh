@@ -1222,6 +1222,7 @@ __device__ __forceinline__ V refract(V uv, V n, float ratio) {
 // as a snapshot) repeats (-1,-1,-1) forever; the bound turns that into a
 // zero offset instead of a hung kernel.
 __device__ __forceinline__ V random_in_unit_sphere(Rng& rng) {
+#pragma unroll 1
     for (int tries = 0; tries < 64; ++tries) {
         const float z = -1.0f + 2.0f * rng.real();
         const float y = -1.0f + 2.0f * rng.real();

@@ -37,3 +37,53 @@ def test_leaf_sizes(built, copies):
                            np.full((n, 1), -1.0)], 1).astype(np.float32)
     assert_hits_equal(s.trace_closest(rays), o.trace_closest(rays, threads=8), rays)
     assert np.array_equal(s.trace_any(rays), o.trace_any(rays))
+
+
+def _frame(torch, scene, cam, st, aux):
+    out = torch.full((st.height, st.width, 3), float("nan"), device="cuda")
+    ax = torch.full((st.height, st.width, 7), float("nan"), device="cuda") if aux else None
+    rays = torch.zeros(1, dtype=torch.int64, device="cuda")
+    return out, ax, rays, lambda: scene.render_device(cam, st, out.data_ptr(), ax.data_ptr() if aux else 0,
+                                                      rays.data_ptr(), torch.cuda.current_stream().cuda_stream)
+
+
+@pytest.mark.parametrize("kind,param,width,height,spp,depth,aux,flags,snapshot", [
+    (10, 0, 2, 2, 4, 10, False, 0, False),          # fewer samples than warps
+    (10, 40, 33, 17, 5, 10, True, 0, False),        # tiles past the right and lower edge
+    (11, 3, 65, 3, 7, 1, True, 0, False),           # one bounce; fewer rows than a tile
+    (11, 3, 200, 113, 2, 10, False, 0, True),       # caller's random states
+    (11, 2, 1024, 1024, 24, 4, False, 0, False),    # more samples than one launch's buffer holds
+    (11, 2, 640, 360, 40, 3, True, 0, False),       # the same with auxiliary outputs
+    (12, 200, 97, 61, 6, 10, True, 0, False),
+    (14, 0, 97, 61, 6, 10, True, 0, False),         # textures, with instances
+    (15, 0, 97, 61, 6, 10, True, 1, False),         # extended light sampling
+    (15, 0, 97, 61, 6, 10, False, 1, False),
+])
+def test_frames_equal_lock_step(built, kind, param, width, height, spp, depth, aux, flags, snapshot):
+    """A captured render cannot keep a sample buffer and takes the lock-step
+    form; the image, the guides and the ray count are the same bit for bit."""
+    import torch
+    from photon_tracer_b200 import abi
+    g = built.Generated(kind, seed=3, param=param)
+    s = built.Scene(g)
+    states = None
+    if snapshot:
+        gen = torch.Generator(device="cuda").manual_seed(5)
+        states = torch.randint(-2**62, 2**62, (width * height * spp, 4), device="cuda", generator=gen)
+    st = built.Scene.settings(width, height, spp, depth, seed=9, first_sample=3, flags=flags,
+                              rng=abi.PT_RNG_SNAPSHOT if snapshot else abi.PT_RNG_SAMPLE,
+                              states_ptr=states.data_ptr() if snapshot else None)
+    out, ax, rays, render = _frame(torch, s, g.camera, st, aux)
+    render()
+    s.sync(torch.cuda.current_stream().cuda_stream)
+    out2, ax2, rays2, render2 = _frame(torch, s, g.camera, st, aux)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        render2()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.isfinite(out).all()
+    assert torch.equal(out.view(torch.int32), out2.view(torch.int32))
+    assert int(rays) == int(rays2) > 0
+    if aux:
+        assert torch.equal(ax.view(torch.int32), ax2.view(torch.int32))
