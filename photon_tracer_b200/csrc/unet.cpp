@@ -21,6 +21,7 @@
 #include <new>
 #include <random>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/photon_cuda.h"
@@ -81,7 +82,8 @@ struct pt_unet {
     DevBuf pool[3];      // p0, p1, p2
     DevBuf cat[3];       // u0, u1, u2
     DevBuf gact[16];     // gradients of x0, a0..a13, out
-    DevBuf g16;          // bf16 copy of the latest ReLU-masked gradient (tensor-core backward)
+    DevBuf g16, g16b;    // bf16 ReLU-masked gradients, the latest and the one before (tensor-core backward)
+    DevBuf g4;           // d loss / d output, float4 per pixel
     DevBuf gpool[3], gcat[3];
     DevBuf loss;
     DevBuf status;
@@ -113,6 +115,8 @@ cudaError_t ensure_workspace(pt_unet* n, int B, int H, int W) {
         g16_elems = c > g16_elems ? c : g16_elems;
     }
     if (!e) e = n->g16.ensure(g16_elems * 2);
+    if (!e) e = n->g16b.ensure(g16_elems * 2);
+    if (!e) e = n->g4.ensure(size_t(pixels_at(n, 0)) * 16);
     const int pool_c[3] = {32, 64, 96}, cat_c[3] = {96, 160, 224};
     for (int l = 0; l < 3 && !e; ++l) {
         const size_t pp = size_t(pixels_at(n, l + 1)), pc = size_t(pixels_at(n, l));
@@ -285,9 +289,91 @@ cudaError_t backward(pt_unet* n, cudaStream_t st) {
     TRY(conv_back(1, bf(1), g(2), true, g(1)));
     TRY(relu_back(1));
     TRY(conv_back(0, bf(0), g(1), true, g(0)));
-#undef TRY
     return cudaSuccess;
 }
+
+// The loss and its backward with the tensor cores: as l1_loss and backward()
+// compute them, with the ReLU masks, the rounding of each gradient to bf16 and
+// the bias sums in the kernels that make the gradients (the epilogue of the
+// input gradient's convolution, or the fused upsample / skip / last-layer
+// steps), so that a float gradient goes through memory only where it has two
+// consumers (the concatenations and pooled inputs). Gradients at activations
+// alternate between two bf16 buffers. input_grad: also d loss / d input, into
+// gact[0].
+cudaError_t loss_backward_tc(pt_unet* n, const float* target, bool input_grad, cudaStream_t st) {
+    cudaError_t e;
+    const int B = n->B, H = n->H, W = n->W;
+    float* G = n->grads.as<float>();
+    unsigned int* status = n->status.as<unsigned int>();
+    __nv_bfloat16* cur = n->g16.as<__nv_bfloat16>();
+    __nv_bfloat16* other = n->g16b.as<__nv_bfloat16>();
+    auto bf = [&](int i) { return n->act[i].as<__nv_bfloat16>(); };
+    auto db = [&](int l) { return G + n->b_off[l]; };
+    auto wt = [&](int l) { return n->wt16.as<__nv_bfloat16>() + n->w_off[l]; };
+    auto wgrad = [&](int l, const __nv_bfloat16* in) {
+        const LayerDef& L = kLayers[l];
+        const unet::ConvShape s{B, H >> L.level, W >> L.level, L.cin, L.cout};
+        return unet::conv_wgrad_tc(s, in, cur, G + n->w_off[l], status, st);
+    };
+    // Layer l's input gradient: into fgrad as float, or (null) masked by the
+    // input activation act[l] into the other buffer, which becomes cur.
+    auto dgrad = [&](int l, float* fgrad) {
+        const LayerDef& L = kLayers[l];
+        const unet::ConvShape t{B, H >> L.level, W >> L.level, L.cout, L.cin};
+        unet::ConvOut o;
+        o.out = fgrad ? static_cast<void*>(fgrad) : other;
+        o.stride = L.cin;
+        if (!fgrad) {
+            o.mask = bf(l);
+            o.colsum = db(l - 1);
+        }
+        const cudaError_t r = unet::conv_fwd_tc(t, cur, wt(l), nullptr, false, o, fgrad != nullptr, status, st);
+        if (!fgrad) std::swap(cur, other);
+        return r;
+    };
+    unet::FlipLayers fl{};
+    fl.n = 15;
+    for (int l = 0; l < 15; ++l) {
+        fl.cin[l] = kLayers[l].cin;
+        fl.cout[l] = kLayers[l].cout;
+        fl.off[l] = long(n->w_off[l]);
+    }
+    const int cat_c[3] = {96, 160, 224};
+    TRY(unet::flip_transpose_all(fl, n->params16.as<__nv_bfloat16>(), n->wt16.as<__nv_bfloat16>(), st));
+    TRY(unet::l1_back(pixels_at(n, 0), n->act[15].as<float>(), target, n->g4.as<float4>(), cur, db(14),
+                      n->loss.as<float>(), st));
+    TRY(wgrad(14, bf(14)));
+    TRY(unet::last_back(B, H, W, n->g4.as<float4>(), wt(14), bf(14), other, db(13), st));
+    std::swap(cur, other);
+    TRY(wgrad(13, bf(13)));
+    TRY(dgrad(13, nullptr));
+    // Decoder levels 0..2: the concatenation's convolution, its upsampled half.
+    for (int lv = 0; lv < 3; ++lv) {
+        const int l = 12 - 2 * lv, up = kLayers[l - 1].cout;  // layer 12, 10, 8 reads cat[lv]
+        TRY(wgrad(l, n->cat[lv].as<__nv_bfloat16>()));
+        TRY(dgrad(l, n->gcat[lv].as<float>()));
+        TRY(unet::up_back(B, H >> (lv + 1), W >> (lv + 1), up, n->gcat[lv].as<float>(), cat_c[lv], bf(l), other,
+                          db(l - 1), st));
+        std::swap(cur, other);
+        TRY(wgrad(l - 1, bf(l - 1)));
+        TRY(dgrad(l - 1, nullptr));
+    }
+    // Encoder levels 3..1: the convolution of the pooled input, the level above it.
+    for (int lv = 2; lv >= 0; --lv) {
+        const int l = 2 * lv + 2, c = kLayers[l - 1].cout;  // layer 6, 4, 2 reads pool[lv]
+        TRY(wgrad(l, n->pool[lv].as<__nv_bfloat16>()));
+        TRY(dgrad(l, n->gpool[lv].as<float>()));
+        TRY(unet::skip_back(B, H >> lv, W >> lv, c, n->gcat[lv].as<float>(), cat_c[lv], cat_c[lv] - c, bf(l),
+                            n->pool[lv].as<__nv_bfloat16>(), n->gpool[lv].as<float>(), other, db(l - 1), st));
+        std::swap(cur, other);
+        TRY(wgrad(l - 1, bf(l - 1)));
+        TRY(dgrad(l - 1, nullptr));
+    }
+    TRY(wgrad(0, bf(0)));
+    if (input_grad) TRY(dgrad(0, n->gact[0].as<float>()));
+    return cudaSuccess;
+}
+#undef TRY
 
 // A tensor-core convolution gave up waiting (bit 0 of the status word):
 // reported once, then cleared.
@@ -420,16 +506,29 @@ pt_status pt_unet_forward(pt_unet* n, int B, int H, int W, const float* d_input,
 // Forward, L1 loss on log radiance and backward; the gradients stay in the
 // network (pt_unet_get_grads), input gradients in d_input_grad if given.
 static pt_status loss_and_grads(pt_unet* n, int B, int H, int W, const float* d_input, const float* d_target,
-                                float* loss_out, cudaStream_t st) {
+                                bool input_grad, float* loss_out, cudaStream_t st) {
     cudaError_t e = ensure_workspace(n, B, H, W);
     const long px = long(B) * H * W;
     if (!e) e = unet::make_input(px, d_input, n->act[0].as<__nv_bfloat16>(), 32, st);
     if (!e) e = forward(n, st, true);
-    if (!e) e = cudaMemsetAsync(n->loss.p, 0, 4, st);
-    if (!e) e = unet::l1_loss(px, kOutStride, n->act[15].as<float>(), d_target, n->gact[15].as<float>(),
-                              n->loss.as<float>(), st);
-    if (!e) e = cudaMemsetAsync(n->grads.p, 0, n->n_params * 4, st);
-    if (!e) e = backward(n, st);
+    auto clear = [&] {
+        const cudaError_t c = cudaMemsetAsync(n->loss.p, 0, 4, st);
+        return c ? c : cudaMemsetAsync(n->grads.p, 0, n->n_params * 4, st);
+    };
+    if (!e) e = clear();
+    bool tc = n->use_tc;
+    if (!e && tc) {
+        e = loss_backward_tc(n, d_target, input_grad, st);
+        if (e == cudaErrorNotSupported) {  // a shape the tensor cores do not take
+            tc = false;
+            e = clear();
+        }
+    }
+    if (!e && !tc) {
+        e = unet::l1_loss(px, kOutStride, n->act[15].as<float>(), d_target, n->gact[15].as<float>(),
+                          n->loss.as<float>(), st);
+        if (!e) e = backward(n, st);
+    }
     float loss = 0;
     unsigned int status = 0;
     if (!e) e = cudaMemcpyAsync(&loss, n->loss.p, 4, cudaMemcpyDeviceToHost, st);
@@ -447,7 +546,7 @@ pt_status pt_unet_train_step(pt_unet* n, int B, int H, int W, const float* d_inp
     if (!n || !d_input || !d_target) return fail(PT_ERR_INVALID_ARG, "pt_unet_train_step: null pointer");
     if (pt_status s = check_size(B, H, W, "pt_unet_train_step")) return s;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (pt_status s = loss_and_grads(n, B, H, W, d_input, d_target, loss_out, st)) return s;
+    if (pt_status s = loss_and_grads(n, B, H, W, d_input, d_target, false, loss_out, st)) return s;
     n->step += 1;
     cudaError_t e = unet::adam(long(n->n_params), n->params.as<float>(), n->grads.as<float>(), n->adam_m.as<float>(),
                                n->adam_v.as<float>(), n->params16.as<__nv_bfloat16>(), lr, n->step, st);
@@ -459,7 +558,7 @@ pt_status pt_unet_loss_grads(pt_unet* n, int B, int H, int W, const float* d_inp
     clear_error();
     if (!n || !d_input || !d_target) return fail(PT_ERR_INVALID_ARG, "pt_unet_loss_grads: null pointer");
     if (pt_status s = check_size(B, H, W, "pt_unet_loss_grads")) return s;
-    if (pt_status s = loss_and_grads(n, B, H, W, d_input, d_target, loss_out, nullptr)) return s;
+    if (pt_status s = loss_and_grads(n, B, H, W, d_input, d_target, host_input_grad != nullptr, loss_out, nullptr)) return s;
     cudaError_t e = cudaSuccess;
     if (host_grads) e = cudaMemcpy(host_grads, n->grads.p, n->n_params * 4, cudaMemcpyDeviceToHost);
     if (!e && host_input_grad)

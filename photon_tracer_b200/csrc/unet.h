@@ -37,6 +37,33 @@ cudaError_t frame_input(int W, int H, int Wp, int Hp, const float* color, const 
 cudaError_t frame_output(int W, int H, int Wp, int stride, const float* pred, float* out, cudaStream_t st);
 cudaError_t l1_loss(long pixels, int stride, const float* pred, const float* target, float* grad, float* loss,
                     cudaStream_t st);
+// The fused steps of the tensor-core backward. Each leaves the gradient at an
+// activation, masked by its ReLU and rounded to bf16, in g16 (the operand of
+// the next weight and input gradients), and adds the masked float gradient's
+// sum over pixels to db, the bias gradient of the layer that made it.
+//
+// l1_back: l1_loss, the gradient as float4 per pixel (g4, channels past the
+// third are zero) and in 16 bf16 channels (g16), and the sums (db).
+cudaError_t l1_back(long pixels, const float* pred, const float* target, float4* g4, __nv_bfloat16* g16, float* db,
+                    float* loss, cudaStream_t st);
+// last_back: through the last layer (wt [32][9][16] flip-transposed) to its
+// input y (32 channels), in float from g4's three channels.
+cudaError_t last_back(int B, int H, int W, const float4* g4, const __nv_bfloat16* wt, const __nv_bfloat16* y,
+                      __nv_bfloat16* g16, float* db, cudaStream_t st);
+// up_back: through the 2x upsampling whose output is channels [0, C) of gcat
+// (stride channels, 2h x 2w) to y (h x w, C channels).
+cudaError_t up_back(int B, int h, int w, int C, const float* gcat, int stride, const __nv_bfloat16* y,
+                    __nv_bfloat16* g16, float* db, cudaStream_t st);
+// skip_back: the gradient at y (H x W, C channels) from its copy in channels
+// [offset, offset + C) of gcat and through its 2x2 max pool.
+cudaError_t skip_back(int B, int H, int W, int C, const float* gcat, int stride, int offset, const __nv_bfloat16* y,
+                      const __nv_bfloat16* pooled, const float* gpool, __nv_bfloat16* g16, float* db, cudaStream_t st);
+// flip_transpose of every layer in one launch.
+struct FlipLayers {
+    int n, cin[16], cout[16];
+    long off[16];
+};
+cudaError_t flip_transpose_all(const FlipLayers& layers, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t st);
 cudaError_t make_output(long pixels, int stride, const float* pred, float* out, cudaStream_t st);
 cudaError_t adam(long n, float* w, const float* g, float* m, float* v, __nv_bfloat16* w16, float lr, int step,
                  cudaStream_t st);
@@ -53,6 +80,11 @@ struct ConvOut {
     __nv_bfloat16* out2 = nullptr;
     int stride2 = 0, offset2 = 0, up2 = 0;
     __nv_bfloat16* pool = nullptr;
+    // Backward: the result is kept where mask ([pixel][Cout], bf16) is
+    // positive and zero elsewhere, and its sum over pixels is added to
+    // colsum (Cout floats). bf16 output, Cout a multiple of 32.
+    const __nv_bfloat16* mask = nullptr;
+    float* colsum = nullptr;
 };
 
 // Tensor-core forward convolution (tcgen05, accumulators in TMEM). Returns

@@ -14,6 +14,8 @@
 
 #include "unet.h"
 
+using unet::FlipLayers;
+
 namespace {
 
 template <class T>
@@ -374,6 +376,220 @@ __global__ void f32_to_bf16_kernel(long n, const float* __restrict__ a, __nv_bfl
         b[i] = __float2bfloat16_rn(a[i]);
 }
 
+// ---- fused backward steps -------------------------------------------------------------------
+// Bound by memory: each reads its float gradients and bf16 activation once and
+// writes bf16, with 16-byte accesses, where separate kernels moved a float
+// gradient through memory two to four times with scalar accesses, and a bias
+// sum on its own ran one block per 4,096 pixels (2.5 ms of a training batch
+// of 16 x 128 x 128; these take 0.1 ms in all). A thread keeps one group of 8
+// channels over all its pixels, so bias sums stay in registers until the end.
+struct Bf8 {
+    float v[8];
+};
+__device__ __forceinline__ Bf8 load_bf8(const __nv_bfloat16* p) {
+    const uint4 q = *reinterpret_cast<const uint4*>(p);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    Bf8 r;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        r.v[2 * i] = __uint_as_float(w[i] << 16);
+        r.v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+    return r;
+}
+__device__ __forceinline__ void store_bf8(__nv_bfloat16* p, const float (&v)[8]) {
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+    }
+    *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void load_f8(const float* p, float (&v)[8]) {
+    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// Masks g by y > 0, stores it as bf16 and adds it to the thread's sums.
+__device__ __forceinline__ void finish8(float (&g)[8], const Bf8& y, __nv_bfloat16* dst, float (&sum)[8]) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        g[i] = y.v[i] > 0.0f ? g[i] : 0.0f;
+        sum[i] += g[i];
+    }
+    store_bf8(dst, g);
+}
+// The block's per-thread sums of channel group `group`, added to db.
+__device__ __forceinline__ void add_sums(float* part, int C, int group, bool active, const float (&sum)[8],
+                                         float* __restrict__ db) {
+    for (int i = threadIdx.x; i < C; i += blockDim.x) part[i] = 0.0f;
+    __syncthreads();
+    if (active)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) atomicAdd(part + 8 * group + i, sum[i]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < C; i += blockDim.x) atomicAdd(db + i, part[i]);
+}
+
+__global__ void __launch_bounds__(256) l1_back_kernel(long pixels, const float* __restrict__ pred,
+                                                      const float* __restrict__ target, float scale,
+                                                      float4* __restrict__ g4, __nv_bfloat16* __restrict__ g16,
+                                                      float* __restrict__ db, float* __restrict__ loss) {
+    float sum[4] = {0, 0, 0, 0};  // three channels' gradients, the loss
+    for (long p = blockIdx.x * long(blockDim.x) + threadIdx.x; p < pixels; p += long(gridDim.x) * blockDim.x) {
+        const float4 q = *reinterpret_cast<const float4*>(pred + 16 * p);
+        const float x[3] = {q.x, q.y, q.z};
+        float g[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float d = x[c] - log1pf(fmaxf(target[p * 3 + c], 0.0f));
+            sum[3] += fabsf(d);
+            g[c] = d > 0 ? scale : d < 0 ? -scale : 0.0f;
+            sum[c] += g[c];
+        }
+        g4[p] = make_float4(g[0], g[1], g[2], 0.0f);
+        store_bf8(g16 + 16 * p, g);
+        *reinterpret_cast<uint4*>(g16 + 16 * p + 8) = make_uint4(0, 0, 0, 0);
+    }
+    __shared__ float part[4];
+    if (threadIdx.x < 4) part[threadIdx.x] = 0.0f;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        for (int off = 16; off > 0; off >>= 1) sum[i] += __shfl_down_sync(0xffffffffu, sum[i], off);
+        if ((threadIdx.x & 31) == 0) atomicAdd(part + i, sum[i]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicAdd(db + threadIdx.x, part[threadIdx.x]);
+    if (threadIdx.x == 3) atomicAdd(loss, part[3]);
+}
+
+// One thread: one pixel, 16 of the 32 channels. The sum runs over taps, then
+// channels, as conv_fwd's does; the gradient's channels past the third are
+// zero and add nothing.
+__global__ void __launch_bounds__(256) last_back_kernel(int B, int H, int W, const float4* __restrict__ g4,
+                                                        const __nv_bfloat16* __restrict__ wt,
+                                                        const __nv_bfloat16* __restrict__ y,
+                                                        __nv_bfloat16* __restrict__ g16, float* __restrict__ db) {
+    __shared__ float4 ws[27][8];  // [tap * 3 + channel][32 outputs]
+    __shared__ float part[32];
+    for (int i = threadIdx.x; i < 27 * 32; i += blockDim.x) {
+        const int ci = i & 31, k = i >> 5, tap = k / 3, c = k - 3 * tap;
+        reinterpret_cast<float*>(ws)[i] = __bfloat162float(wt[(ci * 9 + tap) * 16 + c]);
+    }
+    __syncthreads();
+    const int half = threadIdx.x & 1;
+    float sum[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
+    const long P = long(B) * H * W;
+    for (long p = (blockIdx.x * long(blockDim.x) + threadIdx.x) >> 1; p < P; p += (long(gridDim.x) * blockDim.x) >> 1) {
+        const int x = int(p % W), yy = int((p / W) % H);
+        float acc[2][8];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[i >> 3][i & 7] = 0.0f;
+        for (int tap = 0; tap < 9; ++tap) {
+            const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+            if (yy + dy < 0 || yy + dy >= H || x + dx < 0 || x + dx >= W) continue;
+            const float4 g = __ldg(g4 + p + long(dy) * W + dx);
+            const float gc[3] = {g.x, g.y, g.z};
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 w = ws[tap * 3 + c][4 * half + j];
+                    float* a = &acc[j >> 1][4 * (j & 1)];
+                    a[0] += gc[c] * w.x;
+                    a[1] += gc[c] * w.y;
+                    a[2] += gc[c] * w.z;
+                    a[3] += gc[c] * w.w;
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const size_t at = 32 * size_t(p) + 16 * half + 8 * j;
+            finish8(acc[j], load_bf8(y + at), g16 + at, sum[j]);
+        }
+    }
+    add_sums(part, 32, 2 * half, true, sum[0], db);
+    __syncthreads();
+    add_sums(part, 32, 2 * half + 1, true, sum[1], db);
+}
+
+__global__ void __launch_bounds__(256) up_back_kernel(int B, int h, int w, int C, const float* __restrict__ gcat,
+                                                      int stride, const __nv_bfloat16* __restrict__ y,
+                                                      __nv_bfloat16* __restrict__ g16, float* __restrict__ db) {
+    __shared__ float part[256];
+    const int groups = C / 8, rows = 256 / groups, group = threadIdx.x % groups, row = threadIdx.x / groups;
+    const bool active = row < rows;
+    const int W = 2 * w;
+    const long P = long(B) * h * w;
+    float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (active)
+        for (long p = long(blockIdx.x) * rows + row; p < P; p += long(gridDim.x) * rows) {
+            const int x = int(p % w), yy = int((p / w) % h), b = int(p / (long(w) * h));
+            const float* src = gcat + ((size_t(b) * 2 * h + 2 * yy) * W + 2 * x) * stride + 8 * group;
+            float a0[8], a1[8], a2[8], a3[8], g[8];
+            load_f8(src, a0);
+            load_f8(src + stride, a1);
+            load_f8(src + size_t(W) * stride, a2);
+            load_f8(src + size_t(W + 1) * stride, a3);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) g[i] = a0[i] + a1[i] + a2[i] + a3[i];
+            const size_t at = size_t(p) * C + 8 * group;
+            finish8(g, load_bf8(y + at), g16 + at, sum);
+        }
+    add_sums(part, C, group, active, sum, db);
+}
+
+__global__ void __launch_bounds__(256) skip_back_kernel(int B, int H, int W, int C, const float* __restrict__ gcat,
+                                                        int stride, int offset, const __nv_bfloat16* __restrict__ y,
+                                                        const __nv_bfloat16* __restrict__ pooled,
+                                                        const float* __restrict__ gpool,
+                                                        __nv_bfloat16* __restrict__ g16, float* __restrict__ db) {
+    __shared__ float part[256];
+    const int groups = C / 8, rows = 256 / groups, group = threadIdx.x % groups, row = threadIdx.x / groups;
+    const bool active = row < rows;
+    const int h = H / 2, w = W / 2;
+    const long P = long(B) * h * w;
+    float sum[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (active)
+        for (long p = long(blockIdx.x) * rows + row; p < P; p += long(gridDim.x) * rows) {
+            const int x = int(p % w), yy = int((p / w) % h), b = int(p / (long(w) * h));
+            const size_t px = (size_t(b) * H + 2 * yy) * W + 2 * x;
+            const size_t at[4] = {px, px + 1, px + W, px + W + 1};
+            const Bf8 m = load_bf8(pooled + size_t(p) * C + 8 * group);
+            float gp[8];
+            load_f8(gpool + size_t(p) * C + 8 * group, gp);
+            unsigned taken = 0;  // channels whose maximum has been met
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const Bf8 v = load_bf8(y + at[k] * C + 8 * group);
+                float g[8];
+                load_f8(gcat + at[k] * stride + offset + 8 * group, g);
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (!((taken >> i) & 1u) && v.v[i] == m.v[i]) {
+                        g[i] += gp[i];
+                        taken |= 1u << i;
+                    }
+                finish8(g, v, g16 + at[k] * C + 8 * group, sum);
+            }
+        }
+    add_sums(part, C, group, active, sum, db);
+}
+
+__global__ void __launch_bounds__(256) flip_transpose_all_kernel(const FlipLayers L,
+                                                                 const __nv_bfloat16* __restrict__ w,
+                                                                 __nv_bfloat16* __restrict__ wt) {
+    const int cin = L.cin[blockIdx.y], cout = L.cout[blockIdx.y], n = cin * 9 * cout;
+    w += L.off[blockIdx.y];
+    wt += L.off[blockIdx.y];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int co = i % cout, tap = (i / cout) % 9, ci = i / (cout * 9);
+        wt[i] = w[(co * 9 + (8 - tap)) * cin + ci];
+    }
+}
+
 int grid1(long n) {
     const long g = (n + 255) / 256;
     return int(g < 148 * 16 ? (g > 0 ? g : 1) : 148 * 16);
@@ -501,6 +717,49 @@ cudaError_t frame_output(int W, int H, int Wp, int stride, const float* pred, fl
 cudaError_t l1_loss(long pixels, int stride, const float* pred, const float* target, float* grad, float* loss,
                     cudaStream_t st) {
     l1_kernel<<<grid1(pixels), 256, 0, st>>>(pixels, stride, pred, target, 1.0f / float(pixels * 3), grad, loss);
+    return cudaGetLastError();
+}
+
+namespace {
+// Blocks of the fused backward steps: a few per SM, so that each block's
+// sums cover many pixels and the atomics on db stay few.
+unsigned back_grid(long pixels, int rows) {
+    const long g = (pixels + rows - 1) / rows;
+    return unsigned(g < 148 * 4 ? (g > 0 ? g : 1) : 148 * 4);
+}
+}  // namespace
+
+cudaError_t l1_back(long pixels, const float* pred, const float* target, float4* g4, __nv_bfloat16* g16, float* db,
+                    float* loss, cudaStream_t st) {
+    l1_back_kernel<<<back_grid(pixels, 256), 256, 0, st>>>(pixels, pred, target, 1.0f / float(pixels * 3), g4, g16, db,
+                                                           loss);
+    return cudaGetLastError();
+}
+
+cudaError_t last_back(int B, int H, int W, const float4* g4, const __nv_bfloat16* wt, const __nv_bfloat16* y,
+                      __nv_bfloat16* g16, float* db, cudaStream_t st) {
+    last_back_kernel<<<back_grid(long(B) * H * W, 128), 256, 0, st>>>(B, H, W, g4, wt, y, g16, db);
+    return cudaGetLastError();
+}
+
+cudaError_t up_back(int B, int h, int w, int C, const float* gcat, int stride, const __nv_bfloat16* y,
+                    __nv_bfloat16* g16, float* db, cudaStream_t st) {
+    if (C % 8 || C > 256 || stride % 4) return cudaErrorInvalidValue;
+    up_back_kernel<<<back_grid(long(B) * h * w, 256 / (C / 8)), 256, 0, st>>>(B, h, w, C, gcat, stride, y, g16, db);
+    return cudaGetLastError();
+}
+
+cudaError_t skip_back(int B, int H, int W, int C, const float* gcat, int stride, int offset, const __nv_bfloat16* y,
+                      const __nv_bfloat16* pooled, const float* gpool, __nv_bfloat16* g16, float* db,
+                      cudaStream_t st) {
+    if (C % 8 || C > 256 || stride % 4 || offset % 4) return cudaErrorInvalidValue;
+    skip_back_kernel<<<back_grid(long(B) * H * W / 4, 256 / (C / 8)), 256, 0, st>>>(B, H, W, C, gcat, stride, offset, y,
+                                                                                    pooled, gpool, g16, db);
+    return cudaGetLastError();
+}
+
+cudaError_t flip_transpose_all(const FlipLayers& layers, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t st) {
+    flip_transpose_all_kernel<<<dim3(64, unsigned(layers.n)), 256, 0, st>>>(layers, w, wt);
     return cudaGetLastError();
 }
 

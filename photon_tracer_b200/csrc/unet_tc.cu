@@ -202,7 +202,7 @@ struct TileGrid {
 // TMEM (columns from 0 and from half the allocation, a power of two >= 2N)
 // let the epilogue of one tile overlap the MMAs of the next; the TMA
 // producer runs ahead across tile boundaries.
-template <bool OUT_F32, bool HALO>
+template <bool OUT_F32, bool HALO, bool MASK>
 __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                            const __grid_constant__ CUtensorMap tm_w, int B, int H,
                                                            int W, int Cin, int N, int tmem_cols, int stages,
@@ -258,6 +258,11 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
     // shared-memory broadcasts.
     __shared__ float sbias[kMaxN];
     for (int i = threadIdx.x; i < N; i += kThreads) sbias[i] = bias ? bias[i] : 0.0f;
+    // Backward: each epilogue warp's column sums (a warp's own row, so no
+    // conflicts between warps).
+    __shared__ float scol[4][MASK ? kMaxN : 1];
+    if (MASK)
+        for (int i = threadIdx.x; i < 4 * kMaxN; i += kThreads) scol[i / kMaxN][i % kMaxN] = 0.0f;
     fence_before();
     __syncthreads();
     fence_after();
@@ -384,6 +389,47 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
               tmem_ld16_async(acc_addr + uint32_t(c0), r[0]);
               if (c0 + 16 < N) tmem_ld16_async(acc_addr + uint32_t(c0 + 16), r[1]);
               tmem_wait();
+              if (MASK) {
+                  // the gradient at an activation: zero where its ReLU was
+                  // (mask <= 0), stored as bf16, its column sums kept
+                  float v[32];
+                  const size_t at = pix * size_t(N) + c0;
+                  uint4 y[4], w[4];
+#pragma unroll
+                  for (int j = 0; j < 4; ++j)
+                      y[j] = valid ? __ldg(reinterpret_cast<const uint4*>(o.mask + at) + j) : make_uint4(0, 0, 0, 0);
+                  const uint32_t* yw = reinterpret_cast<const uint32_t*>(y);
+#pragma unroll
+                  for (int j = 0; j < 32; ++j) {
+                      const float yv = __uint_as_float(j & 1 ? yw[j >> 1] & 0xffff0000u : yw[j >> 1] << 16);
+                      v[j] = yv > 0.0f ? __uint_as_float(r[j >> 4][j & 15]) : 0.0f;
+                  }
+#pragma unroll
+                  for (int h = 0; h < 2; ++h) {
+                      float t[16];
+#pragma unroll
+                      for (int j = 0; j < 16; ++j) t[j] = v[16 * h + j];
+                      pack_bf16(t, w[2 * h], w[2 * h + 1]);
+                  }
+                  if (valid) {
+                      uint4* dst = reinterpret_cast<uint4*>(static_cast<__nv_bfloat16*>(o.out) + at);
+#pragma unroll
+                      for (int j = 0; j < 4; ++j) dst[j] = w[j];
+                  }
+                  // Column sums of the warp's 32 pixels: each step halves the
+                  // columns a lane holds, 31 shuffles for all 32.
+#pragma unroll
+                  for (int n = 16; n > 0; n >>= 1) {
+                      const bool hi = (lane & n) != 0;
+#pragma unroll
+                      for (int j = 0; j < n; ++j) {
+                          const float keep = hi ? v[j + n] : v[j], send = hi ? v[j] : v[j + n];
+                          v[j] = keep + __shfl_xor_sync(0xffffffffu, send, n);
+                      }
+                  }
+                  scol[q][c0 + lane] += v[0];
+                  continue;
+              }
 #pragma unroll
               for (int h = 0; h < 2; ++h) {
                 const int c = c0 + 16 * h;
@@ -457,6 +503,9 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
     }
     fence_before();
     __syncthreads();
+    if (MASK)
+        for (int i = threadIdx.x; i < N; i += kThreads)
+            atomicAdd(o.colsum + i, scol[0][i] + scol[1][i] + scol[2][i] + scol[3][i]);
     if (warp == 1) {
         fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
@@ -504,12 +553,12 @@ constexpr size_t kSmemPerSM = 228 * 1024, kResMaxBytes = 80 * 1024;
 #ifndef PT_CONV_RESIDENT
 #define PT_CONV_RESIDENT 1
 #endif
-ConvPlan conv_plan(bool halo, int Cin, int N) {
+ConvPlan conv_plan(bool halo, int Cin, int N, bool mask) {
     ConvPlan p{halo, false, halo ? (N <= 32 ? 3 : 2) : kStagesTile, 0};
     if (PT_CONV_RESIDENT && halo && size_t(9) * Cin * N * 2 <= kResMaxBytes) {
         for (int ctas = 3; ctas >= 2 && !p.res; --ctas)
             for (int st = 6; st >= 2; --st)
-                if (conv_smem(true, true, Cin, N, st) <= kSmemPerSM / ctas - 2048) {
+                if (conv_smem(true, true, Cin, N, st) <= kSmemPerSM / ctas - (mask ? 6144 : 2048)) {
                     p.res = true;
                     p.stages = st;
                     break;
@@ -691,6 +740,10 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
     if (out_f32 && (o.out2 || o.pool)) return cudaErrorNotSupported;
     if (reinterpret_cast<uintptr_t>(o.out2) % 16 || (size_t(o.offset2) * 2) % 16 || (size_t(o.stride2) * 2) % 16)
         return cudaErrorNotSupported;
+    const bool mask = o.mask != nullptr;
+    if (mask && (out_f32 || !o.colsum || !o.out || o.out2 || o.pool || bias || relu || N % 32 || o.stride != N ||
+                 o.offset || reinterpret_cast<uintptr_t>(o.mask) % 16))
+        return cudaErrorNotSupported;
     if (o.pool && (reinterpret_cast<uintptr_t>(o.pool) % 16 || s.H % 2 || s.W % 2)) return cudaErrorNotSupported;
     PFN_cuTensorMapEncodeTiled_v12000 encode = encode_fn();
     if (!encode) return cudaErrorNotSupported;
@@ -735,34 +788,35 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
     }
     int cols = 32;
     while (cols < 2 * N) cols *= 2;  // two accumulators
-    const ConvPlan plan = conv_plan(halo, s.Cin, N);
+    const ConvPlan plan = conv_plan(halo, s.Cin, N, mask);
     const size_t smem = plan.smem;
     const int stages = plan.stages;
     const int tx = halo ? kHaloTX : kTileX, ty = halo ? kHaloTY : kTileY;
     const long tiles = long((s.W + tx - 1) / tx) * ((s.H + ty - 1) / ty) * s.B;
     if (tiles > 0x7fffffffL) return cudaErrorNotSupported;
-    const void* fn = out_f32 ? (halo ? reinterpret_cast<const void*>(conv_tc_kernel<true, true>)
-                                     : reinterpret_cast<const void*>(conv_tc_kernel<true, false>))
-                             : (halo ? reinterpret_cast<const void*>(conv_tc_kernel<false, true>)
-                                     : reinterpret_cast<const void*>(conv_tc_kernel<false, false>));
+    const void* fn = mask      ? (halo ? reinterpret_cast<const void*>(conv_tc_kernel<false, true, true>)
+                                       : reinterpret_cast<const void*>(conv_tc_kernel<false, false, true>))
+                     : out_f32 ? (halo ? reinterpret_cast<const void*>(conv_tc_kernel<true, true, false>)
+                                       : reinterpret_cast<const void*>(conv_tc_kernel<true, false, false>))
+                               : (halo ? reinterpret_cast<const void*>(conv_tc_kernel<false, true, false>)
+                                       : reinterpret_cast<const void*>(conv_tc_kernel<false, false, false>));
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e) return e;
     const long g = grid_size(cols, smem, fn);
     const unsigned blocks = unsigned(tiles < g ? tiles : g);
-#define PT_CONV_LAUNCH(F32, HALO)                                                                                     \
-    conv_tc_kernel<F32, HALO><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N, cols, stages,       \
-                                                             plan.res ? 1 : 0, bias, relu, o, status)
-    if (out_f32) {
-        if (halo)
-            PT_CONV_LAUNCH(true, true);
-        else
-            PT_CONV_LAUNCH(true, false);
-    } else {
-        if (halo)
-            PT_CONV_LAUNCH(false, true);
-        else
-            PT_CONV_LAUNCH(false, false);
-    }
+#define PT_CONV_LAUNCH(F32, MASK)                                                                                    \
+    (halo ? conv_tc_kernel<F32, true, MASK><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N, cols, \
+                                                                           stages, plan.res ? 1 : 0, bias, relu, o,  \
+                                                                           status)                                   \
+          : conv_tc_kernel<F32, false, MASK><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N,     \
+                                                                            cols, stages, plan.res ? 1 : 0, bias,    \
+                                                                            relu, o, status))
+    if (mask)
+        PT_CONV_LAUNCH(false, true);
+    else if (out_f32)
+        PT_CONV_LAUNCH(true, false);
+    else
+        PT_CONV_LAUNCH(false, false);
 #undef PT_CONV_LAUNCH
     return cudaGetLastError();
 }
