@@ -70,6 +70,8 @@ struct pt_scene {
     unsigned long long* rays = nullptr;
     cudaStream_t stream = nullptr;
     Scratch out, aux, states, in_rays, out_hits, counts, wave, sum, samples;
+    float* lent = nullptr;            // a batch's buffer of samples, used instead of `samples`
+    size_t lent_bytes = 0;
     uint32_t* host_counts = nullptr;  // pinned, for the wavefront queue read-back
     int blocks_per_sm[6] = {0, 0, 0, 0, 0, 0};  // megakernel forms: aux, snapshot; extended light sampling
     uint32_t wave_slots = 0;                   // wavefront path-queue capacity; 0: kMaxWaveSlots
@@ -183,9 +185,10 @@ int samples_per_launch(pt_scene* s, const PtRenderParams& p, cudaStream_t stream
         return 0;
     }
     const size_t one = pt_sample_bytes(p);
-    const size_t most = std::max<size_t>(1, kSampleBytes / one);
+    const size_t most = std::max<size_t>(1, (s->lent ? s->lent_bytes : kSampleBytes) / one);
     const int launches = int((size_t(p.spp) + most - 1) / most);
     const int count = (p.spp + launches - 1) / launches;
+    if (s->lent) return one <= s->lent_bytes ? count : 0;
     // growing the buffer must not disturb a capture on another stream
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     cudaThreadExchangeStreamCaptureMode(&mode);
@@ -218,7 +221,7 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
             cudaError_t e = cudaMemsetAsync(s->work, 0, sizeof(unsigned int), stream);
             if (!e)
                 e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first),
-                                      static_cast<float*>(s->samples.ptr), s->sms, stream);
+                                      s->lent ? s->lent : static_cast<float*>(s->samples.ptr), s->sms, stream);
             if (e) return cuda_fail(e, "megakernel launch");
         }
         if (count > 0) return PT_OK;
@@ -238,6 +241,11 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
 }  // namespace
 
 void pt::set_wave_slots(pt_scene* s, uint32_t slots) { s->wave_slots = slots; }
+
+void pt::lend_samples(pt_scene* s, float* buffer, size_t bytes) {
+    s->lent = buffer;
+    s->lent_bytes = bytes;
+}
 
 namespace {
 

@@ -14,6 +14,7 @@
 #include "batch.h"
 #include "kernels.h"
 #include "path.cuh"
+#include "stream_mega.cuh"
 
 using namespace ptd;
 
@@ -254,6 +255,103 @@ __global__ void __launch_bounds__(THREADS, PT_BATCH_MIN_BLOCKS128 * 128 / THREAD
     if (__any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(S0.status, PT_DEV_ERR_STACK);
 }
 
+// ---- the streaming form (stream_mega.cuh) over many frames ----------------------------------------
+// The last of `n` segments whose base is at most `at`.
+template <class Base>
+__device__ __forceinline__ uint32_t segment_of(uint32_t n, uint32_t at, Base&& base) {
+    uint32_t lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi + 1) >> 1;
+        if (base(mid) <= at) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+struct ManyFrames {
+    static constexpr bool kManyScenes = true;
+    PtBatchStream B;
+    int paths;  // a warp keeps in flight
+    __device__ __forceinline__ const PtSceneDev& scene(uint32_t sc) const { return B.b.views[sc]; }
+    __device__ __forceinline__ int depth(uint32_t sc) const { return int(__ldg(&B.b.scenes[sc].depth)); }
+    __device__ __forceinline__ uint32_t items() const { return B.items; }
+    __device__ __forceinline__ int contexts() const { return paths; }
+    __device__ __forceinline__ unsigned int* work() const { return B.b.work; }
+    __device__ __forceinline__ unsigned long long* rays() const { return B.b.rays; }
+    __device__ __forceinline__ unsigned int* status() const { return B.status; }
+    __device__ __forceinline__ float* samples() const { return B.samples; }
+    __device__ __forceinline__ float* guides() const { return nullptr; }
+    __device__ __forceinline__ void started() const {
+        if (threadIdx.x == 0) atomicMin(B.b.start_ns, global_ns());
+    }
+    __device__ __forceinline__ bool locate(uint32_t item, SampleAt& a) const {
+        const PtBatchSegment& G =
+            B.segments[segment_of(B.n_segments, item, [&](uint32_t k) { return __ldg(&B.segments[k].item_base); })];
+        const uint32_t per = __ldg(&G.per_pixel), base = __ldg(&G.item_base), local = item - base;
+        const uint32_t pixel = local / per, s = local - pixel * per;
+        a.scene = __ldg(&G.scene);
+        const PtBatchScene& D = B.b.scenes[a.scene];
+        const uint32_t tx = __ldg(&D.tiles_x), tile = pixel >> 5, ty = tile / tx;
+        a.i = int((tile - ty * tx) * kTileW + (pixel & 7u));
+        a.j = int(ty * kTileH + ((pixel & 31u) >> 3));
+        a.sample = __ldg(&G.first) + s;
+        a.place = base + s * __ldg(&G.pixels) + pixel;
+        return a.i < int(__ldg(&D.width)) && a.j < int(__ldg(&D.height));
+    }
+    __device__ __forceinline__ uint64_t seed(const SampleAt& a) const { return __ldg(&B.b.scenes[a.scene].seed); }
+    __device__ __forceinline__ void ray(const SampleAt& a, float du, float dv, V& o, V& d) const {
+        const PtBatchScene& D = B.b.scenes[a.scene];
+        const float u = (float(a.i) + du) / float(int(__ldg(&D.width)) - 1);
+        const float v = (float(a.j) + dv) / float(int(__ldg(&D.height)) - 1);
+        o = mk(__ldg(&D.cam[0]), __ldg(&D.cam[1]), __ldg(&D.cam[2]));
+        d = mk(__ldg(&D.cam[3]), __ldg(&D.cam[4]), __ldg(&D.cam[5])) +
+            mk(__ldg(&D.cam[6]), __ldg(&D.cam[7]), __ldg(&D.cam[8])) * u +
+            mk(__ldg(&D.cam[9]), __ldg(&D.cam[10]), __ldg(&D.cam[11])) * v - o;
+    }
+    __device__ __forceinline__ void start(const SampleAt& a, Rng& rng) const {
+        rng.seed(sample_stream_seed(seed(a), a.i, a.j, a.sample));
+    }
+};
+
+// Adds one launch's samples to the images' running sums in sample order, and
+// scales them after a pixel's last one.
+__global__ void __launch_bounds__(256) sum_batch_samples(PtBatchStream B) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= B.pixels) return;
+    const PtBatchSegment G =
+        B.segments[segment_of(B.n_segments, p, [&](uint32_t k) { return __ldg(&B.segments[k].pixel_base); })];
+    const PtBatchScene& D = B.b.scenes[G.scene];
+    const uint32_t pixel = p - G.pixel_base, tile = pixel >> 5, ty = tile / D.tiles_x;
+    const uint32_t i = (tile - ty * D.tiles_x) * kTileW + (pixel & 7u), j = ty * kTileH + ((pixel & 31u) >> 3);
+    const bool last = G.first + G.per_pixel >= D.spp;
+    if (i < D.width && j < D.height) {
+        float* out = B.b.out + D.out_offset + 3 * (size_t(D.height - 1 - j) * D.width + i);
+        V acc = G.first ? mk(out[0], out[1], out[2]) : mk(0, 0, 0);
+        for (uint32_t s = 0; s < G.per_pixel; ++s) {
+            const float* r = B.samples + 3 * (size_t(G.item_base) + size_t(s) * G.pixels + pixel);
+            acc = acc + mk(r[0], r[1], r[2]);
+        }
+        const float scale = last ? 1.0f / float(int(D.spp)) : 1.0f;
+        out[0] = acc.x * scale;
+        out[1] = acc.y * scale;
+        out[2] = acc.z * scale;
+    }
+    // a warp's 32 pixels are one tile of one scene
+    if (last && (threadIdx.x & 31) == 0) atomicMax(B.b.done_ns + G.scene, global_ns());
+}
+
+template <bool INST, bool TEX>
+cudaError_t launch_stream(const PtBatchStream& b, int sms, cudaStream_t stream) {
+    ManyFrames F{b, 0};
+    const int blocks =
+        sms * pt_resident_blocks(reinterpret_cast<const void*>(megakernel_stream<false, INST, TEX, false, ManyFrames>),
+                                 128, 0);
+    F.paths = int((b.items + uint32_t(blocks) * 4u - 1) / (uint32_t(blocks) * 4u));
+    megakernel_stream<false, INST, TEX, false, ManyFrames><<<blocks, 128, 0, stream>>>(F);
+    sum_batch_samples<<<(b.pixels + 255) / 256, 256, 0, stream>>>(b);
+    return cudaGetLastError();
+}
+
 template <int THREADS, int TREES, bool TEX>
 void launch(const PtSceneDev& S, const PtBatchLaunch& b, int sms, cudaStream_t stream) {
     const int blocks =
@@ -295,4 +393,10 @@ cudaError_t pt_launch_batch(const PtSceneDev& S, const PtBatchLaunch& b, int thr
         launch_threads<PT_TREES_FLAT, false>(S, b, threads, sms, stream);
     }
     return cudaGetLastError();
+}
+
+cudaError_t pt_launch_batch_stream(const PtSceneDev& S, const PtBatchStream& b, int sms, cudaStream_t stream) {
+    if (S.has_textures)
+        return b.b.any_instances ? launch_stream<true, true>(b, sms, stream) : launch_stream<false, true>(b, sms, stream);
+    return b.b.any_instances ? launch_stream<true, false>(b, sms, stream) : launch_stream<false, false>(b, sms, stream);
 }

@@ -34,5 +34,24 @@ struct PtBatchLaunch {
     int any_instances;                 // some scene has an instance tree: the single-loop traversal
 };
 
+// Streaming form: one launch renders segments, each `per_pixel` samples of
+// every pixel of one scene from sample `first` on, numbered by 8x4 tiles.
+struct PtBatchSegment {
+    uint32_t scene, first, per_pixel;
+    uint32_t pixels;      // tile pixels of the scene's frame
+    uint32_t item_base;   // its first work item in the launch (items: pixels * per_pixel)
+    uint32_t pixel_base;  // its first tile pixel in the launch
+};
+struct PtBatchStream {
+    PtBatchLaunch b;
+    const PtBatchSegment* segments;  // of this launch, in device memory
+    uint32_t n_segments, items, pixels;
+    float* samples;                  // radiance of each sample of the launch, 3 floats each
+    unsigned int* status;
+};
+// Renders the launch's samples and adds them to the images' running sums in
+// sample order. b.work zeroed.
+cudaError_t pt_launch_batch_stream(const PtSceneDev& arena, const PtBatchStream& b, int sms, cudaStream_t stream);
+
 cudaError_t pt_launch_batch(const PtSceneDev& arena, const PtBatchLaunch& b, int threads, int sms,
                             cudaStream_t stream);

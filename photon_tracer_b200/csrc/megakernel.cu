@@ -12,7 +12,7 @@
 // granularity and no lane waits for another lane's pixel.
 #include "kernels.h"
 #include "path.cuh"
-#include "stream.cuh"
+#include "stream_mega.cuh"
 
 using namespace ptd;
 
@@ -282,60 +282,10 @@ __global__ void __launch_bounds__(128, PT_MEGA_MIN_BLOCKS) megakernel(PtSceneDev
     if (__any_sync(0xffffffffu, overflow) && lane == 0) atomicOr(S.status, PT_DEV_ERR_STACK);
 }
 
-// ---- the streaming form ----------------------------------------------------------------------
-// The lock-step form above is bound by divergence: a room-frame query takes
-// 250 warp instructions at 6.6 threads each, because a warp walks until its
-// longest ray is done (4.7 nodes on average, 22 for the longest of 32) and
-// then shades the lanes that happen to hold a path ray. Here a warp keeps up
-// to 64 paths (contexts) in shared memory and works in phases:
-//   shade  32 contexts whose ray was traced, with all lanes busy; ended
-//          samples are written out and their contexts take the next sample;
-//   hand   lanes whose walk is done give their context back and take the
-//          next ray (a shadow ray's context goes straight on to its path ray);
-//   walk   node and leaf steps (stream.cuh), while enough lanes stand at them.
-// 64 contexts are 32 walking and 32 waiting, so that lanes run out of rays just
-// when 32 contexts are ready to shade (48: 10% slower, 40: 20%). It takes 140
-// warp instructions per query at 16.7 threads. What bounds it now: latency of
-// node fetches (L1 hits 78%, long-scoreboard 3.0 of 10 stall cycles per
-// issue) and instruction fetch (65 KB of code, 2.2 of 10).
-//
-// A work item is one sample, not one pixel, so that a small frame fills the
-// GPU and a large one ends without a tail of whole pixels; each sample's
-// radiance goes to a buffer that sum_samples adds up in sample order, which
-// rounds as one pixel's samples rendered in turn. Images are the lock-step
-// form's bit for bit. Measured on one B200, lock-step -> streaming: 1024x1024
-// room, 64 samples 145.0 -> 95.8 ms; 960x540, 16 samples of 10,000 instances
-// 64.3 -> 37.1 ms; 400x225, 16 samples of random spheres 1.86 -> 1.22 ms; one
-// such row of 400 pixels 0.71 -> 0.16 ms.
-//
-// Five resident blocks per SM (96 registers; 4: room 13% slower), four for
-// the forms with more live state, auxiliary outputs (1080p room, 4 samples:
-// 10.0 ms, 5 blocks 11.1) and extended light sampling (8.5 ms, 5 blocks 8.9).
-// Fetch and node thresholds are flat optima (4..12, 8..12: within 2%).
-constexpr int kContexts = 64, kShade = 32, kFetch = 8, kNodes = 12, kStreamBlocks = 5;
-
-// A path's state between the phases, in shared memory: word `field` of
-// context c is ctx[field][c].
-enum : int {
-    C_O = 0,       // origin of the next ray, 3
-    C_D = 3,       // direction of the path's next ray, 3
-    C_SD = 6,      // shadow ray's direction, 3; else the hit's t, u, v
-    C_ST = 9,      // shadow ray's t_max; else the hit's kind
-    C_SV = 10,     // light sample if unblocked, 3; else the hit's index, instance
-    C_TP = 13,     // throughput, 3
-    C_RAD = 16,    // radiance, 3
-    C_FLAGS = 19,  // bounce in bits 0-15, and the CF_ bits
-    C_RNG = 20,    // 8
-    C_SEED = 28,   // the sampler's pixel seed
-    C_INDEX = 29,  // the sampler's index: the sample's number
-    C_ITEM = 30,   // the sample's place in the launch
-    C_MIS = 31     // EXT
-};
-enum : uint32_t { CF_BOUNCE = 0xffffu, CF_SAMPLED = 1u << 16, CF_SHADOW = 1u << 17, CF_ENDED = 1u << 18, CF_LIVE = 1u << 19 };
-
-// One launch over samples: `per_pixel` samples of every pixel from sample
-// `first` on, item = pixel * per_pixel + sample, so that neighbouring items
-// are samples of one pixel. Pixels are numbered by tiles of tile_w x tile_h.
+// ---- the streaming form (stream_mega.cuh) over one frame -----------------------------------------
+// `per_pixel` samples of every pixel from sample `first` on, item = pixel *
+// per_pixel + sample, so that neighbouring items are samples of one pixel.
+// Pixels are numbered by tiles of 8 x 4, rows of a short image by runs of 32.
 struct PtSampleLaunch {
     uint32_t items, pixels, per_pixel, first, tiles_x;
     int tile_w, tile_h;
@@ -353,279 +303,53 @@ __device__ __forceinline__ void sample_pixel(const PtSampleLaunch& L, const PtRe
     pj = P.row0 + int(ty) * L.tile_h + int(l >> sh);
 }
 
-template <bool AUX, bool SNAP, bool INST, bool TEX, bool EXT>
-__global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamBlocks)
-    megakernel_stream(PtSceneDev S, PtRenderParams P, PtSampleLaunch L) {
-    constexpr int C = kContexts, FIELDS = EXT ? 32 : 31;
-    PT_WORD_STACK(stack, 128, 0);
-    constexpr unsigned ALL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    __shared__ uint32_t s_ctx[4][FIELDS][C];
-    __shared__ uint8_t s_ray_q[4][64], s_shade_q[4][64];
-    uint32_t(&ctx)[FIELDS][C] = s_ctx[threadIdx.x >> 5];
-    uint8_t* const ray_q = s_ray_q[threadIdx.x >> 5];
-    uint8_t* const shade_q = s_shade_q[threadIdx.x >> 5];
-    auto getf = [&](int f, int c) { return __uint_as_float(ctx[f][c]); };
-    auto setf = [&](int f, int c, float x) { ctx[f][c] = __float_as_uint(x); };
-    auto getv = [&](int f, int c) { return mk(getf(f, c), getf(f + 1, c), getf(f + 2, c)); };
-    auto setv = [&](int f, int c, V x) {
-        setf(f, c, x.x);
-        setf(f + 1, c, x.y);
-        setf(f + 2, c, x.z);
-    };
-
-    const int contexts = min(L.contexts, C);
-    for (int c = lane; c < contexts; c += 32) {
-        ctx[C_FLAGS][c] = CF_ENDED;
-        shade_q[c] = uint8_t(c);
+template <bool SNAP>
+struct OneFrame {
+    static constexpr bool kManyScenes = false;
+    PtSceneDev S;
+    PtRenderParams P;
+    PtSampleLaunch L;
+    __device__ __forceinline__ const PtSceneDev& scene(uint32_t) const { return S; }
+    __device__ __forceinline__ int depth(uint32_t) const { return P.depth; }
+    __device__ __forceinline__ uint32_t items() const { return L.items; }
+    __device__ __forceinline__ int contexts() const { return L.contexts; }
+    __device__ __forceinline__ unsigned int* work() const { return P.work; }
+    __device__ __forceinline__ unsigned long long* rays() const { return P.rays; }
+    __device__ __forceinline__ unsigned int* status() const { return S.status; }
+    __device__ __forceinline__ float* samples() const { return L.samples; }
+    __device__ __forceinline__ float* guides() const { return L.guides; }
+    __device__ __forceinline__ void started() const {}
+    // False for an item of a tile past the image's edge.
+    __device__ __forceinline__ bool locate(uint32_t item, SampleAt& a) const {
+        const uint32_t pixel = item / L.per_pixel, s = item - pixel * L.per_pixel;
+        sample_pixel(L, P, pixel, a.i, a.j);
+        a.sample = uint32_t(P.first_sample) + L.first + s;
+        a.place = s * L.pixels + pixel;
+        a.scene = 0;
+        return a.i < P.width && a.j < P.row0 + P.rows;
     }
-    __syncwarp();
-    // queue heads and lengths, the same in every lane
-    int ray_h = 0, ray_n = 0, shade_h = 0, shade_n = contexts;
-    unsigned long long rays = 0;
-    bool overflow = false, shadow = false;
-    int state = WALK_DONE, c = -1;  // c: the context this lane walks for
-    Walk<INST> w;
-    w.top = 0;
-    w.h.kind = PT_HIT_NONE;
-
-    while (true) {
-        const unsigned walking = __ballot_sync(ALL, state != WALK_DONE);
-        if (shade_n >= kShade || (shade_n > 0 && ray_n == 0 && shade_n >= __popc(walking))) {
-            // Shade up to 32 contexts.
-            const int m = min(32, shade_n);
-            const bool act = lane < m;
-            const int k = act ? shade_q[(shade_h + lane) & 63] : 0;
-            shade_h += m;
-            shade_n -= m;
-            uint32_t flags = act ? ctx[C_FLAGS][k] : 0u;
-            bool ended = act && (flags & CF_ENDED), push = false;
-            Rng rng;
-            Sampler smp;
-            if (act && !ended) {
-                Path path;
-                path.o = getv(C_O, k);
-                path.d = getv(C_D, k);
-                path.tp = getv(C_TP, k);
-                path.rad = getv(C_RAD, k);
-                path.bounce = int(flags & CF_BOUNCE);
-                path.sampled = (flags & CF_SAMPLED) != 0;
-                if (EXT) path.mis_pdf = getf(C_MIS, k);
-                uint64_t r[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) r[i] = ctx[C_RNG + 2 * i][k] | (uint64_t(ctx[C_RNG + 2 * i + 1][k]) << 32);
-                rng.s0 = r[0];
-                rng.s1 = r[1];
-                rng.s2 = r[2];
-                rng.s3 = r[3];
-                smp.pixel_seed = ctx[C_SEED][k];
-                smp.index = ctx[C_INDEX][k];
-                smp.set_bounce(path.bounce);
-                Hit h;
-                h.kind = ctx[C_ST][k];
-                h.index = ctx[C_SV][k];
-                h.inst = INST ? ctx[C_SV + 1][k] : 0u;
-                h.u = getf(C_SD + 1, k);
-                h.v = getf(C_SD + 2, k);
-                const bool hit = h.kind != PT_HIT_NONE;
-                Rec rec;
-                if (hit) fill<TEX, EXT>(S, h, path.o, path.d, getf(C_SD, k), rec);
-                First first;
-                const bool primary = AUX && path.bounce == 0;
-                bool nee;
-                Shadow sh;
-                const bool done =
-                    shade<AUX, TEX, EXT>(S, path, hit, rec, P.depth, smp, rng, first, nee, sh, rays) == STEP_DONE;
-                if (primary) {  // the first hit's guides
-                    float* g = L.guides + 6 * size_t(ctx[C_ITEM][k]);
-                    g[0] = first.albedo.x;
-                    g[1] = first.albedo.y;
-                    g[2] = first.albedo.z;
-                    g[3] = first.normal.x;
-                    g[4] = first.normal.y;
-                    g[5] = first.normal.z;
-                }
-                setv(C_RAD, k, path.rad);
-                flags = CF_LIVE | (uint32_t(path.bounce) & CF_BOUNCE) | (path.sampled ? CF_SAMPLED : 0u);
-                if (!done) {
-                    setv(C_O, k, path.o);
-                    setv(C_D, k, path.d);
-                    setv(C_TP, k, path.tp);
-                    if (EXT) setf(C_MIS, k, path.mis_pdf);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const uint64_t x = i == 0 ? rng.s0 : i == 1 ? rng.s1 : i == 2 ? rng.s2 : rng.s3;
-                        ctx[C_RNG + 2 * i][k] = uint32_t(x);
-                        ctx[C_RNG + 2 * i + 1][k] = uint32_t(x >> 32);
-                    }
-                }
-                if (nee) {
-                    setv(C_O, k, sh.o);
-                    setv(C_SD, k, sh.d);
-                    setf(C_ST, k, sh.t_max);
-                    setv(C_SV, k, sh.value);
-                    flags |= CF_SHADOW | (done ? CF_ENDED : 0u);
-                    push = true;
-                } else if (done) {
-                    ended = true;
-                } else {
-                    push = true;
-                }
-            }
-            if (ended && (flags & CF_LIVE)) {
-                const V rad = getv(C_RAD, k);
-                float* out = L.samples + 3 * size_t(ctx[C_ITEM][k]);
-                out[0] = rad.x;
-                out[1] = rad.y;
-                out[2] = rad.z;
-            }
-            // Contexts whose sample ended take the next ones; those past the
-            // last are dropped.
-            bool need = ended, fresh = false;
-            int pi = 0, pj = 0;
-            uint32_t s = 0, place = 0;
-            while (true) {
-                const unsigned want = __ballot_sync(ALL, need);
-                if (!want) break;
-                const int leader = __ffs(want) - 1;
-                uint32_t base = 0;
-                if (lane == leader) base = atomicAdd(P.work, uint32_t(__popc(want)));
-                base = __shfl_sync(ALL, base, leader);
-                if (need) {
-                    const uint32_t item = base + __popc(want & ((1u << lane) - 1u));
-                    if (item >= L.items) {
-                        need = false;
-                    } else {
-                        const uint32_t pixel = item / L.per_pixel;
-                        s = item - pixel * L.per_pixel;
-                        place = s * L.pixels + pixel;
-                        sample_pixel(L, P, pixel, pi, pj);
-                        if (pi < P.width && pj < P.row0 + P.rows) {
-                            need = false;
-                            fresh = true;
-                        }
-                    }
-                }
-            }
-            if (fresh) {
-                // render_row_impl's sample loop body (:379-385)
-                const uint32_t idx = uint32_t(P.first_sample) + L.first + s;
-                smp.begin(P.seed, pi, pj, idx);
-                float du, dv;
-                smp.sample_2d(0, rng, du, dv);
-                const float u = (float(pi) + du) / float(P.width - 1);
-                const float v = (float(pj) + dv) / float(P.height - 1);
-                const V org = mk(P.cam.origin[0], P.cam.origin[1], P.cam.origin[2]);
-                setv(C_O, k, org);
-                setv(C_D, k,
-                     mk(P.cam.llc[0], P.cam.llc[1], P.cam.llc[2]) +
-                         mk(P.cam.horizontal[0], P.cam.horizontal[1], P.cam.horizontal[2]) * u +
-                         mk(P.cam.vertical[0], P.cam.vertical[1], P.cam.vertical[2]) * v - org);
-                setv(C_TP, k, mk(1, 1, 1));
-                setv(C_RAD, k, mk(0, 0, 0));
-                if (EXT) setf(C_MIS, k, 0);
-                if (SNAP) {
-                    const uint64_t* st = P.states + 4 * ((size_t(pj) * P.width + pi) * P.spp + L.first + s);
-                    rng.s0 = st[0];
-                    rng.s1 = st[1];
-                    rng.s2 = st[2];
-                    rng.s3 = st[3];
-                } else {
-                    rng.seed(sample_stream_seed(P.seed, pi, pj, idx));
-                }
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint64_t x = i == 0 ? rng.s0 : i == 1 ? rng.s1 : i == 2 ? rng.s2 : rng.s3;
-                    ctx[C_RNG + 2 * i][k] = uint32_t(x);
-                    ctx[C_RNG + 2 * i + 1][k] = uint32_t(x >> 32);
-                }
-                ctx[C_SEED][k] = smp.pixel_seed;
-                ctx[C_INDEX][k] = idx;
-                ctx[C_ITEM][k] = place;
-                flags = CF_LIVE;
-                push = true;
-            }
-            if (push) ctx[C_FLAGS][k] = flags;
-            const unsigned pushed = __ballot_sync(ALL, push);
-            if (push) ray_q[(ray_h + ray_n + __popc(pushed & ((1u << lane) - 1u))) & 63] = uint8_t(k);
-            ray_n += __popc(pushed);
-            __syncwarp();
-        }
-
-        // Lanes whose walk is done hand over their context and take the next.
-        {
-            const unsigned done = __ballot_sync(ALL, state == WALK_DONE);
-            const unsigned full = __ballot_sync(ALL, state == WALK_DONE && c >= 0);
-            if (done == ALL && !full && ray_n == 0 && shade_n == 0) break;
-            if ((full | (ray_n ? done : 0u)) && (__popc(full | (ray_n ? done : 0u)) >= kFetch || done == ALL)) {
-                bool go = false, hand = false;
-                if (state == WALK_DONE && c >= 0) {
-                    if (shadow) {
-                        if (w.h.kind == PT_HIT_NONE) setv(C_RAD, c, getv(C_RAD, c) + getv(C_SV, c));
-                        const uint32_t flags = ctx[C_FLAGS][c] & ~CF_SHADOW;
-                        ctx[C_FLAGS][c] = flags;
-                        hand = (flags & CF_ENDED) != 0;
-                        go = !hand;
-                    } else {
-                        setf(C_SD, c, w.t_max);
-                        setf(C_SD + 1, c, w.h.u);
-                        setf(C_SD + 2, c, w.h.v);
-                        ctx[C_ST][c] = w.h.kind;
-                        ctx[C_SV][c] = w.h.index;
-                        if (INST) ctx[C_SV + 1][c] = w.h.inst;
-                        hand = true;
-                    }
-                }
-                const unsigned handed = __ballot_sync(ALL, hand);
-                if (hand) {
-                    shade_q[(shade_h + shade_n + __popc(handed & ((1u << lane) - 1u))) & 63] = uint8_t(c);
-                    c = -1;
-                }
-                shade_n += __popc(handed);
-                const unsigned take = __ballot_sync(ALL, state == WALK_DONE && c < 0);
-                if (state == WALK_DONE && c < 0) {
-                    const int i = __popc(take & ((1u << lane) - 1u));
-                    if (i < ray_n) {
-                        c = ray_q[(ray_h + i) & 63];
-                        go = true;
-                    }
-                }
-                const int got = min(ray_n, __popc(take));
-                ray_h += got;
-                ray_n -= got;
-                __syncwarp();
-                if (go) {
-                    shadow = (ctx[C_FLAGS][c] & CF_SHADOW) != 0;
-                    if (!shadow) ++rays;
-                    state = w.begin(S, getv(C_O, c), getv(shadow ? C_SD : C_D, c), 0.001f,
-                                    shadow ? getf(C_ST, c) : 1000.0f, shadow, stack);
-                }
-            }
-        }
-
-        if (shade_n >= kShade && ray_n == 0) continue;
-        while (true) {
-            const unsigned nodes = __ballot_sync(ALL, state == AT_NODE);
-            if (!nodes) break;
-            if (__popc(nodes) < kNodes) {
-                const unsigned done = __ballot_sync(ALL, state == WALK_DONE && (c >= 0 || ray_n > 0));
-                const unsigned leaves = __ballot_sync(ALL, state == AT_LEAF);
-                if (leaves || __popc(done) >= kFetch) break;
-                if (shade_n > 0 && ray_n == 0 && shade_n >= __popc(nodes)) break;
-            } else if (ray_n > 0 && __popc(__ballot_sync(ALL, state == WALK_DONE)) >= kFetch) {
-                break;
-            }
-            if (state == AT_NODE) state = w.expand(S, 0.001f, stack, overflow);
-        }
-        if (state == AT_LEAF) state = w.leaf(S, 0.001f, shadow, stack, overflow);
+    __device__ __forceinline__ uint64_t seed(const SampleAt&) const { return P.seed; }
+    __device__ __forceinline__ void ray(const SampleAt& a, float du, float dv, V& o, V& d) const {
+        const float u = (float(a.i) + du) / float(P.width - 1);
+        const float v = (float(a.j) + dv) / float(P.height - 1);
+        o = mk(P.cam.origin[0], P.cam.origin[1], P.cam.origin[2]);
+        d = mk(P.cam.llc[0], P.cam.llc[1], P.cam.llc[2]) +
+            mk(P.cam.horizontal[0], P.cam.horizontal[1], P.cam.horizontal[2]) * u +
+            mk(P.cam.vertical[0], P.cam.vertical[1], P.cam.vertical[2]) * v - o;
     }
-
-    unsigned long long total = rays;
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) total += __shfl_down_sync(ALL, total, off);
-    if (lane == 0 && P.rays) atomicAdd(P.rays, total);
-    if (__any_sync(ALL, overflow) && lane == 0) atomicOr(S.status, PT_DEV_ERR_STACK);
-}
+    __device__ __forceinline__ void start(const SampleAt& a, Rng& rng) const {
+        if (SNAP) {
+            const uint64_t* st =
+                P.states + 4 * ((size_t(a.j) * P.width + a.i) * P.spp + (a.sample - uint32_t(P.first_sample)));
+            rng.s0 = st[0];
+            rng.s1 = st[1];
+            rng.s2 = st[2];
+            rng.s3 = st[3];
+        } else {
+            rng.seed(sample_stream_seed(P.seed, a.i, a.j, a.sample));
+        }
+    }
+};
 
 // Adds one launch's samples to the pixels' running sums in sample order -- the
 // order, and so the rounding, of a pixel's samples rendered one after another
@@ -674,10 +398,10 @@ cudaError_t launch_s(const PtSceneDev& S, const PtRenderParams& p, PtSampleLaunc
     int per_sm = blocks_per_sm;
     if (!per_sm)
         blocks_per_sm = per_sm = pt_resident_blocks(
-            reinterpret_cast<const void*>(megakernel_stream<AUX, SNAP, INST, TEX, EXT>), 128, 0);
+            reinterpret_cast<const void*>(megakernel_stream<AUX, INST, TEX, EXT, OneFrame<SNAP>>), 128, 0);
     const uint32_t warps = uint32_t(sms * per_sm) * 4u;
     L.contexts = int((L.items + warps - 1) / warps);
-    megakernel_stream<AUX, SNAP, INST, TEX, EXT><<<sms * per_sm, 128, 0, stream>>>(S, p, L);
+    megakernel_stream<AUX, INST, TEX, EXT, OneFrame<SNAP>><<<sms * per_sm, 128, 0, stream>>>({S, p, L});
     sum_samples<AUX><<<(L.pixels + 255) / 256, 256, 0, stream>>>(p, L);
     return cudaGetLastError();
 }

@@ -87,3 +87,27 @@ def test_frames_equal_lock_step(built, kind, param, width, height, spp, depth, a
     assert int(rays) == int(rays2) > 0
     if aux:
         assert torch.equal(ax.view(torch.int32), ax2.view(torch.int32))
+
+
+@pytest.mark.parametrize("sizes", [
+    [(2, 2, 70000), (33, 17, 500)],              # more samples of a pixel than a launch of one scene needs
+    [(640, 361, 64), (200, 3, 3), (500, 333, 120), (31, 65, 1)],  # launches that end inside a scene
+])
+def test_streamed_batch(built, sizes):
+    """A batch large enough to stream gives each scene the image its own
+    render gives, whatever launch its samples fall into."""
+    from photon_tracer_b200 import abi
+    items = []
+    for k, (w, h, spp) in enumerate(sizes):
+        g = built.Generated([11, 10, 12][k % 3], seed=k + 1, param=[2, 30, 60][k % 3])
+        items.append((g, g.camera, w, h, spp, 50 + k))
+    b = built.Batch(items, abi.PT_BATCH_ONE_LAUNCH, max_bounces=3)
+    for _ in range(2):
+        rays, total = b.render(), 0
+        for i, (g, cam, w, h, spp, seed) in enumerate(items):
+            img, _, r = built.Scene(g).render(cam, w, h, spp, 3, seed=seed)
+            total += r
+            assert b.image(i).tobytes() == img.tobytes(), f"scene {i}"
+        assert rays == total
+    times = b.scene_times()
+    assert np.all(times > 0) and np.all(np.isfinite(times))
