@@ -70,7 +70,29 @@ struct WordStack {
     ::ptd::WordStack<(SH), (NT)> name{                                                                    \
         static_cast<uint32_t>(__cvta_generic_to_shared(&name##_s[0])) + threadIdx.x * 8u, name##_deep}
 
-// One ray's walk. INST: the scene has instances (wo, wd keep the world ray).
+// Where a walk leaves its nearest hit and finds its world-space ray. In
+// registers, for ray queries:
+struct HitRegs {
+    Hit h;
+    V o, d;  // the ray in world space
+    __device__ __forceinline__ void world(V& wo, V& wd) const {
+        wo = o;
+        wd = d;
+    }
+    __device__ __forceinline__ void clear(uint32_t kind, uint32_t index) { h = {kind, index, 0, 0, 0}; }
+    __device__ __forceinline__ void set(uint32_t kind, uint32_t index, uint32_t inst) {
+        h.kind = kind;
+        h.index = index;
+        h.inst = inst;
+    }
+    __device__ __forceinline__ void set_uv(float u, float v) {
+        h.u = u;
+        h.v = v;
+    }
+    __device__ __forceinline__ void drop() { h.kind = PT_HIT_NONE; }
+};
+
+// One ray's walk. INST: the scene has instances.
 template <bool INST>
 struct Walk {
     V o, d;
@@ -80,10 +102,8 @@ struct Walk {
     float t_max;
     int top;
     uint32_t cur;
-    Hit h;
     uint32_t cur_inst;
     bool in_mesh;
-    V wo, wd;
 
     __device__ __forceinline__ void set(const PtSceneDev& S, V o_, V d_, float t_min) {
         o = o_;
@@ -99,13 +119,15 @@ struct Walk {
     }
 
     // The next entry that is not behind t_max becomes cur.
-    template <class Stack>
-    __device__ __forceinline__ int pop(const PtSceneDev& S, float t_min, Stack& stack) {
+    template <class Stack, class Out>
+    __device__ __forceinline__ int pop(const PtSceneDev& S, float t_min, Stack& stack, const Out& out) {
         while (top > 0) {
             float t;
             stack.get(--top, cur, t);
             if (t >= t_max) continue;
             if (INST && cur == PT_Q_WORLD) {
+                V wo, wd;
+                out.world(wo, wd);
                 set(S, wo, wd, t_min);
                 in_mesh = false;
                 continue;
@@ -116,40 +138,36 @@ struct Walk {
     }
 
     // Large spheres, then the root of the tree; WALK_DONE when nothing is left to walk.
-    template <class Stack>
+    template <class Stack, class Out>
     __device__ __forceinline__ int begin(const PtSceneDev& S, V o_, V d_, float t_min, float t_max_, bool any,
-                                         Stack& stack) {
+                                         Stack& stack, Out& hit) {
         t_max = t_max_;
-        h.kind = PT_HIT_NONE;
-        h.index = 0;
-        h.inst = 0;
-        h.u = 0;
-        h.v = 0;
         top = 0;
+        uint32_t kind = PT_HIT_NONE, index = 0;
 #pragma unroll 1
         for (uint32_t i = 0; i < S.n_large; ++i)
             if (sphere_hit_double(__ldg(S.large + i), o_, d_, t_min, t_max)) {
-                h.kind = PT_HIT_LARGE;
-                h.index = i;
-                if (any) return WALK_DONE;
+                kind = PT_HIT_LARGE;
+                index = i;
+                if (any) break;
             }
+        hit.clear(kind, index);
+        if (any && kind != PT_HIT_NONE) return WALK_DONE;
         set(S, o_, d_, t_min);
         if (INST) {
-            wo = o_;
-            wd = d_;
             in_mesh = false;
             cur_inst = 0;
             if (S.inst_root != PT_NONE) stack.put(top++, S.inst_root, t_min);
         }
         if (S.flat_root != PT_NONE) stack.put(top++, S.flat_root, t_min);
-        return pop(S, t_min, stack);
+        return pop(S, t_min, stack, hit);
     }
 
     // Slab-tests node cur's four children against [t_min, t_max] and pushes
     // the ones hit, farthest first (bvh.hpp:72-103), then pops. The walk
     // ends, with the overflow flag set, if the stack would overflow.
-    template <class Stack>
-    __device__ __forceinline__ int expand(const PtSceneDev& S, float t_min, Stack& stack, bool& overflow) {
+    template <class Stack, class Out>
+    __device__ __forceinline__ int expand(const PtSceneDev& S, float t_min, Stack& stack, Out& out, bool& overflow) {
         const float4* nd = S.qnodes + 8 * size_t(cur);
         const float4 lox = __ldg(nd + nx), loy = __ldg(nd + ny), loz = __ldg(nd + nz);
         const float4 hix = __ldg(nd + (3 - nx)), hiy = __ldg(nd + (5 - ny)), hiz = __ldg(nd + (7 - nz));
@@ -197,7 +215,7 @@ struct Walk {
             const int n = __popc(mask);
             if (top + n > PT_STACK_MAX) {
                 overflow = true;
-                h.kind = PT_HIT_NONE;
+                out.drop();
                 return WALK_DONE;
             }
             const uint32_t ws[4] = {words.x, words.y, words.z, words.w};
@@ -208,19 +226,20 @@ struct Walk {
                 if (mask & (1 << c)) stack.put(top + rank[c], ws[c], tn[c]);
             top += n;
         }
-        return pop(S, t_min, stack);
+        return pop(S, t_min, stack, out);
     }
 
     // The leaf cur: its primitives in order, or its first instance entered.
-    template <class Stack>
-    __device__ __forceinline__ int leaf(const PtSceneDev& S, float t_min, bool any, Stack& stack, bool& overflow) {
+    template <class Stack, class Out>
+    __device__ __forceinline__ int leaf(const PtSceneDev& S, float t_min, bool any, Stack& stack, Out& out,
+                                        bool& overflow) {
         const uint32_t first = cur & PT_Q_FIRST, n = q_count(cur);
         if (INST && (cur & PT_Q_INST)) {
             // hit_instance (include/geometry.hpp:212-229): the rest of the
             // leaf and the return to the world ray wait on the stack, unpruned.
             if (top + 3 > PT_STACK_MAX) {
                 overflow = true;
-                h.kind = PT_HIT_NONE;
+                out.drop();
                 return WALK_DONE;
             }
             const float4* is = S.islots + 4 * size_t(first);
@@ -229,10 +248,12 @@ struct Walk {
             const float never = -__int_as_float(0x7f800000);
             if (n > 1) stack.put(top++, PT_Q_LEAF | PT_Q_INST | ((n - 1) << 25) | (first + 1), never);
             stack.put(top++, PT_Q_WORLD, never);
+            V wo, wd;
+            out.world(wo, wd);
             set(S, aff_point(rows, wo), aff_vector(rows, wd), t_min);
             cur_inst = meta.y;
             in_mesh = true;
-            if (t_min >= t_max) return pop(S, t_min, stack);
+            if (t_min >= t_max) return pop(S, t_min, stack, out);
             cur = meta.x;
             return AT_NODE;
         }
@@ -240,22 +261,23 @@ struct Walk {
 #pragma unroll 1
         for (uint32_t q = first; q < first + n; ++q) {
             const float4* sl = S.slots + 3 * size_t(q);
-            const float4 c = __ldg(sl + 2);
+            const float4 a = __ldg(sl), b = __ldg(sl + 1), c = __ldg(sl + 2);
+            const uint32_t in = INST && in_mesh ? cur_inst : 0u;
             bool hit;
             if (spheres && (fbits(c.y) & PT_SLOT_SPHERE)) {
-                hit = sphere_hit(__ldg(sl), o, d, t_min, t_max);
-                if (hit) h.kind = PT_HIT_SPHERE;
+                hit = sphere_hit(a, o, d, t_min, t_max);
+                if (hit) out.set(PT_HIT_SPHERE, q, in);
             } else {
-                hit = tri_hit(__ldg(sl), __ldg(sl + 1), c, o, d, t_min, t_max, h.u, h.v);
-                if (hit) h.kind = INST && in_mesh ? PT_HIT_INSTANCE : PT_HIT_TRIANGLE;
+                float u, v;
+                hit = tri_hit(a, b, c, o, d, t_min, t_max, u, v);
+                if (hit) {
+                    out.set(INST && in_mesh ? PT_HIT_INSTANCE : PT_HIT_TRIANGLE, q, in);
+                    out.set_uv(u, v);
+                }
             }
-            if (hit) {
-                h.index = q;
-                if (INST) h.inst = in_mesh ? cur_inst : 0u;
-                if (any) return WALK_DONE;
-            }
+            if (hit && any) return WALK_DONE;
         }
-        return pop(S, t_min, stack);
+        return pop(S, t_min, stack, out);
     }
 };
 

@@ -15,20 +15,21 @@
 // when 32 contexts are ready to shade (48: 10% slower, 40: 20%). It takes 140
 // warp instructions per query at 16.7 threads. What bounds it now: latency of
 // node fetches (L1 hits 78%, long-scoreboard 3.0 of 10 stall cycles per
-// issue) and instruction fetch (65 KB of code, 2.2 of 10).
+// issue) and instruction fetch (65 KB of code, 2.2 of 10: 3.7 KB more cost the
+// room frame 14%, so duplicates in the code count).
 //
 // A work item is one sample, not one pixel, so that a small frame fills the
 // GPU and a large one ends without a tail of whole pixels; each sample's
 // radiance goes to a buffer that a second kernel adds up in sample order, which
 // rounds as one pixel's samples rendered in turn. Images are the lock-step
 // form's bit for bit. Measured on one B200, lock-step -> streaming: 1024x1024
-// room, 64 samples 145.0 -> 95.8 ms; 960x540, 16 samples of 10,000 instances
-// 64.3 -> 37.1 ms; 400x225, 16 samples of random spheres 1.86 -> 1.22 ms; one
+// room, 64 samples 145.0 -> 94.4 ms; 960x540, 16 samples of 10,000 instances
+// 64.3 -> 35.9 ms; 400x225, 16 samples of random spheres 1.86 -> 1.22 ms; one
 // such row of 400 pixels 0.71 -> 0.16 ms.
 //
 // Five resident blocks per SM (96 registers; 4: room 13% slower), four for
 // the forms with more live state, auxiliary outputs (1080p room, 4 samples:
-// 10.0 ms, 5 blocks 11.1) and extended light sampling (8.5 ms, 5 blocks 8.9).
+// 10.0 ms, 5 blocks 11.1) and extended light sampling (8.5 ms, 5 blocks 8.9; 7.1 with one copy of its draws).
 // Fetch and node thresholds are flat optima (4..12, 8..12: within 2%).
 #pragma once
 #include "path.cuh"
@@ -65,6 +66,72 @@ struct SampleAt {
     uint32_t sample, scene, place;
 };
 
+// The context a lane walks for, and its hit: in registers until the walk is
+// done, or (IN_CONTEXT) a path ray's straight in its context's words. In
+// registers the plain forms are faster (room frame 1%, instances 2.6%), in the
+// context the forms with more live state (a batch 4.5%, guides 1.3%).
+template <int C, bool INST, bool IN_CONTEXT>
+struct WalkHit;
+
+template <int C, bool INST>
+struct WalkHit<C, INST, false> : HitRegs {
+    uint32_t (*ctx)[C];
+    int c;
+    bool shadow;
+    __device__ __forceinline__ void start(V o_, V d_) {
+        o = o_;
+        d = d_;
+    }
+    __device__ __forceinline__ bool is_blocked() const { return h.kind != PT_HIT_NONE; }
+    __device__ __forceinline__ void keep() const {
+        ctx[C_SD + 1][c] = __float_as_uint(h.u);
+        ctx[C_SD + 2][c] = __float_as_uint(h.v);
+        ctx[C_ST][c] = h.kind;
+        ctx[C_SV][c] = h.index;
+        if (INST) ctx[C_SV + 1][c] = h.inst;
+    }
+};
+
+template <int C, bool INST>
+struct WalkHit<C, INST, true> {
+    uint32_t (*ctx)[C];
+    int c;
+    bool shadow, blocked;
+    __device__ __forceinline__ V get(int f) const {
+        return mk(__uint_as_float(ctx[f][c]), __uint_as_float(ctx[f + 1][c]), __uint_as_float(ctx[f + 2][c]));
+    }
+    __device__ __forceinline__ void start(V, V) {}
+    __device__ __forceinline__ bool is_blocked() const { return blocked; }
+    __device__ __forceinline__ void keep() const {}
+    __device__ __forceinline__ void world(V& wo, V& wd) const {
+        wo = get(C_O);
+        wd = get(shadow ? C_SD : C_D);
+    }
+    __device__ __forceinline__ void clear(uint32_t kind, uint32_t index) {
+        blocked = kind != PT_HIT_NONE;
+        if (!shadow) {
+            set(kind, index, 0);
+            set_uv(0, 0);
+        }
+    }
+    __device__ __forceinline__ void set(uint32_t kind, uint32_t index, uint32_t inst) {
+        blocked = true;
+        if (shadow) return;
+        ctx[C_ST][c] = kind;
+        ctx[C_SV][c] = index;
+        if (INST) ctx[C_SV + 1][c] = inst;
+    }
+    __device__ __forceinline__ void set_uv(float u, float v) {
+        if (shadow) return;
+        ctx[C_SD + 1][c] = __float_as_uint(u);
+        ctx[C_SD + 2][c] = __float_as_uint(v);
+    }
+    __device__ __forceinline__ void drop() {
+        blocked = false;
+        if (!shadow) ctx[C_ST][c] = PT_HIT_NONE;
+    }
+};
+
 // Frame: what is rendered -- its items, scenes, cameras and buffers.
 template <bool AUX, bool INST, bool TEX, bool EXT, class Frame>
 __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamBlocks)
@@ -97,13 +164,17 @@ __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamB
     __syncwarp();
     // queue heads and lengths, the same in every lane
     int ray_h = 0, ray_n = 0, shade_h = 0, shade_n = contexts;
-    unsigned long long rays = 0;
-    bool overflow = false, shadow = false;
-    int state = WALK_DONE, c = -1;  // c: the context this lane walks for
+    uint32_t rays = 0;
+    bool overflow = false;
+    int state = WALK_DONE;
+    WalkHit<C, INST, AUX || EXT || Frame::kManyScenes> hit;
+    hit.ctx = ctx;
+    hit.shadow = false;
+    int& c = hit.c;  // the context this lane walks for
+    c = -1;
     uint32_t walk_scene = 0;
     Walk<INST> w;
     w.top = 0;
-    w.h.kind = PT_HIT_NONE;
 
     while (true) {
         const unsigned walking = __ballot_sync(ALL, state != WALK_DONE);
@@ -143,17 +214,19 @@ __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamB
                 h.inst = INST ? ctx[C_SV + 1][k] : 0u;
                 h.u = getf(C_SD + 1, k);
                 h.v = getf(C_SD + 2, k);
-                const bool hit = h.kind != PT_HIT_NONE;
+                const bool found = h.kind != PT_HIT_NONE;
                 Rec rec;
                 const uint32_t sc = scene_of(k);
                 const PtSceneDev& S = F.scene(sc);
-                if (hit) fill<TEX, EXT>(S, h, path.o, path.d, getf(C_SD, k), rec);
+                if (found) fill<TEX, EXT>(S, h, path.o, path.d, getf(C_SD, k), rec);
                 First first;
                 const bool primary = AUX && path.bounce == 0;
                 bool nee;
                 Shadow sh;
-                const bool done =
-                    shade<AUX, TEX, EXT>(S, path, hit, rec, F.depth(sc), smp, rng, first, nee, sh, rays) == STEP_DONE;
+                unsigned long long shadow_rays = 0;
+                const bool done = shade<AUX, TEX, EXT>(S, path, found, rec, F.depth(sc), smp, rng, first, nee, sh,
+                                                       shadow_rays) == STEP_DONE;
+                rays += uint32_t(shadow_rays);
                 if (primary) {  // the first hit's guides
                     float* g = F.guides() + 6 * size_t(ctx[C_ITEM][k]);
                     g[0] = first.albedo.x;
@@ -259,19 +332,15 @@ __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamB
             if ((full | (ray_n ? done : 0u)) && (__popc(full | (ray_n ? done : 0u)) >= kFetch || done == ALL)) {
                 bool go = false, hand = false;
                 if (state == WALK_DONE && c >= 0) {
-                    if (shadow) {
-                        if (w.h.kind == PT_HIT_NONE) setv(C_RAD, c, getv(C_RAD, c) + getv(C_SV, c));
+                    if (hit.shadow) {
+                        if (!hit.is_blocked()) setv(C_RAD, c, getv(C_RAD, c) + getv(C_SV, c));
                         const uint32_t flags = ctx[C_FLAGS][c] & ~CF_SHADOW;
                         ctx[C_FLAGS][c] = flags;
                         hand = (flags & CF_ENDED) != 0;
                         go = !hand;
                     } else {
                         setf(C_SD, c, w.t_max);
-                        setf(C_SD + 1, c, w.h.u);
-                        setf(C_SD + 2, c, w.h.v);
-                        ctx[C_ST][c] = w.h.kind;
-                        ctx[C_SV][c] = w.h.index;
-                        if (INST) ctx[C_SV + 1][c] = w.h.inst;
+                        hit.keep();
                         hand = true;
                     }
                 }
@@ -294,11 +363,15 @@ __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamB
                 ray_n -= got;
                 __syncwarp();
                 if (go) {
-                    shadow = (ctx[C_FLAGS][c] & CF_SHADOW) != 0;
+                    const bool shadow = (ctx[C_FLAGS][c] & CF_SHADOW) != 0;
+                    const V d = getv(shadow ? C_SD : C_D, c);
+                    const float t = shadow ? getf(C_ST, c) : 1000.0f;
+                    hit.shadow = shadow;
                     if (!shadow) ++rays;
                     walk_scene = scene_of(c);
-                    state = w.begin(F.scene(walk_scene), getv(C_O, c), getv(shadow ? C_SD : C_D, c), 0.001f,
-                                    shadow ? getf(C_ST, c) : 1000.0f, shadow, stack);
+                    const V o = getv(C_O, c);
+                    hit.start(o, d);
+                    state = w.begin(F.scene(walk_scene), o, d, 0.001f, t, shadow, stack, hit);
                 }
             }
         }
@@ -315,9 +388,9 @@ __global__ void __launch_bounds__(128, AUX || EXT ? kStreamBlocks - 1 : kStreamB
             } else if (ray_n > 0 && __popc(__ballot_sync(ALL, state == WALK_DONE)) >= kFetch) {
                 break;
             }
-            if (state == AT_NODE) state = w.expand(F.scene(walk_scene), 0.001f, stack, overflow);
+            if (state == AT_NODE) state = w.expand(F.scene(walk_scene), 0.001f, stack, hit, overflow);
         }
-        if (state == AT_LEAF) state = w.leaf(F.scene(walk_scene), 0.001f, shadow, stack, overflow);
+        if (state == AT_LEAF) state = w.leaf(F.scene(walk_scene), 0.001f, hit.shadow, stack, hit, overflow);
     }
 
     unsigned long long total = rays;

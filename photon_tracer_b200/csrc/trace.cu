@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(128) trace_any_kernel(PtSceneDev S, const floa
 // (warps)-th run of 32 rays, and its lanes take their next rays as they
 // finish. Issue- and latency-bound: 1M random rays in the room scene take 106
 // warp instructions per ray at 14.5 threads each, the lock-step kernel above
-// 199 at 5.6. On one B200 (identical hits): 4M such rays 1,087 -> 630 us, 1M
-// rays among instances 335 -> 204 us, 1M rays among 488 spheres 93 -> 84 us.
+// 199 at 5.6. On one B200 (identical hits): 4M such rays 1,087 -> 607 us, 1M
+// rays among instances 335 -> 197 us, 1M rays among 488 spheres 93 -> 84 us.
 // Six resident blocks per SM, one wave of them (5: 686 us, four waves of
 // short-lived warps: 703 us); refills at 8 idle lanes and node phases while
 // 12 lanes stand at nodes are flat optima (4..16 lanes: within 2%).
@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(128, kStreamBlocks)
     const size_t warps = size_t(gridDim.x) * 4, warp = blockIdx.x * size_t(4) + (threadIdx.x >> 5);
     constexpr unsigned ALL = 0xffffffffu;
     Walk<INST> w;
+    HitRegs hit;
     w.top = 0;
     int state = WALK_DONE;
     size_t ray = n;      // the lane's ray; n: none
@@ -109,26 +110,25 @@ __global__ void __launch_bounds__(128, kStreamBlocks)
             if (state == WALK_DONE) {
                 if (ray < n) {
                     if (ANY) {
-                        occ[ray] = w.h.kind != PT_HIT_NONE ? 1 : 0;
+                        occ[ray] = hit.h.kind != PT_HIT_NONE ? 1 : 0;
                     } else {
                         uint32_t index, sub;
-                        resolve(S, w.h, index, sub);
+                        resolve(S, hit.h, index, sub);
                         pt_hit out;
-                        out.kind = w.h.kind;
-                        out.index = w.h.kind == PT_HIT_NONE ? 0u : index;
+                        out.kind = hit.h.kind;
+                        out.index = hit.h.kind == PT_HIT_NONE ? 0u : index;
                         out.sub = sub;
                         out.t = w.t_max;
-                        out.u = w.h.u;
-                        out.v = w.h.v;
+                        out.u = hit.h.u;
+                        out.v = hit.h.v;
                         hits[ray] = out;
                     }
                 }
                 const size_t k = next + __popc(idle & ((1u << lane) - 1u));
                 ray = ((k >> 5) * warps + warp) * 32 + (k & 31);
                 if (ray < n) {
-                    V o, d;
-                    load_ray(rays, ray, o, d);
-                    state = w.begin(S, o, d, tmin, tmax, ANY, stack);
+                    load_ray(rays, ray, hit.o, hit.d);
+                    state = w.begin(S, hit.o, hit.d, tmin, tmax, ANY, stack, hit);
                 } else {
                     ray = n;
                 }
@@ -144,9 +144,9 @@ __global__ void __launch_bounds__(128, kStreamBlocks)
                 const unsigned done = __ballot_sync(ALL, state == WALK_DONE);
                 if ((nodes | done) != ALL || (more && __popc(done) >= kStreamFetch)) break;
             }
-            if (state == AT_NODE) state = w.expand(S, tmin, stack, overflow);
+            if (state == AT_NODE) state = w.expand(S, tmin, stack, hit, overflow);
         }
-        if (state == AT_LEAF) state = w.leaf(S, tmin, ANY, stack, overflow);
+        if (state == AT_LEAF) state = w.leaf(S, tmin, ANY, stack, hit, overflow);
     }
     if (__any_sync(ALL, overflow) && lane == 0) atomicOr(S.status, PT_DEV_ERR_STACK);
 }

@@ -1221,13 +1221,19 @@ __device__ __forceinline__ V refract(V uv, V n, float ratio) {
 // real stream, but an all-zero xoshiro state (which a caller could supply
 // as a snapshot) repeats (-1,-1,-1) forever; the bound turns that into a
 // zero offset instead of a hung kernel.
+template <bool SMALL = false>  // one copy of the draw in the code, in a loop
 __device__ __forceinline__ V random_in_unit_sphere(Rng& rng) {
 #pragma unroll 1
     for (int tries = 0; tries < 64; ++tries) {
-        const float z = -1.0f + 2.0f * rng.real();
-        const float y = -1.0f + 2.0f * rng.real();
-        const float x = -1.0f + 2.0f * rng.real();
-        const V p = mk(x, y, z);
+        V p = mk(0, 0, 0);
+        if (SMALL) {
+#pragma unroll 1
+            for (int k = 0; k < 3; ++k) p = mk(-1.0f + 2.0f * rng.real(), p.x, p.y);
+        } else {
+            p.z = -1.0f + 2.0f * rng.real();
+            p.y = -1.0f + 2.0f * rng.real();
+            p.x = -1.0f + 2.0f * rng.real();
+        }
         if (dot(p, p) >= 1) continue;
         return p;
     }
@@ -1235,7 +1241,9 @@ __device__ __forceinline__ V random_in_unit_sphere(Rng& rng) {
 }
 
 // material::scatter for the four kinds: lambertian :59-74, metal :85-91,
-// diffuse_light :97-102, dielectric :113-136.
+// diffuse_light :97-102, dielectric :113-136. SMALL: d_in is normalized
+// already, and the code is kept small.
+template <bool SMALL = false>
 __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_in, const Rec& rec,
                                         const Sampler& smp, Rng& rng, V& attenuation, V& dir) {
     if (type == PT_MAT_LAMBERTIAN) {
@@ -1254,8 +1262,8 @@ __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_
         return true;
     }
     if (type == PT_MAT_METAL) {
-        const V reflected = reflect(normalize(d_in), rec.normal);
-        dir = reflected + random_in_unit_sphere(rng) * m.emission_fuzz.w;
+        const V reflected = reflect(SMALL ? d_in : normalize(d_in), rec.normal);
+        dir = reflected + random_in_unit_sphere<SMALL>(rng) * m.emission_fuzz.w;
         attenuation = xyz(m.albedo_type);
         return dot(dir, rec.normal) > 0;
     }
@@ -1263,7 +1271,7 @@ __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_
         attenuation = mk(1, 1, 1);
         const float ior = m.ior_flags.x;
         const float ratio = rec.front_face ? (1 / ior) : ior;
-        const V unit = normalize(d_in);
+        const V unit = SMALL ? d_in : normalize(d_in);
         const float cos_theta = fminf(dot(-unit, rec.normal), 1.0f);
         const float sin_theta = sqrtf(1 - cos_theta * cos_theta);
         const bool cannot_refract = ratio * sin_theta > 1;
