@@ -174,7 +174,15 @@ unet::ConvOut to_cat(pt_unet* n, int l, int up) {
 // its 2x2-pooled output and its copy into the decoder's concatenation; each
 // decoder level's last convolution (and the bottleneck's) writes its
 // upsampled output into the next finer concatenation.
-cudaError_t forward(pt_unet* n, cudaStream_t st, bool training) {
+// image: where to put the image_w x image_h radiance directly (inference with
+// tensor cores; *imaged tells whether that happened, else act[15] holds the
+// output).
+struct ImageOut {
+    float* image;
+    int w, h;
+    bool imaged;
+};
+cudaError_t forward(pt_unet* n, cudaStream_t st, bool training, ImageOut* image = nullptr) {
     cudaError_t e;
     auto A = [&](int i) { return n->act[i].p; };
     const bool drop = !training;
@@ -183,15 +191,15 @@ cudaError_t forward(pt_unet* n, cudaStream_t st, bool training) {
     TRY(conv(n, 0, A(0), A(1), false, {}, false, st));
     unet::ConvOut o = to_cat(n, 0, 0);
     o.pool = n->pool[0].as<__nv_bfloat16>();
-    TRY(conv(n, 1, A(1), A(2), false, o, false, st));
+    TRY(conv(n, 1, A(1), A(2), false, o, drop, st));
     TRY(conv(n, 2, n->pool[0].p, A(3), false, {}, false, st));
     o = to_cat(n, 1, 0);
     o.pool = n->pool[1].as<__nv_bfloat16>();
-    TRY(conv(n, 3, A(3), A(4), false, o, false, st));
+    TRY(conv(n, 3, A(3), A(4), false, o, drop, st));
     TRY(conv(n, 4, n->pool[1].p, A(5), false, {}, false, st));
     o = to_cat(n, 2, 0);
     o.pool = n->pool[2].as<__nv_bfloat16>();
-    TRY(conv(n, 5, A(5), A(6), false, o, false, st));
+    TRY(conv(n, 5, A(5), A(6), false, o, drop, st));
     TRY(conv(n, 6, n->pool[2].p, A(7), false, {}, false, st));
     TRY(conv(n, 7, A(7), A(8), false, to_cat(n, 2, 1), drop, st));  // level 2: [up(a7) 128 | a5 96]
     TRY(conv(n, 8, n->cat[2].p, A(9), false, {}, false, st));
@@ -200,6 +208,21 @@ cudaError_t forward(pt_unet* n, cudaStream_t st, bool training) {
     TRY(conv(n, 11, A(11), A(12), false, to_cat(n, 0, 1), drop, st));  // level 0: [up(a11) 64 | a1 32]
     TRY(conv(n, 12, n->cat[0].p, A(13), false, {}, false, st));
     TRY(conv(n, 13, A(13), A(14), false, {}, false, st));
+    if (image) image->imaged = false;
+    if (image && n->use_tc) {
+        const LayerDef& L = kLayers[14];
+        const unet::ConvShape s{n->B, n->H, n->W, L.cin, L.cout};
+        unet::ConvOut im;
+        im.image = image->image;
+        im.image_w = image->w;
+        im.image_h = image->h;
+        e = unet::conv_fwd_tc(s, static_cast<const __nv_bfloat16*>(A(14)), w16(n, 14), bias(n, 14), L.relu, im, false,
+                              n->status.as<unsigned int>(), st);
+        if (e != cudaErrorNotSupported) {
+            image->imaged = true;
+            return e;
+        }
+    }
     TRY(conv(n, 14, A(14), A(15), true, {}, false, st));
     return cudaSuccess;
 }
@@ -498,8 +521,9 @@ pt_status pt_unet_forward(pt_unet* n, int B, int H, int W, const float* d_input,
     cudaError_t e = ensure_workspace(n, B, H, W);
     const long px = long(B) * H * W;
     if (!e) e = unet::make_input(px, d_input, n->act[0].as<__nv_bfloat16>(), 32, st);
-    if (!e) e = forward(n, st, false);
-    if (!e) e = unet::make_output(px, kOutStride, n->act[15].as<float>(), d_output, st);
+    ImageOut im{d_output, W, H, false};
+    if (!e) e = forward(n, st, false, &im);
+    if (!e && !im.imaged) e = unet::make_output(px, kOutStride, n->act[15].as<float>(), d_output, st);
     return e ? cuda_fail(e, "pt_unet_forward") : PT_OK;
 }
 
@@ -576,8 +600,9 @@ pt_status pt_denoise_unet(pt_unet* n, int width, int height, const float* d_colo
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     cudaError_t e = ensure_workspace(n, 1, Hp, Wp);
     if (!e) e = unet::frame_input(width, height, Wp, Hp, d_color, d_aux, d_depth, n->act[0].as<__nv_bfloat16>(), 32, st);
-    if (!e) e = forward(n, st, false);
-    if (!e) e = unet::frame_output(width, height, Wp, kOutStride, n->act[15].as<float>(), d_out, st);
+    ImageOut im{d_out, width, height, false};
+    if (!e) e = forward(n, st, false, &im);
+    if (!e && !im.imaged) e = unet::frame_output(width, height, Wp, kOutStride, n->act[15].as<float>(), d_out, st);
     return e ? cuda_fail(e, "pt_denoise_unet") : PT_OK;
 }
 

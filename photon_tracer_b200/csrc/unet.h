@@ -85,6 +85,11 @@ struct ConvOut {
     // colsum (Cout floats). bf16 output, Cout a multiple of 32.
     const __nv_bfloat16* mask = nullptr;
     float* colsum = nullptr;
+    // The network's last layer: the first three channels as radiance, 3
+    // floats per pixel of an image of image_w x image_h per batch entry (the
+    // part of the padded frame that the caller asked for).
+    float* image = nullptr;
+    int image_w = 0, image_h = 0;
 };
 
 // Tensor-core forward convolution (tcgen05, accumulators in TMEM). Returns

@@ -202,7 +202,10 @@ struct TileGrid {
 // TMEM (columns from 0 and from half the allocation, a power of two >= 2N)
 // let the epilogue of one tile overlap the MMAs of the next; the TMA
 // producer runs ahead across tile boundaries.
-template <bool OUT_F32, bool HALO, bool MASK>
+// What the epilogue does with the sums (ConvOut): activations, a masked
+// gradient, or the image.
+enum Epilogue : int { EPI_STORE = 0, EPI_MASK = 1, EPI_IMAGE = 2 };
+template <bool OUT_F32, bool HALO, int EPI>
 __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                            const __grid_constant__ CUtensorMap tm_w, int B, int H,
                                                            int W, int Cin, int N, int tmem_cols, int stages,
@@ -258,6 +261,7 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
     // shared-memory broadcasts.
     __shared__ float sbias[kMaxN];
     for (int i = threadIdx.x; i < N; i += kThreads) sbias[i] = bias ? bias[i] : 0.0f;
+    constexpr bool MASK = EPI == EPI_MASK;
     // Backward: each epilogue warp's column sums (a warp's own row, so no
     // conflicts between warps).
     __shared__ float scol[4][MASK ? kMaxN : 1];
@@ -389,6 +393,16 @@ __global__ void __launch_bounds__(kThreads) conv_tc_kernel(const __grid_constant
               tmem_ld16_async(acc_addr + uint32_t(c0), r[0]);
               if (c0 + 16 < N) tmem_ld16_async(acc_addr + uint32_t(c0 + 16), r[1]);
               tmem_wait();
+              if (EPI == EPI_IMAGE) {
+                  // log(1 + radiance) in the first three columns
+                  if (c0 == 0 && valid && px < o.image_w && py < o.image_h) {
+                      float* dst = o.image + 3 * ((size_t(b) * o.image_h + py) * o.image_w + px);
+#pragma unroll
+                      for (int j = 0; j < 3; ++j)
+                          dst[j] = fmaxf(expm1f(__uint_as_float(r[0][j]) + sbias[j]), 0.0f);
+                  }
+                  continue;
+              }
               if (MASK) {
                   // the gradient at an activation: zero where its ReLU was
                   // (mask <= 0), stored as bf16, its column sums kept
@@ -740,7 +754,8 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
     if (out_f32 && (o.out2 || o.pool)) return cudaErrorNotSupported;
     if (reinterpret_cast<uintptr_t>(o.out2) % 16 || (size_t(o.offset2) * 2) % 16 || (size_t(o.stride2) * 2) % 16)
         return cudaErrorNotSupported;
-    const bool mask = o.mask != nullptr;
+    const bool mask = o.mask != nullptr, image = o.image != nullptr;
+    if (image && (out_f32 || mask || relu || o.out || o.out2 || o.pool)) return cudaErrorNotSupported;
     if (mask && (out_f32 || !o.colsum || !o.out || o.out2 || o.pool || bias || relu || N % 32 || o.stride != N ||
                  o.offset || reinterpret_cast<uintptr_t>(o.mask) % 16))
         return cudaErrorNotSupported;
@@ -794,29 +809,33 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
     const int tx = halo ? kHaloTX : kTileX, ty = halo ? kHaloTY : kTileY;
     const long tiles = long((s.W + tx - 1) / tx) * ((s.H + ty - 1) / ty) * s.B;
     if (tiles > 0x7fffffffL) return cudaErrorNotSupported;
-    const void* fn = mask      ? (halo ? reinterpret_cast<const void*>(conv_tc_kernel<false, true, true>)
-                                       : reinterpret_cast<const void*>(conv_tc_kernel<false, false, true>))
-                     : out_f32 ? (halo ? reinterpret_cast<const void*>(conv_tc_kernel<true, true, false>)
-                                       : reinterpret_cast<const void*>(conv_tc_kernel<true, false, false>))
-                               : (halo ? reinterpret_cast<const void*>(conv_tc_kernel<false, true, false>)
-                                       : reinterpret_cast<const void*>(conv_tc_kernel<false, false, false>));
+#define PT_CONV_FN(F32, EPI)                                                  \
+    (halo ? reinterpret_cast<const void*>(conv_tc_kernel<F32, true, EPI>)     \
+          : reinterpret_cast<const void*>(conv_tc_kernel<F32, false, EPI>))
+    const void* fn = mask      ? PT_CONV_FN(false, EPI_MASK)
+                     : image   ? PT_CONV_FN(false, EPI_IMAGE)
+                     : out_f32 ? PT_CONV_FN(true, EPI_STORE)
+                               : PT_CONV_FN(false, EPI_STORE);
+#undef PT_CONV_FN
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e) return e;
     const long g = grid_size(cols, smem, fn);
     const unsigned blocks = unsigned(tiles < g ? tiles : g);
-#define PT_CONV_LAUNCH(F32, MASK)                                                                                    \
-    (halo ? conv_tc_kernel<F32, true, MASK><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N, cols, \
+#define PT_CONV_LAUNCH(F32, EPI)                                                                                     \
+    (halo ? conv_tc_kernel<F32, true, EPI><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N, cols, \
                                                                            stages, plan.res ? 1 : 0, bias, relu, o,  \
                                                                            status)                                   \
-          : conv_tc_kernel<F32, false, MASK><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N,     \
+          : conv_tc_kernel<F32, false, EPI><<<blocks, kThreads, smem, st>>>(tm_in, tm_w, s.B, s.H, s.W, s.Cin, N,     \
                                                                             cols, stages, plan.res ? 1 : 0, bias,    \
                                                                             relu, o, status))
     if (mask)
-        PT_CONV_LAUNCH(false, true);
+        PT_CONV_LAUNCH(false, EPI_MASK);
+    else if (image)
+        PT_CONV_LAUNCH(false, EPI_IMAGE);
     else if (out_f32)
-        PT_CONV_LAUNCH(true, false);
+        PT_CONV_LAUNCH(true, EPI_STORE);
     else
-        PT_CONV_LAUNCH(false, false);
+        PT_CONV_LAUNCH(false, EPI_STORE);
 #undef PT_CONV_LAUNCH
     return cudaGetLastError();
 }
