@@ -346,7 +346,7 @@ cudaError_t loss_backward_tc(pt_unet* n, const float* target, bool input_grad, c
         unet::ConvOut o;
         o.out = fgrad ? static_cast<void*>(fgrad) : other;
         o.stride = L.cin;
-        if (!fgrad) {
+        if (!fgrad && l > 0) {
             o.mask = bf(l);
             o.colsum = db(l - 1);
         }

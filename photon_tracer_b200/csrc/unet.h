@@ -99,9 +99,9 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
                         bool relu, const ConvOut& o, bool out_f32, unsigned int* status, cudaStream_t st);
 
 // Tensor-core weight gradient (tcgen05, MN-major operands): dw += d loss /
-// d w from the layer input and the bf16 gradient of its output (Cout <= 128,
-// Cin <= 256, both multiples of 8), float atomics. cudaErrorNotSupported for
-// other shapes, which then run on conv_wgrad.
+// d w from the layer input and the bf16 gradient of its output (Cout <= 128, a
+// multiple of 8, Cin a multiple of 32), float atomics. cudaErrorNotSupported
+// for other shapes, which then run on conv_wgrad.
 cudaError_t conv_wgrad_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw,
                           unsigned int* status, cudaStream_t st);
 

@@ -465,9 +465,12 @@ __global__ void __launch_bounds__(256) l1_back_kernel(long pixels, const float* 
     if (threadIdx.x == 3) atomicAdd(loss, part[3]);
 }
 
-// One thread: one pixel, 16 of the 32 channels. The sum runs over taps, then
-// channels, as conv_fwd's does; the gradient's channels past the third are
-// zero and add nothing.
+// One thread: one pixel, all 32 channels, so that a weight is one shared-memory
+// broadcast for the warp. The sum runs over taps, then channels, as
+// conv_fwd's does, product and sum rounded one after the other (packed f32x2
+// operations gave other sums here, which moved bf16 roundings); the gradient's
+// channels past the third are zero and add nothing. Two threads per pixel, which read two weights per warp, took 112
+// us at 16 x 128 x 128; this takes 45.
 __global__ void __launch_bounds__(256) last_back_kernel(int B, int H, int W, const float4* __restrict__ g4,
                                                         const __nv_bfloat16* __restrict__ wt,
                                                         const __nv_bfloat16* __restrict__ y,
@@ -479,24 +482,26 @@ __global__ void __launch_bounds__(256) last_back_kernel(int B, int H, int W, con
         reinterpret_cast<float*>(ws)[i] = __bfloat162float(wt[(ci * 9 + tap) * 16 + c]);
     }
     __syncthreads();
-    const int half = threadIdx.x & 1;
-    float sum[2][8] = {{0, 0, 0, 0, 0, 0, 0, 0}, {0, 0, 0, 0, 0, 0, 0, 0}};
-    const long P = long(B) * H * W;
-    for (long p = (blockIdx.x * long(blockDim.x) + threadIdx.x) >> 1; p < P; p += (long(gridDim.x) * blockDim.x) >> 1) {
-        const int x = int(p % W), yy = int((p / W) % H);
-        float acc[2][8];
+    float sum[4][8];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) acc[i >> 3][i & 7] = 0.0f;
+    for (int i = 0; i < 32; ++i) sum[i >> 3][i & 7] = 0.0f;
+    const int P = B * H * W;
+    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
+        const int x = p % W, yy = (p / W) % H;
+        float acc[4][8];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i >> 3][i & 7] = 0.0f;
+#pragma unroll 1
         for (int tap = 0; tap < 9; ++tap) {
             const int dy = tap / 3 - 1, dx = tap % 3 - 1;
             if (yy + dy < 0 || yy + dy >= H || x + dx < 0 || x + dx >= W) continue;
-            const float4 g = __ldg(g4 + p + long(dy) * W + dx);
+            const float4 g = __ldg(g4 + p + dy * W + dx);
             const float gc[3] = {g.x, g.y, g.z};
 #pragma unroll
             for (int c = 0; c < 3; ++c)
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 w = ws[tap * 3 + c][4 * half + j];
+                for (int j = 0; j < 8; ++j) {
+                    const float4 w = ws[tap * 3 + c][j];
                     float* a = &acc[j >> 1][4 * (j & 1)];
                     a[0] += gc[c] * w.x;
                     a[1] += gc[c] * w.y;
@@ -505,14 +510,21 @@ __global__ void __launch_bounds__(256) last_back_kernel(int B, int H, int W, con
                 }
         }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const size_t at = 32 * size_t(p) + 16 * half + 8 * j;
+        for (int j = 0; j < 4; ++j) {
+            const size_t at = 32 * size_t(p) + 8 * j;
             finish8(acc[j], load_bf8(y + at), g16 + at, sum[j]);
         }
     }
-    add_sums(part, 32, 2 * half, true, sum[0], db);
+    if (threadIdx.x < 32) part[threadIdx.x] = 0.0f;
     __syncthreads();
-    add_sums(part, 32, 2 * half + 1, true, sum[1], db);
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        float s = sum[i >> 3][i & 7];
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+        if ((threadIdx.x & 31) == 0) atomicAdd(part + i, s);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) atomicAdd(db + threadIdx.x, part[threadIdx.x]);
 }
 
 __global__ void __launch_bounds__(256) up_back_kernel(int B, int h, int w, int C, const float* __restrict__ gcat,
@@ -738,7 +750,7 @@ cudaError_t l1_back(long pixels, const float* pred, const float* target, float4*
 
 cudaError_t last_back(int B, int H, int W, const float4* g4, const __nv_bfloat16* wt, const __nv_bfloat16* y,
                       __nv_bfloat16* g16, float* db, cudaStream_t st) {
-    last_back_kernel<<<back_grid(long(B) * H * W, 128), 256, 0, st>>>(B, H, W, g4, wt, y, g16, db);
+    last_back_kernel<<<back_grid(long(B) * H * W, 256), 256, 0, st>>>(B, H, W, g4, wt, y, g16, db);
     return cudaGetLastError();
 }
 

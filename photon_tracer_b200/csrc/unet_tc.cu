@@ -147,21 +147,8 @@ __device__ __forceinline__ void mma_commit(uint32_t bar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// 16 consecutive accumulator columns of this thread's TMEM lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t addr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(addr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-// The same load without the wait: several may be in flight before one
+// 16 consecutive accumulator columns of this thread's TMEM lane, without
+// waiting: several may be in flight before one
 // tmem_wait(), and their registers are read only after it.
 __device__ __forceinline__ void tmem_ld16_async(uint32_t addr, uint32_t (&r)[16]) {
     asm volatile(
@@ -599,46 +586,63 @@ int grid_size(int cols, size_t smem, const void* fn) {
 }
 
 // ---- weight gradient -------------------------------------------------------
-// dW[co][tap][ci] = sum over pixels p of dY[p][co] * X[p + offset(tap)][ci]:
-// per tap a GEMM with M = Cout (padded to 128), N = Cin (padded to a
-// multiple of 64), K = pixels. A K step is a 16 x 4 pixel box: dY unshifted
-// and X shifted by the tap (zeros outside the image), both channel-contiguous
-// -- MN-major operands, 128-byte swizzle, one 64-channel TMA box per 64
-// rows of M or N. A CTA reduces one tap over a range of pixel boxes in TMEM
-// and adds its partial sums to dW with float atomics.
-constexpr int kWgBoxX = 16, kWgBoxY = 4, kWgK = kWgBoxX * kWgBoxY;  // 64 pixels per K step
-constexpr int kWgStages = 4;
-constexpr uint32_t kWgBox = kWgK * 64 * 2;  // one 64-channel box: 8 KB
+// dW[co][tap][ci] = sum over pixels p of dY[p][co] * X[p + offset(tap)][ci]: a
+// GEMM with M = Cout (padded to 128), N = 32 input channels, K = pixels, for
+// each of the nine taps. A CTA takes 32 input channels and a range of 8 x 16
+// pixel tiles, and keeps all nine taps' sums in TMEM (288 columns): a tile's
+// dY and the 10 x 18 halo of X are loaded once, as planes of 8 channels (16
+// bytes per pixel), and a tap's operand is the halo seen from its offset. Both
+// are MN-major without swizzle: 8 pixels x 8 channels per core matrix, the next
+// 8 pixels one tile row on, the next 8 channels one plane on. The sums are
+// added to dW with vector float atomics.
+//
+// Bound by the tensor pipe's reads of the 4 KB dY operand per 128 x 32 x 16
+// step. One CTA per tap, which loaded dY and a shifted X nine times and read
+// them with the 128-byte swizzle, took 990 us for the 15 layers of a 16 x 128 x
+// 128 batch; this takes 537.
+constexpr int kWgStages = 4, kWgTaps = 9, kWgN = 32;
+constexpr uint32_t kWgPlane = kHaloTX * kHaloTY * 16;  // 2,048 bytes: 8 channels of dY
+constexpr uint32_t kWgA = 16 * kWgPlane;               // what an M = 128 operand spans
+constexpr int kWgCols = 512;                           // 9 x 32 columns, a power of two
 
-// UMMA descriptor of an MN-major operand with the 128-byte swizzle: 64
-// elements of M or N per 128-byte row, one row per K index; 8-row groups
-// 1024 bytes apart (stride byte offset), 64-element blocks of M or N one
-// 8 KB box apart (leading byte offset), descriptor version 1.
-__device__ __forceinline__ uint64_t mn_sw128_desc(uint32_t addr) {
-    return uint64_t((addr >> 4) & 0x3fff) | (uint64_t(kWgBox >> 4) << 16) | (uint64_t(1024 >> 4) << 32) |
-           (uint64_t(1) << 46) | (uint64_t(2) << 61);
+// UMMA descriptor of an MN-major operand without swizzle: `lbo` bytes between
+// groups of 8 K indices, `sbo` bytes between groups of 8 rows of M or N.
+__device__ __forceinline__ uint64_t mn_plain_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+    return plain_desc(addr, lbo, sbo);
+}
+
+__device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+}
+
+size_t wgrad_smem(int Cout) {
+    const size_t stage = size_t(Cout / 8) * kWgPlane + kHaloBytes;
+    // The last stage's operand may reach past its planes (rows of M beyond Cout, never read).
+    return 1024 + kWgStages * stage + (stage < kWgA ? kWgA - stage : 0) + (2 * kWgStages + 1) * 8 + 8;
 }
 
 __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constant__ CUtensorMap tm_dy,
                                                             const __grid_constant__ CUtensorMap tm_x, int B, int H,
-                                                            int W, int Cin, int Cout, int N, int tmem_cols, int splits,
+                                                            int W, int Cin, int Cout, int splits,
                                                             float* __restrict__ dw, unsigned int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    const int nb = N / 64;  // X boxes per stage
-    const uint32_t stage_bytes = (2 + nb) * kWgBox;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWgStages * stage_bytes);  // full[S], empty[S], done
+    const uint32_t dy_bytes = uint32_t(Cout / 8) * kWgPlane, stage_bytes = dy_bytes + kHaloBytes;
+    const uint32_t pad = stage_bytes < kWgA ? kWgA - stage_bytes : 0;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWgStages * stage_bytes + pad);  // full[S], empty[S], done
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * kWgStages + 1);
     volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + kWgStages), done = smem_u32(bars + 2 * kWgStages);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int tap = blockIdx.x % 9, split = blockIdx.x / 9;
-    const int bx = (W + kWgBoxX - 1) / kWgBoxX, by = (H + kWgBoxY - 1) / kWgBoxY;
-    const long boxes = long(bx) * by * B;
-    const long k0 = boxes * split / splits, k1 = boxes * (split + 1) / splits;
-    const int iters = int(k1 - k0);
-    const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+    const int chunk = blockIdx.x / splits, split = blockIdx.x % splits;
+    TileGrid grid;
+    grid.tx = kHaloTX;
+    grid.ty = kHaloTY;
+    grid.tiles_x = (W + kHaloTX - 1) / kHaloTX;
+    grid.tiles_y = (H + kHaloTY - 1) / kHaloTY;
+    grid.n = grid.tiles_x * grid.tiles_y * B;
+    const int t0 = int(long(grid.n) * split / splits), iters = int(long(grid.n) * (split + 1) / splits) - t0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kWgStages; ++s) {
@@ -651,7 +655,7 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                     "r"(tmem_cols)
+                     "r"(kWgCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -672,15 +676,12 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
                     ok = false;
                     break;
                 }
-                long k = k0 + it;
-                const int x0 = int(k % bx) * kWgBoxX;
-                k /= bx;
-                const int y0 = int(k % by) * kWgBoxY, b = int(k / by);
+                int x0, y0, b;
+                grid.origin(t0 + it, x0, y0, b);
                 const uint32_t st = smem_u32(smem + s * stage_bytes), bar = full0 + 8 * s;
                 bar_expect_tx(bar, stage_bytes);
-                tma_load_4d(st, &tm_dy, 0, x0, y0, b, bar);
-                tma_load_4d(st + kWgBox, &tm_dy, 64, x0, y0, b, bar);
-                for (int j = 0; j < nb; ++j) tma_load_4d(st + (2 + j) * kWgBox, &tm_x, 64 * j, x0 + dx, y0 + dy, b, bar);
+                tma_load_5d(st, &tm_dy, 0, x0, y0, 0, b, bar);
+                tma_load_5d(st + dy_bytes, &tm_x, 0, x0 - 1, y0 - 1, chunk * (kWgN / 8), b, bar);
             }
             for (int k = it > kWgStages ? it - kWgStages : 0; k < it; ++k)
                 if (!wait_bar(full0 + 8 * (k % kWgStages), (k / kWgStages) & 1, nullptr)) ok = false;
@@ -690,7 +691,7 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
             // kind::f16: f32 accumulate, A and B bf16, both MN-major (bits 15,
             // 16), N >> 3 at bit 17, M = 128 >> 4 at bit 24.
             const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
-                                   (uint32_t(N >> 3) << 17) | (uint32_t(128 >> 4) << 24);
+                                   (uint32_t(kWgN >> 3) << 17) | (uint32_t(128 >> 4) << 24);
             for (int it = 0; it < iters; ++it) {
                 const int s = it % kWgStages;
                 if (!wait_bar(full0 + 8 * s, (it / kWgStages) & 1, abort)) {
@@ -698,12 +699,15 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
                     break;
                 }
                 fence_after();
-                const uint32_t st = smem_u32(smem + s * stage_bytes);
-                const uint64_t ad = mn_sw128_desc(st), bd = mn_sw128_desc(st + 2 * kWgBox);
+                const uint32_t st = smem_u32(smem + s * stage_bytes), sx = st + dy_bytes;
+                for (int r = 0; r < kHaloTY; r += 2) {  // K = 16: two rows of 8 pixels
+                    const uint64_t ad = mn_plain_desc(st + r * (kHaloTX * 16), kHaloTX * 16, kWgPlane);
 #pragma unroll
-                for (int k = 0; k < kWgK / 16; ++k)  // K = 16 rows = two 1024-byte groups per MMA
-                    mma_bf16(tmem, ad + uint64_t(k * (2048 >> 4)), bd + uint64_t(k * (2048 >> 4)), idesc,
-                             (it | k) != 0);
+                    for (int tap = 0; tap < kWgTaps; ++tap)
+                        mma_bf16(tmem + tap * kWgN, ad,
+                                 mn_plain_desc(sx + ((r + tap / 3) * kHaloW + tap % 3) * 16, kHaloW * 16, kPlane), idesc,
+                                 (it | r) != 0);
+                }
                 mma_commit(empty0 + 8 * s);
             }
             mma_commit(done);
@@ -713,15 +717,20 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
         const int co = q * 32 + lane;
         if (iters > 0 && __all_sync(0xffffffffu, wait_bar(done, 0, abort))) {
             fence_after();
-            for (int c = 0; c < N; c += 16) {
-                float v[16];
-                tmem_ld16(tmem + (uint32_t(q * 32) << 16) + uint32_t(c), v);
-                if (co >= Cout) continue;
-                float* dst = dw + (size_t(co) * 9 + tap) * Cin + c;
+            if (q * 32 < Cout)
+                for (int tap = 0; tap < kWgTaps; ++tap) {
+                    uint32_t r[2][16];
+                    const uint32_t at = tmem + (uint32_t(q * 32) << 16) + uint32_t(tap * kWgN);
+                    tmem_ld16_async(at, r[0]);
+                    tmem_ld16_async(at + 16, r[1]);
+                    tmem_wait();
+                    if (co >= Cout) continue;
+                    float* dst = dw + (size_t(co) * kWgTaps + tap) * Cin + chunk * kWgN;
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (c + j < Cin) atomicAdd(dst + j, v[j]);
-            }
+                    for (int j = 0; j < 32; j += 4)
+                        red_add4(dst + j, __uint_as_float(r[j >> 4][j & 15]), __uint_as_float(r[j >> 4][(j & 15) + 1]),
+                                 __uint_as_float(r[j >> 4][(j & 15) + 2]), __uint_as_float(r[j >> 4][(j & 15) + 3]));
+                }
         } else if (iters > 0) {
             ok = false;
         }
@@ -735,8 +744,21 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
     __syncthreads();
     if (warp == 1) {
         fence_after();
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(tmem_cols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kWgCols) : "memory");
     }
+}
+
+// [B][H][W][C] seen as (8 channels, x, y, channel group, image), boxes of
+// bw x bh pixels and `groups` channel groups.
+bool plane_map(PFN_cuTensorMapEncodeTiled_v12000 encode, CUtensorMap* map, const __nv_bfloat16* p, int B, int H, int W,
+               int C, int bw, int bh, int groups) {
+    const cuuint64_t dims[5] = {8, cuuint64_t(W), cuuint64_t(H), cuuint64_t(C / 8), cuuint64_t(B)};
+    const cuuint64_t strides[4] = {cuuint64_t(C) * 2, cuuint64_t(W) * C * 2, 16, cuuint64_t(H) * W * C * 2};
+    const cuuint32_t box[5] = {8, cuuint32_t(bw), cuuint32_t(bh), cuuint32_t(groups), 1};
+    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(p), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace
@@ -768,18 +790,7 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
     // tensor map is refused.
     bool halo = N <= PT_CONV_HALO_MAX_N;
     CUtensorMap tm_in, tm_w;
-    if (halo) {
-        // [B][H][W][Cin] seen as (8 channels, x, y, channel group, image): the
-        // box (8, 10, 18, 4, 1) lands as four 8-channel planes of the halo.
-        const cuuint64_t dims[5] = {8, cuuint64_t(s.W), cuuint64_t(s.H), cuuint64_t(s.Cin / 8), cuuint64_t(s.B)};
-        const cuuint64_t strides[4] = {cuuint64_t(s.Cin) * 2, cuuint64_t(s.W) * s.Cin * 2, 16,
-                                       cuuint64_t(s.H) * s.W * s.Cin * 2};
-        const cuuint32_t box[5] = {8, kHaloW, kHaloH, 4, 1};
-        const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-        halo = encode(&tm_in, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16*>(in), dims, strides, box,
-                      estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-    }
+    if (halo) halo = plane_map(encode, &tm_in, in, s.B, s.H, s.W, s.Cin, kHaloW, kHaloH, 4);  // 32 channels of the halo
     if (!halo) {
         const cuuint64_t dims[4] = {cuuint64_t(s.Cin), cuuint64_t(s.W), cuuint64_t(s.H), cuuint64_t(s.B)};
         const cuuint64_t strides[3] = {cuuint64_t(s.Cin) * 2, cuuint64_t(s.W) * s.Cin * 2,
@@ -842,46 +853,28 @@ cudaError_t conv_fwd_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_
 
 cudaError_t conv_wgrad_tc(const ConvShape& s, const __nv_bfloat16* in, const __nv_bfloat16* dout, float* dw,
                           unsigned int* status, cudaStream_t st) {
-    const int N = (s.Cin + 63) / 64 * 64;
-    if (s.Cout > 128 || s.Cout % 8 || s.Cin % 8 || N > 256 || s.B < 1 || s.H < 1 || s.W < 1)
+    if (s.Cout > 128 || s.Cout < 8 || s.Cout % 8 || s.Cin % kWgN || s.Cin < kWgN || s.B < 1 || s.H < 1 || s.W < 1)
         return cudaErrorNotSupported;
-    if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(dout)) % 16) return cudaErrorNotSupported;
+    if ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dw)) % 16)
+        return cudaErrorNotSupported;
     PFN_cuTensorMapEncodeTiled_v12000 encode = encode_fn();
     if (!encode) return cudaErrorNotSupported;
     CUtensorMap tm_dy, tm_x;
-    const cuuint32_t box[4] = {64, kWgBoxX, kWgBoxY, 1};
-    const cuuint32_t estr[4] = {1, 1, 1, 1};
-    {
-        const cuuint64_t dims[4] = {cuuint64_t(s.Cout), cuuint64_t(s.W), cuuint64_t(s.H), cuuint64_t(s.B)};
-        const cuuint64_t strides[3] = {cuuint64_t(s.Cout) * 2, cuuint64_t(s.W) * s.Cout * 2,
-                                       cuuint64_t(s.H) * s.W * s.Cout * 2};
-        if (encode(&tm_dy, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(dout), dims, strides, box,
-                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorNotSupported;
-    }
-    {
-        const cuuint64_t dims[4] = {cuuint64_t(s.Cin), cuuint64_t(s.W), cuuint64_t(s.H), cuuint64_t(s.B)};
-        const cuuint64_t strides[3] = {cuuint64_t(s.Cin) * 2, cuuint64_t(s.W) * s.Cin * 2,
-                                       cuuint64_t(s.H) * s.W * s.Cin * 2};
-        if (encode(&tm_x, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16*>(in), dims, strides, box,
-                   estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-            return cudaErrorNotSupported;
-    }
-    int cols = 32;
-    while (cols < N) cols *= 2;
-    const size_t smem = 1024 + kWgStages * size_t(2 + N / 64) * kWgBox + (2 * kWgStages + 1) * 8 + 8;
+    if (!plane_map(encode, &tm_dy, dout, s.B, s.H, s.W, s.Cout, kHaloTX, kHaloTY, s.Cout / 8) ||
+        !plane_map(encode, &tm_x, in, s.B, s.H, s.W, s.Cin, kHaloW, kHaloH, kWgN / 8))
+        return cudaErrorNotSupported;
+    const size_t smem = wgrad_smem(s.Cout);
     cudaError_t e = cudaFuncSetAttribute(wgrad_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     if (e) return e;
-    const long boxes = long((s.W + kWgBoxX - 1) / kWgBoxX) * ((s.H + kWgBoxY - 1) / kWgBoxY) * s.B;
-    // About two CTAs per SM over the 9 taps, at least 8 boxes each.
-    const int target = grid_size(cols, smem, reinterpret_cast<const void*>(wgrad_tc_kernel));
-    long splits = (2L * target + 8) / 9;
-    if (splits > boxes / 8) splits = boxes / 8;
-    if (splits < 1) splits = 1;
-    wgrad_tc_kernel<<<unsigned(9 * splits), kThreads, smem, st>>>(tm_dy, tm_x, s.B, s.H, s.W, s.Cin, s.Cout, N, cols,
-                                                                 int(splits), dw, status);
+    const long tiles = long((s.W + kHaloTX - 1) / kHaloTX) * ((s.H + kHaloTY - 1) / kHaloTY) * s.B;
+    if (tiles > 0x7fffffffL) return cudaErrorNotSupported;
+    // One CTA per SM (each takes all of TMEM): the channel chunks, times as
+    // many ranges of tiles as fill the SMs.
+    const int chunks = s.Cin / kWgN;
+    const int sms = grid_size(kWgCols, smem, reinterpret_cast<const void*>(wgrad_tc_kernel));
+    const long splits = std::max(1L, std::min(tiles, long(sms / chunks)));
+    wgrad_tc_kernel<<<unsigned(chunks * splits), kThreads, smem, st>>>(tm_dy, tm_x, s.B, s.H, s.W, s.Cin, s.Cout,
+                                                                      int(splits), dw, status);
     return cudaGetLastError();
 }
 
