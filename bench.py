@@ -111,6 +111,17 @@ class ClockSampler:
                 "samples": len(sm)}
 
 
+def frame_launches(mode) -> int:
+    """Kernels of the library in one frame: the megakernel renders as many
+    samples per launch as a 256 MB buffer of radiances holds, and a second
+    kernel adds them to the frame (the wavefront's own count is left at one)."""
+    from photon_tracer_b200 import abi
+    if mode != abi.PT_MODE_MEGAKERNEL:
+        return 1
+    per_launch = max(1, (256 << 20) // (12 * WIDTH * HEIGHT))
+    return 2 * -(-SPP // per_launch)
+
+
 def bytes_per_ray(desc, cam, width=WIDTH, height=HEIGHT, spp=SPP):
     """Algorithmic bytes per counted ray from the CPU oracle's traversal
     counters on a bounded sample of the frame (8 rows at `spp`)."""
@@ -795,7 +806,7 @@ def main():
             "convergence": conv,
             "batch": batch,
             "cpu_baseline": cpu,
-            "gpu_launches": args.steps,
+            "gpu_launches": args.steps * frame_launches(mode),
             "clocks": clocks.summary(),
             "wall_s_timed_region": round(t_wall, 3),
         }

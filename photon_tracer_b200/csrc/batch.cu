@@ -1,5 +1,7 @@
-// Batched rendering: many scenes of different size, resolution and spp in one
-// persistent launch over one node arena.
+// Batched rendering: many scenes of different size, resolution and spp over one
+// node arena, in one persistent lock-step launch or, for batches of enough
+// samples (batch.cpp), with the streaming form (stream_mega.cuh) at the end of
+// this file.
 //
 // The scenes' arenas are merged on the host with every index rebased
 // (batch.cpp), so the arena pointers are shared and a scene differs only by

@@ -1,6 +1,8 @@
-// Persistent-thread megakernel path tracer.
+// Persistent-thread megakernel path tracer: the lock-step form, and the frames
+// and sums of the streaming form (stream_mega.cuh), which renders whatever
+// api.cpp's streams() sends there.
 //
-// The CPU renderer gives each thread a whole scanline, taken from an atomic
+// The lock-step form. The CPU renderer gives each thread a whole scanline, taken from an atomic
 // row counter (src/main.cpp:137-158), and runs samples_per_pixel paths per
 // pixel one after another (include/renderer.hpp:366-409). Here each LANE owns
 // a pixel, runs its samples one path after another (so the per-pixel sums
