@@ -100,30 +100,36 @@ int act_level(int i) { return i == 0 ? 0 : i == 15 ? 0 : kLayers[i - 1].level; }
 
 cudaError_t ensure_workspace(pt_unet* n, int B, int H, int W) {
     if (B == n->B && H == n->H && W == n->W) return cudaSuccess;
-    n->B = B;
-    n->H = H;
-    n->W = W;
+    // The shape is kept only once every buffer is there: after a failed
+    // allocation no later call may take the buffers for a workspace.
+    n->B = n->H = n->W = 0;
+    auto px_at = [&](int level) { return size_t(B) * (H >> level) * (W >> level); };
     cudaError_t e = cudaSuccess;
     for (int i = 0; i < 16 && !e; ++i) {
-        const size_t px = size_t(pixels_at(n, act_level(i))), c = size_t(act_channels(i));
+        const size_t px = px_at(act_level(i)), c = size_t(act_channels(i));
         e = n->act[i].ensure(px * c * (i == 15 ? 4 : 2));
         if (!e) e = n->gact[i].ensure(px * c * 4);
     }
     size_t g16_elems = 0;
     for (int i = 1; i < 15; ++i) {
-        const size_t c = size_t(pixels_at(n, act_level(i))) * act_channels(i);
+        const size_t c = px_at(act_level(i)) * act_channels(i);
         g16_elems = c > g16_elems ? c : g16_elems;
     }
     if (!e) e = n->g16.ensure(g16_elems * 2);
     if (!e) e = n->g16b.ensure(g16_elems * 2);
-    if (!e) e = n->g4.ensure(size_t(pixels_at(n, 0)) * 16);
+    if (!e) e = n->g4.ensure(px_at(0) * 16);
     const int pool_c[3] = {32, 64, 96}, cat_c[3] = {96, 160, 224};
     for (int l = 0; l < 3 && !e; ++l) {
-        const size_t pp = size_t(pixels_at(n, l + 1)), pc = size_t(pixels_at(n, l));
+        const size_t pp = px_at(l + 1), pc = px_at(l);
         e = n->pool[l].ensure(pp * pool_c[l] * 2);
         if (!e) e = n->gpool[l].ensure(pp * pool_c[l] * 4);
         if (!e) e = n->cat[l].ensure(pc * cat_c[l] * 2);
         if (!e) e = n->gcat[l].ensure(pc * cat_c[l] * 4);
+    }
+    if (!e) {
+        n->B = B;
+        n->H = H;
+        n->W = W;
     }
     return e;
 }
