@@ -279,12 +279,15 @@ pt_status pt_render(pt_scene* scene, const pt_camera* cam, const pt_settings* se
  * for the legacy default stream) without synchronising. d_rays (may be NULL)
  * is one device uint64 that the ray count is ADDED to. settings->rng_states
  * must be a device pointer. Kernel-side errors (stack overflow, timeouts)
- * are reported by the next pt_sync(). A frame of several samples per pixel
- * renders through a buffer of its samples (12 bytes each, 36 with aux, at
- * most 256 MB at a time or one sample per pixel) that the scene allocates at
- * its first such frame, keeps, grows and frees when it is destroyed; without
- * memory for it, and under stream capture, frames render without it, the same
- * image more slowly. */
+ * are reported by the next pt_sync(). Renders of one scene may be enqueued on
+ * several streams; captured ones (below) and wavefront renders must be ordered
+ * with the scene's other renders of those kinds by the caller. A frame of
+ * several samples per pixel renders through a buffer of its samples (12 bytes
+ * each, 36 with aux, at most 256 MB at a time or one sample per pixel), taken
+ * from a memory pool of the device and given back in stream order; the pool
+ * keeps up to 512 MB for later renders of any scene and goes with the device's
+ * last scene. Without memory for the buffer, and under stream capture, frames
+ * render without it, the same image more slowly. */
 pt_status pt_render_device(pt_scene* scene, const pt_camera* cam, const pt_settings* settings, float* d_out,
                            float* d_aux, uint64_t* d_rays, void* stream);
 

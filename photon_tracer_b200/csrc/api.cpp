@@ -12,6 +12,7 @@
 #include <string>
 
 #include "kernels.h"
+#include "pool.h"
 #include "wavefront.h"
 #include "scene_host.hpp"
 
@@ -66,12 +67,10 @@ struct pt_scene {
     int sms = 148;
     void* arena = nullptr;
     unsigned int* status = nullptr;    // device error word
-    unsigned int* work = nullptr;      // megakernel work counter
+    unsigned int* work = nullptr;      // work counter of renders that borrow none (RenderMemory)
     unsigned long long* rays = nullptr;
     cudaStream_t stream = nullptr;
-    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum, samples;
-    float* lent = nullptr;            // a batch's buffer of samples, used instead of `samples`
-    size_t lent_bytes = 0;
+    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum;
     uint32_t* host_counts = nullptr;  // pinned, for the wavefront queue read-back
     int blocks_per_sm[6] = {0, 0, 0, 0, 0, 0};  // megakernel forms: aux, snapshot; extended light sampling
     uint32_t wave_slots = 0;                   // wavefront path-queue capacity; 0: kMaxWaveSlots
@@ -175,62 +174,75 @@ bool streams(const pt_scene* s, const PtRenderParams& p) {
     return p.spp > 3 || s->dev.tree_kib > 64;
 }
 
-// Samples per pixel of one streaming launch, as many as the scene's sample
-// buffer of at most kSampleBytes holds (more launches each wait for their last
-// paths: a 1024x1024 frame of 64 samples takes 4); 0 when the frame has to be
-// rendered without a buffer: under stream capture, where a graph would keep
-// its address, or when there is no memory for it.
+// Samples per pixel of one streaming launch, as many as kSampleBytes hold
+// (more launches each wait for their last paths: a 1024x1024 frame of 64
+// samples takes 4); 0 for a frame too large for a buffer of one each.
 constexpr size_t kSampleBytes = size_t(256) << 20;
 
-int samples_per_launch(pt_scene* s, const PtRenderParams& p, cudaStream_t stream) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
-        cudaGetLastError();
-        return 0;
-    }
+int samples_per_launch(const PtRenderParams& p) {
     const size_t one = pt_sample_bytes(p);
-    const size_t most = std::max<size_t>(1, (s->lent ? s->lent_bytes : kSampleBytes) / one);
+    if (one > 4 * kSampleBytes) return 0;
+    const size_t most = std::max<size_t>(1, kSampleBytes / one);
     const int launches = int((size_t(p.spp) + most - 1) / most);
-    const int count = (p.spp + launches - 1) / launches;
-    if (s->lent) return one <= s->lent_bytes ? count : 0;
-    // growing the buffer must not disturb a capture on another stream
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const bool ok = one <= 4 * kSampleBytes && s->samples.ensure(one * size_t(count), "samples") == PT_OK;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    if (!ok) {
-        clear_error();
-        cudaGetLastError();
-        return 0;
+    return (p.spp + launches - 1) / launches;
+}
+
+// The device memory of one render: its work counter, then its samples,
+// borrowed from the device's pool for as long as its launches need it.
+constexpr size_t kCounterBytes = 256;
+
+struct RenderMemory {
+    void* ptr = nullptr;
+    cudaStream_t stream = nullptr;
+    bool borrow(pt_scene* s, size_t bytes, cudaStream_t st) {  // false without memory for it
+        stream = st;
+        return pool_borrow(s->device, &ptr, bytes, st) == cudaSuccess;
     }
-    return count;
+    ~RenderMemory() { pool_return(ptr, stream); }
+};
+
+bool is_capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool none =
+        cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
+    if (!none) cudaGetLastError();
+    return !none;
 }
 
 pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t stream) {
     if (mode == PT_MODE_WAVEFRONT) {
         const uint64_t px = uint64_t(p.width) * uint64_t(p.rows);
-        const uint32_t cap = s->wave_slots ? s->wave_slots : kMaxWaveSlots;
-        const uint32_t slots = uint32_t(px < cap ? px : cap);
-        if (pt_status e = s->wave.ensure(pt_wavefront_bytes(slots), "wavefront state")) return e;
-        if (!s->host_counts)
-            if (cudaError_t e = cudaMallocHost(&s->host_counts, 256)) return cuda_fail(e, "wavefront counters");
+        const uint32_t most = s->wave_slots ? s->wave_slots : kMaxWaveSlots;
+        const uint32_t slots = uint32_t(std::min<uint64_t>(std::max<uint64_t>(px, 128), most));
+        if (!s->host_counts && cudaMallocHost(&s->host_counts, 4 * sizeof(uint32_t)) != cudaSuccess)
+            return fail(PT_ERR_OUT_OF_MEMORY, "wavefront: pinned counters");
+        if (pt_status e = s->wave.ensure(pt_wavefront_bytes(slots), "wavefront: path state")) return e;
         if (cudaError_t e = pt_launch_wavefront(s->dev, p, s->wave.ptr, slots, s->sms, stream, s->host_counts))
             return cuda_fail(e, "wavefront");
         return PT_OK;
     }
-    p.work = s->work;
-    if (streams(s, p)) {
-        const int count = samples_per_launch(s, p, stream);
-        for (int first = 0; count > 0 && first < p.spp; first += count) {
-            cudaError_t e = cudaMemsetAsync(s->work, 0, sizeof(unsigned int), stream);
+    // A captured render borrows nothing (a graph would keep the address): it
+    // counts in the scene's own word and takes the lock-step form, as a render
+    // without memory for its samples does.
+    RenderMemory memory;
+    int count = 0;
+    if (!is_capturing(stream)) {
+        count = streams(s, p) ? samples_per_launch(p) : 0;
+        if (count > 0 && !memory.borrow(s, kCounterBytes + pt_sample_bytes(p) * size_t(count), stream)) count = 0;
+        if (count == 0) memory.borrow(s, kCounterBytes, stream);
+    }
+    p.work = memory.ptr ? static_cast<unsigned int*>(memory.ptr) : s->work;
+    if (count > 0) {
+        float* samples = reinterpret_cast<float*>(static_cast<char*>(memory.ptr) + kCounterBytes);
+        for (int first = 0; first < p.spp; first += count) {
+            cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream);
             if (!e)
-                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first),
-                                      s->lent ? s->lent : static_cast<float*>(s->samples.ptr), s->sms, stream);
+                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first), samples, s->sms, stream);
             if (e) return cuda_fail(e, "megakernel launch");
         }
-        if (count > 0) return PT_OK;
+        return PT_OK;
     }
-    if (cudaError_t e = cudaMemsetAsync(s->work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
+    if (cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
     const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
     PtLaunchShape shape;
     shape.threads = 128;
@@ -245,11 +257,6 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
 }  // namespace
 
 void pt::set_wave_slots(pt_scene* s, uint32_t slots) { s->wave_slots = slots; }
-
-void pt::lend_samples(pt_scene* s, float* buffer, size_t bytes) {
-    s->lent = buffer;
-    s->lent_bytes = bytes;
-}
 
 namespace {
 
@@ -406,6 +413,7 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     s->info.max_depth = A.max_depth;
     s->info.stack_entries = A.stack_entries;
     s->info.device_bytes = bytes;
+    pool_join(device);
     *out = s;
     return PT_OK;
 }
@@ -423,10 +431,10 @@ pt_status pt_scene_destroy(pt_scene* s) {
     s->out_hits.release();
     s->counts.release();
     s->wave.release();
-    s->samples.release();
     if (s->host_counts) cudaFreeHost(s->host_counts);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->arena) cudaFree(s->arena);
+    pool_leave(s->device);
     delete s;
     return PT_OK;
 }

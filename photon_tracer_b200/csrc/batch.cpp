@@ -57,7 +57,7 @@ struct pt_batch {
     uint32_t total_items = 0;
     uint64_t total_pixels = 0, total_samples = 0, total_tris = 0;
     // Streaming form of the single launch: its launches' segments, and the
-    // buffer of samples, which the per-scene renders share (one at a time).
+    // buffer of samples.
     struct Launch {
         uint32_t first, n, items, pixels;
     };
@@ -573,7 +573,6 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
             pt_scene* s = nullptr;
             if (pt_status st = pt_scene_create(items[i].desc, &s)) return st;
             b->singles.push_back(s);
-            if (!b->launches.empty()) lend_samples(s, b->d_samples, b->sample_bytes);
         }
     }
     *out = guard.release();

@@ -34,9 +34,6 @@ uint32_t tree_depth(const std::vector<pt_bvh_node>& nodes, uint32_t root);
 // The path-queue capacity of a scene's wavefront renders (0: the default,
 // 2^20 paths in flight); the batch autotuner tries several.
 void set_wave_slots(pt_scene* s, uint32_t slots);
-// Renders of s use this buffer of samples (device memory that outlives s's
-// renders) instead of one of its own.
-void lend_samples(pt_scene* s, float* buffer, size_t bytes);
 
 // ---- float vector arithmetic, in the reference's evaluation order -------------------
 // (include/vec3.hpp:58-118: dot is (x*x' + y*y') + z*z', normalize divides

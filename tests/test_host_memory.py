@@ -59,3 +59,89 @@ def test_unet_after_a_failed_allocation(fake, call, sizes, tensor_cores):
         assert first == second == abi.PT_ERR_OUT_OF_MEMORY
         failures += 1
     assert failures > 10
+
+
+class DeviceScene:
+    """A generated scene whose renders go to the fake's log."""
+
+    def __init__(self, kind, param):
+        import photon_tracer_b200 as pt
+        self.g = pt.Generated(kind, seed=1, param=param)
+        self.s = pt.Scene(self.g)
+
+    def render(self, w, h, spp, stream, aux=False, mode=1):
+        st = self.s.settings(w, h, spp, 10, seed=1, mode=mode)
+        self.s.render_device(self.g.camera, st, SOME.value, SOME.value if aux else 0, 0, stream)
+
+
+def launches(lines, kind):
+    """(stream, work counter, buffer or None) of the logged megakernel launches of one form."""
+    out = []
+    for line in lines:
+        w = line.split()
+        if w[0] == kind:
+            out.append((w[1], w[3], w[5] if len(w) > 5 else None))
+    return out
+
+
+ROOM, SPHERES = 11, 10  # large enough trees to stream at any sample count from two; small ones from four
+
+
+@pytest.mark.parametrize("kind,param,spp,form", [(ROOM, 4, 4, "samples"), (SPHERES, 20, 1, "megakernel")])
+def test_renders_on_two_streams_share_nothing(fake, kind, param, spp, form):
+    """Frames of one scene enqueued on two streams, neither waited for: each has its own counter and samples until
+    its own launches are done."""
+    d = DeviceScene(kind, param)
+    fake.log()
+    a, b = 0x7000, 0x8000
+    d.render(400, 300, spp, a)
+    d.render(320, 200, spp, b)
+    lines = fake.log()
+    on_a, on_b = launches(lines, form)
+    assert (int(on_a[0], 16), int(on_b[0], 16)) == (a, b)
+    assert on_a[1] != on_b[1] and (form == "megakernel" or on_a[2] != on_b[2])
+    assert not any(line.startswith("bad") for line in lines)
+
+
+def test_a_device_render_does_not_wait(fake):
+    """Neither the first frame nor larger ones after it, nor guides, allocate or free in a way that waits for the
+    device; what a frame borrows it gives back on its own stream after its last launch."""
+    d = DeviceScene(ROOM, 4)
+    fake.log()
+    for w, h, spp, aux in ((64, 48, 4, False), (640, 360, 8, False), (1024, 1024, 24, True), (33, 17, 2, False)):
+        d.render(w, h, spp, 0x7000, aux)
+        lines = fake.log()
+        assert not [x for x in lines if x.split()[0] in ("malloc", "free", "wait", "bad")], lines
+        assert [x.split()[0] for x in lines if x.split()[0] in ("borrow", "return")] == ["borrow", "return"]
+        assert lines[-1].startswith("return") and lines[-1].endswith(" 0x7000")
+
+
+def test_scenes_hold_no_samples_between_renders(fake):
+    """Many scenes' renders leave only what the device's pool keeps, which is bounded and goes with the last scene."""
+    scenes = [DeviceScene(ROOM, 3) for _ in range(3)]
+    fake.log()
+    for d in scenes:
+        d.render(640, 360, 8, 0x7000)
+    lines = fake.log()
+    assert [x for x in lines if x.startswith("pool")] == ["pool create", f"pool keeps {512 << 20}"]
+    assert sum(x.startswith("borrow") for x in lines) == sum(x.startswith("return") for x in lines) == 3
+    for k, d in enumerate(scenes):
+        d.s.close()
+        assert ("pool destroy" in fake.log()) == (k == 2)
+
+
+def test_captured_and_memoryless_renders_borrow_no_samples(fake):
+    d = DeviceScene(ROOM, 4)
+    fake.lib.fake_capture(0x7000)
+    fake.log()
+    d.render(400, 300, 4, 0x7000)
+    fake.lib.fake_capture(None)
+    lines = fake.log()
+    assert len(launches(lines, "megakernel")) == 1 and not any(x.startswith("borrow") for x in lines)
+    with fake.failing_above(1 << 20):
+        d.render(400, 300, 4, 0x7000)
+    with fake.failing_above(0):
+        d.render(400, 300, 4, 0x7000)
+    lines = fake.log()
+    assert len(launches(lines, "megakernel")) == 2 and not launches(lines, "samples")
+    assert not any(x.startswith("bad") for x in lines)
