@@ -30,6 +30,7 @@
 
 #include "batch.h"
 #include "kernels.h"
+#include "pool.h"
 #include "scene_host.hpp"
 
 namespace pt {
@@ -57,7 +58,8 @@ struct pt_batch {
     uint32_t total_items = 0;
     uint64_t total_pixels = 0, total_samples = 0, total_tris = 0;
     // Streaming form of the single launch: its launches' segments, and the
-    // buffer of samples.
+    // buffer of samples with the segments behind it, borrowed from the device's
+    // pool for as long as the batch may run that launch.
     struct Launch {
         uint32_t first, n, items, pixels;
     };
@@ -65,7 +67,7 @@ struct pt_batch {
     std::vector<Launch> launches;
     PtBatchSegment* d_segments = nullptr;
     float* d_samples = nullptr;
-    size_t sample_bytes = 0;
+    size_t sample_bytes = 0, stream_bytes = 0;
     std::vector<pt_scene*> singles;  // per-scene scenes for the per-scene strategies
     cudaStream_t stream = nullptr;
     cudaGraphExec_t one_graph[3] = {nullptr, nullptr, nullptr};  // the single launch at 64, 128, 256 threads
@@ -280,6 +282,39 @@ void plan_stream(pt_batch* b) {
     b->sample_bytes = size_t(most) * 12;
 }
 
+// Plans the streaming launches and gets the memory they need; without it the
+// batch has none, and the lock-step form renders.
+pt_status make_stream(pt_batch* b) {
+    plan_stream(b);
+    const size_t segment_bytes = b->segments.size() * sizeof(PtBatchSegment);
+    const size_t at = align256(b->sample_bytes);
+    void* memory = nullptr;
+    if (b->sample_bytes > 4 * 12 * kBatchSamples || pool_borrow(b->device, &memory, at + segment_bytes, b->stream)) {
+        b->launches.clear();
+        return PT_OK;
+    }
+    b->d_samples = static_cast<float*>(memory);
+    b->d_segments = reinterpret_cast<PtBatchSegment*>(static_cast<char*>(memory) + at);
+    b->stream_bytes = at + segment_bytes;
+    b->arena_bytes += b->stream_bytes;
+    cudaError_t e = cudaMemcpyAsync(b->d_segments, b->segments.data(), segment_bytes, cudaMemcpyHostToDevice, b->stream);
+    if (!e) e = cudaStreamSynchronize(b->stream);
+    return e ? cuda_fail(e, "pt_batch_create: segments") : PT_OK;
+}
+
+// Gives that memory back. Nothing of the batch may be in flight.
+void drop_stream(pt_batch* b) {
+    for (cudaGraphExec_t& g : b->one_graph) {
+        if (g) cudaGraphExecDestroy(g);
+        g = nullptr;
+    }
+    pool_return(b->d_samples, b->stream);
+    b->d_samples = nullptr;
+    b->launches.clear();
+    b->arena_bytes -= b->stream_bytes;
+    b->stream_bytes = 0;
+}
+
 // Captures `body` on the batch's stream into an executable graph.
 template <class Body>
 pt_status capture(pt_batch* b, cudaGraphExec_t* exec, Body&& body) {
@@ -417,6 +452,7 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->device = device;
     b->sms = sms;
     b->strategy = strategy;
+    pool_join(device);
     HostArena all;
     uint64_t out_floats = 0;
     uint32_t items_total = 0;
@@ -552,22 +588,10 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     // memory for its buffer the lock-step form renders.
     bool depths = true;
     for (const PtBatchScene& sc : b->scenes) depths &= int(sc.depth) > 0 && int(sc.depth) <= PT_SAMPLES_MAX_DEPTH;
-    if (D.words && depths && b->total_samples >= 2 * b->total_pixels && b->total_samples >= (1u << 18)) {
-        plan_stream(b);
-        err = b->sample_bytes <= 4 * 12 * kBatchSamples ? cudaMalloc(&b->d_samples, b->sample_bytes)
-                                                        : cudaErrorMemoryAllocation;
-        if (!err) err = cudaMalloc(&b->d_segments, b->segments.size() * sizeof(PtBatchSegment));
-        if (!err) {
-            err = cudaMemcpy(b->d_segments, b->segments.data(), b->segments.size() * sizeof(PtBatchSegment),
-                             cudaMemcpyHostToDevice);
-            if (err) return cuda_fail(err, "pt_batch_create: segments");
-            b->arena_bytes += b->sample_bytes + b->segments.size() * sizeof(PtBatchSegment);
-        } else {
-            cudaGetLastError();
-            b->launches.clear();
-        }
-    }
-    // Per-scene scenes for the strategies that launch scene by scene.
+    const bool wants_stream =
+        D.words && depths && b->total_samples >= 2 * b->total_pixels && b->total_samples >= (1u << 18);
+    // Per-scene scenes for the strategies that launch scene by scene. They come
+    // before the buffer of samples, which the batch can do without.
     if (strategy != PT_BATCH_ONE_LAUNCH) {
         for (uint32_t i = 0; i < n; ++i) {
             pt_scene* s = nullptr;
@@ -575,6 +599,8 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
             b->singles.push_back(s);
         }
     }
+    if (wants_stream && (strategy == PT_BATCH_ONE_LAUNCH || strategy == PT_BATCH_AUTO))
+        if (pt_status st = make_stream(b)) return st;
     *out = guard.release();
     return PT_OK;
 }
@@ -583,8 +609,11 @@ pt_status pt_batch_render(pt_batch* b, void* stream_, uint64_t* rays_out) {
     clear_error();
     if (!b) return fail(PT_ERR_INVALID_ARG, "pt_batch_render: null batch");
     if (cudaError_t e = cudaSetDevice(b->device)) return cuda_fail(e, "cudaSetDevice");
-    if (b->strategy == PT_BATCH_AUTO && !b->tuned)
+    if (b->strategy == PT_BATCH_AUTO && !b->tuned) {
         if (pt_status st = tune(b)) return st;
+        // the single launch's memory, when scene by scene is the choice
+        if (b->strategy != PT_BATCH_ONE_LAUNCH) drop_stream(b);
+    }
     cudaStream_t stream = stream_ ? static_cast<cudaStream_t>(stream_) : b->stream;
     if (cudaError_t e = cudaMemsetAsync(b->d_rays, 0, 8, stream)) return cuda_fail(e, "pt_batch_render");
     const int strategy = b->strategy == PT_BATCH_AUTO ? PT_BATCH_ONE_LAUNCH : b->strategy;
@@ -670,16 +699,16 @@ pt_status pt_batch_destroy(pt_batch* b) {
     if (!b) return PT_OK;
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
-    for (auto g : b->one_graph)
-        if (g) cudaGraphExecDestroy(g);
+    // A render may still run on a caller's stream.
+    if (b->done_event) cudaEventSynchronize(b->done_event);
+    drop_stream(b);
     for (pt_scene* s : b->singles) pt_scene_destroy(s);
     for (cudaEvent_t e : b->scene_events) cudaEventDestroy(e);
     if (b->start_event) cudaEventDestroy(b->start_event);
     if (b->done_event) cudaEventDestroy(b->done_event);
     if (b->stream) cudaStreamDestroy(b->stream);
-    if (b->d_segments) cudaFree(b->d_segments);
-    if (b->d_samples) cudaFree(b->d_samples);
     if (b->arena) cudaFree(b->arena);
+    pool_leave(b->device);
     delete b;
     return PT_OK;
 }

@@ -23,7 +23,8 @@ namespace {
 std::map<const char*, size_t> g_live;  // allocation -> bytes
 std::string g_log;
 long g_fail_after = -1;  // allocations that still succeed; -1: all
-size_t g_fail_above = ~size_t(0);
+size_t g_fail_above = ~size_t(0), g_budget = ~size_t(0);
+bool g_falling_times = false;
 cudaStream_t g_capturing = nullptr;
 bool g_tensor_cores = true;
 long g_next = 0;
@@ -36,7 +37,9 @@ std::string hex(const void* p) {
 }
 cudaError_t allocate(void** p, size_t bytes) {
     *p = nullptr;
-    if (g_fail_after == 0 || bytes > g_fail_above) return cudaErrorMemoryAllocation;
+    size_t used = 0;
+    for (const auto& a : g_live) used += a.second;
+    if (g_fail_after == 0 || bytes > g_fail_above || used + bytes > g_budget) return cudaErrorMemoryAllocation;
     if (g_fail_after > 0) --g_fail_after;
     *p = std::malloc(bytes ? bytes : 1);
     g_live[static_cast<const char*>(*p)] = bytes;
@@ -76,6 +79,8 @@ void fake_clear() { g_log.clear(); }
 const char* fake_log() { return g_log.c_str(); }
 void fake_fail_after(long n) { g_fail_after = n; }
 void fake_fail_above(size_t bytes) { g_fail_above = bytes; }
+void fake_budget(size_t bytes) { g_budget = bytes; }
+void fake_falling_times(int on) { g_falling_times = on != 0; }
 void fake_tensor_cores(int on) { g_tensor_cores = on != 0; }
 void fake_capture(void* stream) { g_capturing = static_cast<cudaStream_t>(stream); }
 size_t fake_live_bytes() {
@@ -116,7 +121,8 @@ cudaError_t cudaMemPoolDestroy(cudaMemPool_t pool) { return delete pool, log("po
 cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t st) {
     return log("borrow " + std::to_string(n) + " " + hex(st)), allocate(p, n);
 }
-cudaError_t cudaFreeAsync(void* p, cudaStream_t st) {  // kept allocated: its stream may still be using it
+cudaError_t cudaFreeAsync(void* p, cudaStream_t st) {  // its address is not used again: its stream may still be using it
+    g_live.erase(static_cast<const char*>(p));
     return log("return " + hex(p) + " " + hex(st)), cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return std::memcpy(d, s, n), cudaSuccess; }
@@ -154,7 +160,10 @@ cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEven
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { return *ms = 1.0f, cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
+    *ms = g_falling_times ? 1.0f / float(++g_next) : 1.0f;
+    return log("timed"), cudaSuccess;
+}
 
 pt_status pt_accumulate_pass(const float*, size_t, double, double*, void*) { return PT_OK; }
 

@@ -41,6 +41,7 @@ class Fake:
         self.lib.fake_live_bytes.restype = C.c_size_t
         self.lib.fake_fail_after.argtypes = [C.c_long]
         self.lib.fake_fail_above.argtypes = [C.c_size_t]
+        self.lib.fake_budget.argtypes = [C.c_size_t]
         self.lib.fake_capture.argtypes = [C.c_void_p]
 
     def log(self):
@@ -63,3 +64,21 @@ class Fake:
             yield
         finally:
             self.lib.fake_fail_above(2**64 - 1)
+
+    @contextlib.contextmanager
+    def budget(self, n_bytes):
+        """Device memory for n_bytes in all."""
+        self.lib.fake_budget(n_bytes)
+        try:
+            yield
+        finally:
+            self.lib.fake_budget(2**64 - 1)
+
+    @contextlib.contextmanager
+    def falling_times(self):
+        """Events measure less time from call to call, so that the last of several candidates is the fastest."""
+        self.lib.fake_falling_times(1)
+        try:
+            yield
+        finally:
+            self.lib.fake_falling_times(0)

@@ -145,3 +145,80 @@ def test_captured_and_memoryless_renders_borrow_no_samples(fake):
     lines = fake.log()
     assert len(launches(lines, "megakernel")) == 2 and not launches(lines, "samples")
     assert not any(x.startswith("bad") for x in lines)
+
+
+BATCH_SAMPLES = 4 * 256 * 256 * 4 * 12  # bytes of make_batch()'s samples at least
+ONE_LAUNCH, PER_SCENE_MEGA, PER_SCENE_WAVE, AUTO = 1, 2, 3, 0
+
+
+def make_batch(strategy, side=256, spp=4, max_bounces=10):
+    """Four rooms; at the default size the single launch streams."""
+    import photon_tracer_b200 as pt
+    items = []
+    for k in range(4):
+        g = pt.Generated(ROOM, seed=k + 1, param=3)
+        items.append((g, g.camera, side, side, spp, k))
+    return pt.Batch(items, strategy, max_bounces=max_bounces)
+
+
+def one_launch_lines(fake, batch):
+    fake.log()
+    batch.render()
+    return [x for x in fake.log() if x.startswith(("batch", "bad"))]
+
+
+@pytest.mark.parametrize("strategy", [PER_SCENE_MEGA, PER_SCENE_WAVE])
+def test_per_scene_batches_hold_no_samples(fake, strategy):
+    before = fake.live_bytes()
+    b = make_batch(strategy)
+    held = b.info().device_bytes
+    assert fake.live_bytes() - before < BATCH_SAMPLES and held < BATCH_SAMPLES
+    b.close()
+    assert fake.live_bytes() == before
+
+
+def test_batch_without_memory_for_its_samples(fake):
+    """Whatever allocation fails, a batch either is refused and leaves nothing, or renders in lock step and holds no
+    samples; one that is made streams when all succeed."""
+    before, forms = fake.live_bytes(), []
+    for k in range(10):
+        fake.fail_after(k)
+        try:
+            b = make_batch(ONE_LAUNCH)
+        except Exception:
+            fake.fail_after(-1)
+            assert fake.live_bytes() == before
+            continue
+        fake.fail_after(-1)
+        forms += one_launch_lines(fake, b)
+        if forms[-1] != "batch stream":
+            assert fake.live_bytes() - before < BATCH_SAMPLES
+        b.close()
+        assert fake.live_bytes() == before
+        if forms[-1] == "batch stream":
+            break
+    assert forms == ["batch 128", "batch stream"]
+
+
+def test_batch_scenes_come_before_its_samples(fake):
+    """A batch that needs its per-scene scenes is accepted in the memory that they and its arena take."""
+    before = fake.live_bytes()
+    small = make_batch(AUTO, max_bounces=0)  # nothing to stream
+    need = fake.live_bytes() - before
+    small.close()
+    with fake.budget(before + need + BATCH_SAMPLES - 4096):
+        b = make_batch(AUTO)
+        assert one_launch_lines(fake, b)[0].split()[1] != "stream"
+    b.close()
+
+
+def test_a_tuned_batch_keeps_only_what_its_choice_needs(fake):
+    before = fake.live_bytes()
+    b = make_batch(AUTO, side=260)
+    assert fake.live_bytes() - before > BATCH_SAMPLES
+    with fake.falling_times():
+        b.render()
+    info = b.info()
+    assert info.strategy == PER_SCENE_WAVE and info.device_bytes < BATCH_SAMPLES
+    b.close()
+    assert fake.live_bytes() == before
