@@ -469,9 +469,11 @@ uint8_t pt_to_display(float linear);
 
 /* ---- batched rendering (no reference counterpart) ------------------------------ */
 /* Many scenes of different size, resolution and spp rendered together: their
- * trees share one device arena and, with PT_BATCH_ONE_LAUNCH, one persistent
- * launch (captured in a CUDA graph) covers every scene's pixels. Each scene's
- * image is what pt_render would give for it (PT_RNG_SAMPLE streams). */
+ * trees share one device arena and, with PT_BATCH_ONE_LAUNCH, one CUDA graph
+ * covers every scene's pixels: one persistent launch, or, for batches of
+ * enough samples, launches that each render as many samples as a buffer of
+ * 256 MB holds, of all scenes in turn. Each scene's image is what pt_render
+ * would give for it (PT_RNG_SAMPLE streams). */
 enum { PT_BATCH_AUTO = 0, PT_BATCH_ONE_LAUNCH = 1, PT_BATCH_PER_SCENE_MEGA = 2, PT_BATCH_PER_SCENE_WAVE = 3 };
 typedef struct pt_batch_item {
     const pt_scene_desc* desc; /* with use_bvh set */
@@ -482,10 +484,11 @@ typedef struct pt_batch_item {
 typedef struct pt_batch_info {
     uint32_t n_scenes;
     int32_t strategy;   /* the one used (the autotuner's choice for PT_BATCH_AUTO) */
-    int32_t threads;    /* block size of the single launch */
+    int32_t threads;    /* block size of the single launch (128 where samples go through the buffer) */
     int32_t tuned;
     uint64_t total_pixels, total_samples, device_bytes;
-    double tune_ms[8];  /* autotuner timings: one launch at 64/128/256 threads per block, per-scene megakernel,
+    double tune_ms[8];  /* autotuner timings: one launch at 64/128/256 threads per block (one timing for all three
+                           where samples go through the buffer), per-scene megakernel,
                            per-scene wavefront with 2^20, 2^19, 2^18 paths in flight, (unused) */
 } pt_batch_info;
 typedef struct pt_batch pt_batch;
@@ -501,7 +504,9 @@ pt_status pt_batch_render(pt_batch* batch, void* stream, uint64_t* rays_out);
 pt_status pt_batch_output(const pt_batch* batch, uint32_t i, const float** d_image);
 /* Copies scene i's image to host memory (waits for the batch). */
 pt_status pt_batch_download(pt_batch* batch, uint32_t i, float* host);
-/* Completion time of each scene in the last render, ms from its start. */
+/* Completion time of each scene in the last render, ms from its start. An
+ * image whose samples go through the buffer is complete, and its time taken,
+ * when the launch with its last samples ends: scenes of one launch share it. */
 pt_status pt_batch_scene_times(pt_batch* batch, double* ms);
 pt_status pt_batch_get_info(const pt_batch* batch, pt_batch_info* info);
 pt_status pt_batch_destroy(pt_batch* batch);

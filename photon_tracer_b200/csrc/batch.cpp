@@ -364,8 +364,10 @@ double time_ms(pt_batch* b, int strategy, int threads) {
     return st ? -double(st) : double(ms);
 }
 
+// What the autotuner's choice is remembered by: a batch that streams and one
+// of the same totals that does not are timed on their own.
 std::string shape_key(const pt_batch* b) {
-    return std::to_string(b->scenes.size()) + ":" + std::to_string(b->total_pixels) + ":" +
+    return std::string(b->launches.empty() ? "lock-step:" : "streams:") + std::to_string(b->scenes.size()) + ":" + std::to_string(b->total_pixels) + ":" +
            std::to_string(b->total_samples) + ":" + std::to_string(b->total_tris);
 }
 
@@ -382,7 +384,7 @@ pt_status tune(pt_batch* b) {
         }
     }
     // Every candidate once to warm up, then timed: the single launch at three
-    // block shapes, per-scene megakernel launches, and per-scene wavefronts
+    // block shapes (the streaming form has one), per-scene megakernel launches, and per-scene wavefronts
     // at three path-queue capacities.
     struct Cand {
         int strategy, threads;
@@ -400,6 +402,7 @@ pt_status tune(pt_batch* b) {
     std::string first_message;
     bool any = false;
     for (const Cand& c : cands) {
+        if (c.strategy == PT_BATCH_ONE_LAUNCH && c.threads != 128 && !b->launches.empty()) continue;
         b->wave_slots = c.wave_slots;
         double ms = time_ms(b, c.strategy, c.threads);
         if (ms >= 0) ms = time_ms(b, c.strategy, c.threads);
@@ -420,6 +423,7 @@ pt_status tune(pt_batch* b) {
             best_slots = c.wave_slots;
         }
     }
+    if (!b->launches.empty()) b->tune_ms[0] = b->tune_ms[2] = b->tune_ms[1];
     b->wave_slots = any ? best_slots : keep_slots;
     if (!any) return fail(first_error, first_message.c_str());
     b->tuned = true;

@@ -222,3 +222,21 @@ def test_a_tuned_batch_keeps_only_what_its_choice_needs(fake):
     assert info.strategy == PER_SCENE_WAVE and info.device_bytes < BATCH_SAMPLES
     b.close()
     assert fake.live_bytes() == before
+
+
+def test_autotuner_times_the_streaming_launch_once(fake):
+    """The streaming form has one block shape: it is captured and timed as one candidate, whose time stands for all
+    three, and its choice is not taken for a batch of the same totals that renders in lock step."""
+    b = make_batch(AUTO, side=264)
+    fake.log()
+    b.render()
+    assert fake.log().count("captured") == 1
+    info = b.info()
+    assert info.tuned and info.strategy == ONE_LAUNCH and info.threads == 128
+    assert info.tune_ms[0] == info.tune_ms[1] == info.tune_ms[2] > 0
+    b.close()
+    b = make_batch(AUTO, side=264, max_bounces=0)
+    fake.log()
+    b.render()
+    assert fake.log().count("captured") == 3 and all(ms > 0 for ms in b.info().tune_ms[:7])
+    b.close()
