@@ -72,7 +72,7 @@ struct pt_scene {
     cudaStream_t stream = nullptr;
     Scratch out, aux, states, in_rays, out_hits, counts, wave, sum;
     uint32_t* host_counts = nullptr;  // pinned, for the wavefront queue read-back
-    int blocks_per_sm[6] = {0, 0, 0, 0, 0, 0};  // megakernel forms: aux, snapshot; extended light sampling
+    int blocks_per_sm[2][6] = {};     // megakernel forms: lock-step, streaming; aux, snapshot, extended light sampling
     uint32_t wave_slots = 0;                   // wavefront path-queue capacity; 0: kMaxWaveSlots
 };
 
@@ -231,25 +231,27 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
         if (count > 0 && !memory.borrow(s, kCounterBytes + pt_sample_bytes(p) * size_t(count), stream)) count = 0;
         if (count == 0) memory.borrow(s, kCounterBytes, stream);
     }
+    const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
     p.work = memory.ptr ? static_cast<unsigned int*>(memory.ptr) : s->work;
     if (count > 0) {
         float* samples = reinterpret_cast<float*>(static_cast<char*>(memory.ptr) + kCounterBytes);
         for (int first = 0; first < p.spp; first += count) {
             cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream);
             if (!e)
-                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first), samples, s->sms, stream);
+                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first), samples, s->sms,
+                                      s->blocks_per_sm[1][variant], stream);
             if (e) return cuda_fail(e, "megakernel launch");
         }
         return PT_OK;
     }
     if (cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
-    const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
     PtLaunchShape shape;
     shape.threads = 128;
-    if (!s->blocks_per_sm[variant])
-        s->blocks_per_sm[variant] = pt_megakernel_blocks_per_sm(s->dev, shape.threads, p.aux != nullptr,
-                                                                p.rng_mode == PT_RNG_SNAPSHOT, p.nee_ext != 0);
-    shape.blocks = s->sms * s->blocks_per_sm[variant];
+    int& per_sm = s->blocks_per_sm[0][variant];
+    if (!per_sm)
+        per_sm = pt_megakernel_blocks_per_sm(s->dev, shape.threads, p.aux != nullptr, p.rng_mode == PT_RNG_SNAPSHOT,
+                                             p.nee_ext != 0);
+    shape.blocks = s->sms * per_sm;
     if (cudaError_t e = pt_launch_megakernel(s->dev, p, shape, stream)) return cuda_fail(e, "megakernel launch");
     return PT_OK;
 }

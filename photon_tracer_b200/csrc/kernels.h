@@ -43,9 +43,11 @@ int pt_megakernel_blocks_per_sm(const PtSceneDev& scene, int threads, bool aux, 
 // sample's radiance into `buffer`, then added to the pixels' running sums in
 // p.out / p.aux in sample order (scaled after the last one). buffer holds
 // count * pt_sample_bytes(p) bytes, at most 2^32 - 1 samples. p.work zeroed.
+// blocks_per_sm: the caller's, for frames of this scene with p's aux, rng_mode
+// and nee_ext; worked out by the first launch, 0 until then.
 size_t pt_sample_bytes(const PtRenderParams& p);
 cudaError_t pt_launch_samples(const PtSceneDev& scene, const PtRenderParams& p, int first, int count, float* buffer,
-                              int sms, cudaStream_t stream);
+                              int sms, int& blocks_per_sm, cudaStream_t stream);
 
 // Ray queries: closest hit (pt_hit records), any hit (bytes), and traversal
 // work counters (5 x u64, added to).

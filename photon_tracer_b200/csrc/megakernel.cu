@@ -395,31 +395,30 @@ __global__ void __launch_bounds__(256) sum_samples(PtRenderParams P, PtSampleLau
 }
 
 template <bool AUX, bool SNAP, bool INST, bool TEX, bool EXT>
-cudaError_t launch_s(const PtSceneDev& S, const PtRenderParams& p, PtSampleLaunch L, int sms, cudaStream_t stream) {
-    static int blocks_per_sm = 0;
-    int per_sm = blocks_per_sm;
-    if (!per_sm)
-        blocks_per_sm = per_sm = pt_resident_blocks(
+cudaError_t launch_s(const PtSceneDev& S, const PtRenderParams& p, PtSampleLaunch L, int sms, int& blocks_per_sm,
+                     cudaStream_t stream) {
+    if (!blocks_per_sm)
+        blocks_per_sm = pt_resident_blocks(
             reinterpret_cast<const void*>(megakernel_stream<AUX, INST, TEX, EXT, OneFrame<SNAP>>), 128, 0);
-    const uint32_t warps = uint32_t(sms * per_sm) * 4u;
+    const uint32_t warps = uint32_t(sms * blocks_per_sm) * 4u;
     L.contexts = int((L.items + warps - 1) / warps);
-    megakernel_stream<AUX, INST, TEX, EXT, OneFrame<SNAP>><<<sms * per_sm, 128, 0, stream>>>({S, p, L});
+    megakernel_stream<AUX, INST, TEX, EXT, OneFrame<SNAP>><<<sms * blocks_per_sm, 128, 0, stream>>>({S, p, L});
     sum_samples<AUX><<<(L.pixels + 255) / 256, 256, 0, stream>>>(p, L);
     return cudaGetLastError();
 }
 
 template <bool INST, bool TEX>
 cudaError_t launch_stream(const PtSceneDev& S, const PtRenderParams& p, const PtSampleLaunch& L, int sms,
-                          cudaStream_t stream) {
+                          int& per_sm, cudaStream_t stream) {
     const bool aux = p.aux != nullptr, snap = p.rng_mode == 1;
     if (p.nee_ext)  // production streams only (the host refuses it with snapshots)
-        return aux ? launch_s<true, false, INST, TEX, true>(S, p, L, sms, stream)
-                   : launch_s<false, false, INST, TEX, true>(S, p, L, sms, stream);
+        return aux ? launch_s<true, false, INST, TEX, true>(S, p, L, sms, per_sm, stream)
+                   : launch_s<false, false, INST, TEX, true>(S, p, L, sms, per_sm, stream);
     if (aux)
-        return snap ? launch_s<true, true, INST, TEX, false>(S, p, L, sms, stream)
-                    : launch_s<true, false, INST, TEX, false>(S, p, L, sms, stream);
-    return snap ? launch_s<false, true, INST, TEX, false>(S, p, L, sms, stream)
-                : launch_s<false, false, INST, TEX, false>(S, p, L, sms, stream);
+        return snap ? launch_s<true, true, INST, TEX, false>(S, p, L, sms, per_sm, stream)
+                    : launch_s<true, false, INST, TEX, false>(S, p, L, sms, per_sm, stream);
+    return snap ? launch_s<false, true, INST, TEX, false>(S, p, L, sms, per_sm, stream)
+                : launch_s<false, false, INST, TEX, false>(S, p, L, sms, per_sm, stream);
 }
 
 template <bool AUX, bool SNAP, int TREES, bool TEX, bool EXT>
@@ -498,7 +497,7 @@ size_t pt_sample_bytes(const PtRenderParams& p) {
 }
 
 cudaError_t pt_launch_samples(const PtSceneDev& S, const PtRenderParams& p, int first, int count, float* buffer, int sms,
-                              cudaStream_t stream) {
+                              int& per_sm, cudaStream_t stream) {
     PtSampleLaunch L{};
     L.tile_h = p.rows >= 4 ? 4 : 1;
     L.tile_w = 32 / L.tile_h;
@@ -511,6 +510,6 @@ cudaError_t pt_launch_samples(const PtSceneDev& S, const PtRenderParams& p, int 
     L.guides = p.aux ? buffer + 3 * size_t(L.items) : nullptr;
     const bool flat = flat_only(S);
     if (S.has_textures)
-        return flat ? launch_stream<false, true>(S, p, L, sms, stream) : launch_stream<true, true>(S, p, L, sms, stream);
-    return flat ? launch_stream<false, false>(S, p, L, sms, stream) : launch_stream<true, false>(S, p, L, sms, stream);
+        return flat ? launch_stream<false, true>(S, p, L, sms, per_sm, stream) : launch_stream<true, true>(S, p, L, sms, per_sm, stream);
+    return flat ? launch_stream<false, false>(S, p, L, sms, per_sm, stream) : launch_stream<true, false>(S, p, L, sms, per_sm, stream);
 }

@@ -183,7 +183,11 @@ cudaError_t pt_launch_megakernel(const PtSceneDev&, const PtRenderParams& p, con
 int pt_megakernel_blocks_per_sm(const PtSceneDev&, int, bool, bool, bool) { return 4; }
 size_t pt_sample_bytes(const PtRenderParams& p) { return size_t(p.width) * p.rows * (p.aux ? 36 : 12); }
 cudaError_t pt_launch_samples(const PtSceneDev&, const PtRenderParams& p, int, int count, float* buffer, int,
-                              cudaStream_t st) {
+                              int& blocks_per_sm, cudaStream_t st) {
+    if (!blocks_per_sm) {
+        log("blocks worked out");
+        blocks_per_sm = 5;
+    }
     return launch("samples " + hex(st) + " work " + hex(p.work) + " buffer " + hex(buffer),
                   {{p.work, 4}, {buffer, pt_sample_bytes(p) * size_t(count)}});
 }

@@ -240,3 +240,13 @@ def test_autotuner_times_the_streaming_launch_once(fake):
     b.render()
     assert fake.log().count("captured") == 3 and all(ms > 0 for ms in b.info().tune_ms[:7])
     b.close()
+
+
+def test_each_scene_keeps_its_own_launch_shapes(fake):
+    """What a launch works out once belongs to its scene and form, as scenes may be on other devices and rendered by
+    other threads."""
+    a, b = DeviceScene(ROOM, 3), DeviceScene(ROOM, 3)
+    fake.log()
+    for d, aux, new in ((a, False, 1), (a, False, 0), (a, True, 1), (b, False, 1), (a, True, 0), (b, False, 0)):
+        d.render(320, 200, 4, 0x7000, aux)
+        assert fake.log().count("blocks worked out") == new
