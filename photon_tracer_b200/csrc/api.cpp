@@ -341,7 +341,7 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     if (!s) return fail(PT_ERR_OUT_OF_MEMORY, "pt_scene_create: out of host memory");
     s->device = device;
     s->sms = sms;
-    const size_t bytes = 2 * align256(A.nodes.size() * 4) + align256(A.slots.size() * 4) + align256(A.islots.size() * 4) +
+    size_t bytes = align256(A.nodes.size() * 4) + align256(A.slots.size() * 4) + align256(A.islots.size() * 4) +
                          align256(A.large.size() * sizeof(float4)) + align256(A.large_mat.size() * 4) +
                          align256(A.sph.size() * sizeof(PtShadeSphere)) + align256(A.tri.size() * sizeof(PtShadeTri)) +
                          align256(A.inst.size() * sizeof(PtShadeInst)) + align256(A.mat.size() * sizeof(PtMaterial)) +
@@ -349,7 +349,18 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
                          align256(A.tex.size() * sizeof(int4)) + align256(A.texels.size() * 4) +
                          align256(A.tri_lights.size() * sizeof(PtTriLight)) + align256(A.light_cdf.size() * 4) +
                          3 * 256;
-    cudaError_t err = cudaMalloc(&s->arena, bytes);
+    // The nodes' second copy is for the streaming walks only: a scene that does
+    // not stream has none, nor one that fits without it alone.
+    bool words = A.use_bvh && stack_words(A.nodes);
+    const size_t q_bytes = words ? align256(A.nodes.size() * 4) : 0;
+    cudaError_t err = cudaMalloc(&s->arena, bytes + q_bytes);
+    if (err == cudaSuccess) {
+        bytes += q_bytes;
+    } else if (words) {
+        words = false;
+        cudaGetLastError();
+        err = cudaMalloc(&s->arena, bytes);
+    }
     if (err != cudaSuccess) {
         delete s;
         return cuda_fail(err, "pt_scene_create: device allocation");
@@ -373,12 +384,14 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     D.tri_uv = upload(base, off, A.tri_uv, err);
     D.tex = upload(base, off, A.tex, err);
     D.texels = upload(base, off, A.texels, err);
-    D.qnodes = reinterpret_cast<const float4*>(base + off);
-    if (err == cudaSuccess)
-        err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(A.nodes.size() / 32), nullptr);
-    off += align256(A.nodes.size() * 4);
+    if (words) {
+        D.qnodes = reinterpret_cast<const float4*>(base + off);
+        if (err == cudaSuccess)
+            err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(A.nodes.size() / 32), nullptr);
+        off += align256(A.nodes.size() * 4);
+    }
     D.has_textures = A.has_textures;
-    D.words = A.use_bvh && stack_words(A.nodes);
+    D.words = words;
     D.ordered_boxes = ordered_boxes(A.nodes);
     D.stack_pack8 = stack_pack8(A.nodes);
     D.tree_kib = tree_kib(A.nodes, A.slots);

@@ -501,7 +501,7 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->total_items = items_total;
     b->out_floats = out_floats;
     all.n_flat_slots = 0;
-    const size_t bytes = 2 * align256(all.nodes.size() * 4) + align256(all.slots.size() * 4) + align256(all.islots.size() * 4) +
+    size_t bytes = align256(all.nodes.size() * 4) + align256(all.slots.size() * 4) + align256(all.islots.size() * 4) +
                          align256(all.large.size() * sizeof(float4)) + align256(all.large_mat.size() * 4) +
                          align256(all.sph.size() * sizeof(PtShadeSphere)) + align256(all.tri.size() * sizeof(PtShadeTri)) +
                          align256(all.inst.size() * sizeof(PtShadeInst)) + align256(all.mat.size() * sizeof(PtMaterial)) +
@@ -509,7 +509,17 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
                          align256(all.tex.size() * sizeof(int4)) + align256(all.texels.size() * 4) +
                          align256(n * sizeof(PtBatchScene)) + align256(n * sizeof(PtSceneDev)) +
                          align256(out_floats * 4) + align256(n * 4) + align256(n * 8) + 4 * 256;
-    cudaError_t err = cudaMalloc(&b->arena, bytes);
+    // as in pt_scene_create: a second copy of the nodes, where it fits and is used
+    bool words = stack_words(all.nodes);
+    const size_t q_bytes = words ? align256(all.nodes.size() * 4) : 0;
+    cudaError_t err = cudaMalloc(&b->arena, bytes + q_bytes);
+    if (!err) {
+        bytes += q_bytes;
+    } else if (words) {
+        words = false;
+        cudaGetLastError();
+        err = cudaMalloc(&b->arena, bytes);
+    }
     if (err) return cuda_fail(err, "pt_batch_create: device allocation");
     b->arena_bytes = bytes;
     char* base = static_cast<char*>(b->arena);
@@ -529,11 +539,14 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     D.tri_uv = upload(base, off, all.tri_uv, err);
     D.tex = upload(base, off, all.tex, err);
     D.texels = upload(base, off, all.texels, err);
-    D.qnodes = reinterpret_cast<const float4*>(base + off);
-    if (!err) err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(all.nodes.size() / 32), nullptr);
-    off += align256(all.nodes.size() * 4);
+    if (words) {
+        D.qnodes = reinterpret_cast<const float4*>(base + off);
+        if (!err)
+            err = pt_build_qnodes(D.nodes, reinterpret_cast<float4*>(base + off), uint32_t(all.nodes.size() / 32), nullptr);
+        off += align256(all.nodes.size() * 4);
+    }
     D.has_textures = all.has_textures;
-    D.words = stack_words(all.nodes);
+    D.words = words;
     D.ordered_boxes = ordered_boxes(all.nodes);
     D.stack_pack8 = stack_pack8(all.nodes);
     D.tree_kib = tree_kib(all.nodes, all.slots);

@@ -250,3 +250,29 @@ def test_each_scene_keeps_its_own_launch_shapes(fake):
     for d, aux, new in ((a, False, 1), (a, False, 0), (a, True, 1), (b, False, 1), (a, True, 0), (b, False, 0)):
         d.render(320, 200, 4, 0x7000, aux)
         assert fake.log().count("blocks worked out") == new
+
+
+def test_a_scene_that_fits_only_without_its_second_nodes_is_accepted(fake):
+    """The streaming walks' copy of the nodes is left out where it does not fit: the scene and the batch are made, and
+    render in lock step. Scenes that cannot stream (leaves past a stack word, no tree) hold no copy."""
+    import photon_tracer_b200 as pt
+    before = fake.live_bytes()
+    d = DeviceScene(ROOM, 4)
+    full, nodes = d.s.info().device_bytes, 128 * d.s.info().n_nodes
+    assert fake.live_bytes() - before == full
+    d.s.close()
+    with fake.budget(before + full - 4096):
+        d = DeviceScene(ROOM, 4)
+        assert d.s.info().device_bytes == full - (nodes + 255) // 256 * 256
+    fake.log()
+    d.render(320, 200, 16, 0x7000)
+    assert not launches(fake.log(), "samples")
+    d.s.close()
+    b = make_batch(ONE_LAUNCH, max_bounces=0)
+    arena = fake.live_bytes() - before
+    b.close()
+    with fake.budget(before + arena - 4096):
+        b = make_batch(ONE_LAUNCH)
+    assert one_launch_lines(fake, b) == ["batch 128"]
+    b.close()
+    assert pt.Scene(pt.Generated(0, seed=1)).info().n_nodes == 0 and "build_qnodes" not in fake.log()
