@@ -276,3 +276,17 @@ def test_a_scene_that_fits_only_without_its_second_nodes_is_accepted(fake):
     assert one_launch_lines(fake, b) == ["batch 128"]
     b.close()
     assert pt.Scene(pt.Generated(0, seed=1)).info().n_nodes == 0 and "build_qnodes" not in fake.log()
+
+
+def test_inference_allocates_nothing_for_the_backward(fake):
+    """The buffers that only the tensor-core backward uses come with the first gradients of a size: two bf16 buffers'
+    worth of the largest activation, one of which the workspace has, and 16 bytes per pixel."""
+    from photon_tracer_b200 import abi
+    net = C.c_void_p()
+    abi.check(fake.lib.pt_unet_create(1, C.byref(net)))
+    pixels = 2 * 64 * 40
+    abi.check(fake.lib.pt_unet_forward(net, 2, 64, 40, SOME, SOME, None))
+    inference = fake.live_bytes()
+    assert grads(fake, net, 2, 64, 40) == abi.PT_OK
+    assert fake.live_bytes() - inference == pixels * 32 * 2 + pixels * 16
+    fake.lib.pt_unet_destroy(net)
