@@ -174,8 +174,13 @@ void run_atrous(int w, int h, const float* color, const float* albedo, const flo
     const int n = w * h;
     // A caller may filter into its albedo buffer: the last pass, which reads
     // neighbours' albedo, must then not write there.
-    const bool in_albedo = reinterpret_cast<uintptr_t>(out) < reinterpret_cast<uintptr_t>(albedo + 3 * size_t(n)) &&
-                           reinterpret_cast<uintptr_t>(albedo) < reinterpret_cast<uintptr_t>(out + 3 * size_t(n));
+    // Nor where the caller reuses the scratch for the image: that pass still
+    // reads lighting and normals there.
+    auto meets_out = [&](const float* p, size_t floats) {
+        return reinterpret_cast<uintptr_t>(out) < reinterpret_cast<uintptr_t>(p + floats) &&
+               reinterpret_cast<uintptr_t>(p) < reinterpret_cast<uintptr_t>(out + 3 * size_t(n));
+    };
+    const bool in_albedo = meets_out(albedo, 3 * size_t(n)), in_scratch = meets_out(scratch, 11 * size_t(n));
     float* lv = scratch;
     float* lv_next = lv + 4 * size_t(n);
     float* nrm = lv_next + 4 * size_t(n);
@@ -184,9 +189,12 @@ void run_atrous(int w, int h, const float* color, const float* albedo, const flo
     launch_pass<2, ALIGNED, false>(w, h, 2, albedo, nrm, lv_next, lv, nullptr, stream);
     launch_pass<4, ALIGNED, false>(w, h, 4, albedo, nrm, lv, lv_next, nullptr, stream);
     launch_pass<4, ALIGNED, false>(w, h, 8, albedo, nrm, lv_next, lv, nullptr, stream);
-    if (in_albedo) {
+    if (in_albedo || in_scratch) {
         launch_pass<4, ALIGNED, false>(w, h, 16, albedo, nrm, lv, lv_next, nullptr, stream);
-        finish<ALIGNED><<<(n + 255) / 256, 256, 0, stream>>>(n, lv_next, albedo, out);
+        // beside lv_next, in a part of the scratch that is free by now and that out does not meet
+        float* image = !in_scratch ? out : meets_out(lv, 4 * size_t(n)) ? nrm : lv;
+        finish<ALIGNED><<<(n + 255) / 256, 256, 0, stream>>>(n, lv_next, albedo, image);
+        if (in_scratch) cudaMemcpyAsync(out, image, 12 * size_t(n), cudaMemcpyDeviceToDevice, stream);
     } else {
         launch_pass<4, ALIGNED, true>(w, h, 16, albedo, nrm, lv, nullptr, out, stream);
     }

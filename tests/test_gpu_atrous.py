@@ -33,3 +33,22 @@ def test_atrous_sizes(built, w, h, shift, into_albedo):
     got = out.cpu().numpy()
     # expf may differ by an ulp, which the variance-scaled luminance weights of later passes amplify
     np.testing.assert_allclose(got, want, rtol=1e-3, atol=1e-5)
+
+
+@pytest.mark.parametrize("at", [0.0, 1.5, 3.0, 4.0, 5.5, 6.0, 8.0])
+def test_atrous_into_its_scratch(built, at):
+    """The image may go into the scratch itself, at any place (floats per pixel from its start)."""
+    import torch
+    from photon_tracer_b200 import abi
+    w, h = 70, 42
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    d = [torch.rand((h, w) + s, device="cuda", generator=gen) for s in ((3,), (3,), (3,), ())]
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    run = lambda out, scratch: abi.check(built.load().pt_denoise_atrous_device(
+        w, h, *[ptr(t) for t in d], ptr(out), ptr(scratch), stream))
+    want, scratch = torch.empty((h, w, 3), device="cuda"), torch.empty(11 * w * h, device="cuda")
+    run(want, scratch)
+    out = scratch[int(at * w * h):][:3 * w * h]
+    run(out, scratch)
+    assert torch.equal(out.view(h, w, 3), want)
