@@ -161,17 +161,10 @@ PtRenderParams make_params(const pt_camera* cam, const pt_settings* st) {
 // Paths the wavefront keeps in flight: one per pixel up to 2^20.
 constexpr uint32_t kMaxWaveSlots = 1u << 20;
 
-// Whether a frame renders with the streaming megakernel. It gains from
-// samples in flight; where a lane per pixel already is one per sample, the
-// lock-step form is as fast or faster: with one sample per pixel up to about a
-// million pixels (room, 360,000 pixels: 0.66 against 0.77 ms; 1.44 million:
-// 2.05 against 1.72), and, in scenes of a few nodes, whose walks are short,
-// with up to three (488 spheres, 1.44 million pixels, 2 samples: 1.90 against
-// 2.01 ms; 3: 2.92 against 2.94).
 bool streams(const pt_scene* s, const PtRenderParams& p) {
-    if (!s->dev.words || p.depth < 1 || p.depth > PT_SAMPLES_MAX_DEPTH) return false;
-    if (p.spp == 1) return s->dev.tree_kib > 64 && int64_t(p.width) * p.rows >= (1 << 20);
-    return p.spp > 3 || s->dev.tree_kib > 64;
+    return s->dev.words && p.depth >= 1 && p.depth <= PT_SAMPLES_MAX_DEPTH &&
+           stream_gains(s->dev.tree_kib, s->dev.sky != 0, p.spp, p.depth, uint64_t(p.width) * uint64_t(p.rows),
+                        p.aux != nullptr, s->sms);
 }
 
 // Samples per pixel of one streaming launch, as many as kSampleBytes hold
@@ -257,6 +250,36 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
 }
 
 }  // namespace
+
+// The streaming form gains from samples in flight: where pixels leave lanes
+// idle, where a few pixels take long, where walks of a warp differ. It pays for
+// it with a pass of each sample's radiance through memory and with code that is
+// fetched for less work where paths are short. (Times: lock-step, streaming,
+// in us.)
+bool pt::stream_gains(uint32_t kib, bool sky, int spp, int depth, uint64_t pixels, bool aux, int sms) {
+    const uint64_t lanes = uint64_t(sms) * 640;  // of the lock-step form
+    // Under an open sky paths end early, so the trees have to be larger for the
+    // walks to be long.
+    const uint32_t small = sky ? 256 : 64;
+    // One sample: a lane per pixel already is one per sample (room, 360,000
+    // pixels 660, 770; 1.44 million 2,050, 1,720; 2,000 spheres, 2 million
+    // slower by 18%), and a few are little more (488 spheres, 1.44 million, 2
+    // samples 1,900, 2,010; 2,000 spheres 4-7% slower with 2).
+    if (spp == 1) return kib > small && depth > 2 && pixels >= (1 << 20);
+    if (spp <= 3 && kib <= small) return false;
+    // Camera rays and one bounce, or two among a few spheres under the sky, gain
+    // only with idle lanes, and by the large scenes' long walks: the reference's
+    // room, 640x360, 8 samples, depth 1 163, 188; depth 2 736, 955; at 400x225, 4
+    // samples 162, 195; the room of 81,920 triangles 0.54 and 0.74 of the time at
+    // 640x360, 8 samples, but 1.33 at 1920x1080, 4, depth 1, and 1.06 at 320x180, 3.
+    if (depth <= (sky && kib <= 40 ? 3 : 2))
+        return spp > 3 && (pixels <= (kib > 64 ? lanes : lanes / 2) || (kib > 1024 && pixels <= 4 * lanes));
+    // Small open scenes whose pixels fill the lanes several times over: 24
+    // spheres, 1280x720, 8 samples 12% slower, the reference's field 4% (1920x1080:
+    // 9%); 488 spheres 6% faster, with guides 2% slower at 1920x1080.
+    if (sky && pixels > 4 * lanes && (kib <= 40 || (aux && kib <= 64 && pixels > 12 * lanes))) return false;
+    return true;
+}
 
 void pt::set_wave_slots(pt_scene* s, uint32_t slots) { s->wave_slots = slots; }
 

@@ -48,6 +48,10 @@ int stack_pack8(const std::vector<float>& nodes);
 // 1 when every entry of the scene's trees fits a stack word of stream.cuh:
 // leaves of at most 15 entries from below 2^25, node indices below 2^31.
 int stack_words(const std::vector<float>& nodes);
+// Whether `spp` samples of each of `pixels` pixels render faster as streams of
+// samples (stream_mega.cuh) than with a lane per pixel, in a scene of kib KiB
+// of trees.
+bool stream_gains(uint32_t kib, bool sky, int spp, int depth, uint64_t pixels, bool aux, int sms);
 // KiB of nodes and leaf slots (PtSceneDev::tree_kib), saturating.
 uint32_t tree_kib(const std::vector<float>& nodes, const std::vector<float>& slots);
 

@@ -290,3 +290,36 @@ def test_inference_allocates_nothing_for_the_backward(fake):
     assert grads(fake, net, 2, 64, 40) == abi.PT_OK
     assert fake.live_bytes() - inference == pixels * 32 * 2 + pixels * 16
     fake.lib.pt_unet_destroy(net)
+
+
+# Scenes by (generator, parameter): 24 and 488 spheres and the reference's field under the sky, its room, rooms with
+# 1,280 and 81,920 triangles, 300 instances under the sky.
+SPHERES_24, SPHERES_488, FIELD, REF_ROOM, ROOM_1K, ROOM_80K, INSTANCES = (
+    (10, 20), (10, 0), (1, 0), (3, 0), (11, 3), (11, 6), (12, 300))
+
+
+@pytest.mark.parametrize("scene,streams,not_streams", [
+    # (width, height, samples, bounces, guides)
+    (SPHERES_24, [(640, 360, 8, 10, 0), (128, 72, 4, 10, 1)], [(1280, 720, 8, 10, 0), (640, 360, 3, 10, 0),
+                                                             (640, 360, 8, 2, 0), (640, 360, 4, 3, 0)]),
+    (SPHERES_488, [(400, 225, 16, 10, 0), (1920, 1080, 8, 10, 0), (1280, 720, 8, 10, 1)],
+     [(1920, 1080, 8, 10, 1), (1280, 720, 3, 10, 0), (640, 360, 8, 1, 0)]),
+    (FIELD, [(640, 360, 4, 10, 1)], [(1920, 1080, 8, 10, 0), (1280, 720, 4, 10, 0)]),
+    (REF_ROOM, [(1920, 1080, 4, 3, 0), (640, 360, 4, 10, 1)], [(640, 360, 8, 1, 0), (640, 360, 8, 2, 1),
+                                                            (1920, 1080, 4, 2, 0), (640, 360, 3, 10, 0),
+                                                            (400, 225, 4, 2, 0)]),
+    (ROOM_1K, [(640, 360, 2, 10, 0), (256, 256, 16, 1, 0), (1920, 1080, 1, 10, 0)],
+     [(640, 360, 8, 2, 0), (1920, 1080, 4, 1, 0), (640, 360, 1, 10, 0)]),
+    (ROOM_80K, [(1024, 1024, 64, 10, 0), (640, 360, 8, 1, 0), (640, 360, 8, 2, 0)],
+     [(1920, 1080, 4, 1, 1), (1920, 1080, 4, 2, 0), (320, 180, 3, 2, 0)]),
+    (INSTANCES, [(960, 540, 16, 10, 0), (640, 360, 2, 10, 0)], [(1920, 1080, 4, 1, 0)]),
+])
+def test_which_frames_stream(fake, scene, streams, not_streams):
+    """Frames take the form that was measured faster for frames like them."""
+    d = DeviceScene(*scene)
+    for sizes, form in ((streams, "samples"), (not_streams, "megakernel")):
+        for w, h, spp, depth, aux in sizes:
+            st = d.s.settings(w, h, spp, depth, seed=1)
+            fake.log()
+            d.s.render_device(d.g.camera, st, SOME.value, SOME.value if aux else 0, 0, 0x7000)
+            assert launches(fake.log(), form), (w, h, spp, depth, aux, form)
