@@ -60,6 +60,8 @@ struct Scratch {
     }
 };
 
+constexpr int kCounters = 32, kCounterWords = 8;  // words apart
+
 struct pt_scene {
     PtSceneDev dev{};
     pt_scene_info info;
@@ -67,7 +69,9 @@ struct pt_scene {
     int sms = 148;
     void* arena = nullptr;
     unsigned int* status = nullptr;    // device error word
-    unsigned int* work = nullptr;      // work counter of renders that borrow none (RenderMemory)
+    unsigned int* work = nullptr;      // kCounters work counters: captured renders', then one per stream (counter_of)
+    unsigned long long counter_stream[kCounters] = {};  // ids of the streams that have one
+    int counters = 1;
     unsigned long long* rays = nullptr;
     cudaStream_t stream = nullptr;
     Scratch out, aux, states, in_rays, out_hits, counts, wave, sum;
@@ -194,6 +198,24 @@ struct RenderMemory {
     ~RenderMemory() { pool_return(ptr, stream); }
 };
 
+// The work counter of the scene's lock-step renders on a stream: renders in
+// flight on several streams each have their own, and those on one stream are
+// ordered. (A borrowed one costs 3 us, of 22 for a small frame.) Streams are
+// told apart by their ids, which are not used again; null when too many have
+// rendered.
+unsigned int* counter_of(pt_scene* s, cudaStream_t stream) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(stream, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    int k = 1;
+    while (k < s->counters && s->counter_stream[k] != id) ++k;
+    if (k == kCounters) return nullptr;
+    if (k == s->counters) s->counter_stream[s->counters++] = id;
+    return s->work + k * kCounterWords;
+}
+
 bool is_capturing(cudaStream_t stream) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     const bool none =
@@ -215,18 +237,18 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
         return PT_OK;
     }
     // A captured render borrows nothing (a graph would keep the address): it
-    // counts in the scene's own word and takes the lock-step form, as a render
-    // without memory for its samples does.
+    // takes the lock-step form, as a render without memory for its samples does,
+    // with a counter of its own.
     RenderMemory memory;
     int count = 0;
-    if (!is_capturing(stream)) {
+    const bool captured = is_capturing(stream);
+    if (!captured) {
         count = streams(s, p) ? samples_per_launch(p) : 0;
         if (count > 0 && !memory.borrow(s, kCounterBytes + pt_sample_bytes(p) * size_t(count), stream)) count = 0;
-        if (count == 0) memory.borrow(s, kCounterBytes, stream);
     }
     const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
-    p.work = memory.ptr ? static_cast<unsigned int*>(memory.ptr) : s->work;
     if (count > 0) {
+        p.work = static_cast<unsigned int*>(memory.ptr);
         float* samples = reinterpret_cast<float*>(static_cast<char*>(memory.ptr) + kCounterBytes);
         for (int first = 0; first < p.spp; first += count) {
             cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream);
@@ -236,6 +258,12 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
             if (e) return cuda_fail(e, "megakernel launch");
         }
         return PT_OK;
+    }
+    p.work = s->work;
+    if (!captured) {
+        p.work = counter_of(s, stream);
+        if (!p.work)
+            p.work = memory.borrow(s, kCounterBytes, stream) ? static_cast<unsigned int*>(memory.ptr) : s->work;
     }
     if (cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
     PtLaunchShape shape;
@@ -365,13 +393,13 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     s->device = device;
     s->sms = sms;
     size_t bytes = align256(A.nodes.size() * 4) + align256(A.slots.size() * 4) + align256(A.islots.size() * 4) +
-                         align256(A.large.size() * sizeof(float4)) + align256(A.large_mat.size() * 4) +
-                         align256(A.sph.size() * sizeof(PtShadeSphere)) + align256(A.tri.size() * sizeof(PtShadeTri)) +
-                         align256(A.inst.size() * sizeof(PtShadeInst)) + align256(A.mat.size() * sizeof(PtMaterial)) +
-                         align256(A.lights.size() * sizeof(PtLight)) + align256(A.tri_uv.size() * 4) +
-                         align256(A.tex.size() * sizeof(int4)) + align256(A.texels.size() * 4) +
-                         align256(A.tri_lights.size() * sizeof(PtTriLight)) + align256(A.light_cdf.size() * 4) +
-                         3 * 256;
+                   align256(A.large.size() * sizeof(float4)) + align256(A.large_mat.size() * 4) +
+                   align256(A.sph.size() * sizeof(PtShadeSphere)) + align256(A.tri.size() * sizeof(PtShadeTri)) +
+                   align256(A.inst.size() * sizeof(PtShadeInst)) + align256(A.mat.size() * sizeof(PtMaterial)) +
+                   align256(A.lights.size() * sizeof(PtLight)) + align256(A.tri_uv.size() * 4) +
+                   align256(A.tex.size() * sizeof(int4)) + align256(A.texels.size() * 4) +
+                   align256(A.tri_lights.size() * sizeof(PtTriLight)) + align256(A.light_cdf.size() * 4) +
+                   2 * 256 + kCounters * kCounterWords * 4;
     // The nodes' second copy is for the streaming walks only: a scene that does
     // not stream has none, nor one that fits without it alone.
     bool words = A.use_bvh && stack_words(A.nodes);
@@ -421,10 +449,10 @@ pt_status pt_scene_create(const pt_scene_desc* desc, pt_scene** out) {
     s->status = reinterpret_cast<unsigned int*>(base + off);
     off += 256;
     s->work = reinterpret_cast<unsigned int*>(base + off);
-    off += 256;
+    off += kCounters * kCounterWords * 4;
     s->rays = reinterpret_cast<unsigned long long*>(base + off);
     off += 256;
-    if (err == cudaSuccess) err = cudaMemset(s->status, 0, 3 * 256);
+    if (err == cudaSuccess) err = cudaMemset(s->status, 0, 2 * 256 + kCounters * kCounterWords * 4);
     if (err == cudaSuccess) err = cudaStreamSynchronize(nullptr);
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
     if (err != cudaSuccess) {

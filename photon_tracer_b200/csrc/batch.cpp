@@ -502,13 +502,13 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->out_floats = out_floats;
     all.n_flat_slots = 0;
     size_t bytes = align256(all.nodes.size() * 4) + align256(all.slots.size() * 4) + align256(all.islots.size() * 4) +
-                         align256(all.large.size() * sizeof(float4)) + align256(all.large_mat.size() * 4) +
-                         align256(all.sph.size() * sizeof(PtShadeSphere)) + align256(all.tri.size() * sizeof(PtShadeTri)) +
-                         align256(all.inst.size() * sizeof(PtShadeInst)) + align256(all.mat.size() * sizeof(PtMaterial)) +
-                         align256(all.lights.size() * sizeof(PtLight)) + align256(all.tri_uv.size() * 4) +
-                         align256(all.tex.size() * sizeof(int4)) + align256(all.texels.size() * 4) +
-                         align256(n * sizeof(PtBatchScene)) + align256(n * sizeof(PtSceneDev)) +
-                         align256(out_floats * 4) + align256(n * 4) + align256(n * 8) + 4 * 256;
+                   align256(all.large.size() * sizeof(float4)) + align256(all.large_mat.size() * 4) +
+                   align256(all.sph.size() * sizeof(PtShadeSphere)) + align256(all.tri.size() * sizeof(PtShadeTri)) +
+                   align256(all.inst.size() * sizeof(PtShadeInst)) + align256(all.mat.size() * sizeof(PtMaterial)) +
+                   align256(all.lights.size() * sizeof(PtLight)) + align256(all.tri_uv.size() * 4) +
+                   align256(all.tex.size() * sizeof(int4)) + align256(all.texels.size() * 4) +
+                   align256(n * sizeof(PtBatchScene)) + align256(n * sizeof(PtSceneDev)) +
+                   align256(out_floats * 4) + align256(n * 4) + align256(n * 8) + 4 * 256;
     // as in pt_scene_create: a second copy of the nodes, where it fits and is used
     bool words = stack_words(all.nodes);
     const size_t q_bytes = words ? align256(all.nodes.size() * 4) : 0;

@@ -137,6 +137,9 @@ cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) {
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     return *s = reinterpret_cast<cudaStream_t>(0x1000 + 16 * ++g_next), cudaSuccess;
 }
+cudaError_t cudaStreamGetId(cudaStream_t s, unsigned long long* id) {
+    return *id = reinterpret_cast<unsigned long long>(s), cudaSuccess;
+}
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t) { return log("wait stream"), cudaSuccess; }
 cudaError_t cudaStreamIsCapturing(cudaStream_t s, cudaStreamCaptureStatus* c) {

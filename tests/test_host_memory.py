@@ -323,3 +323,27 @@ def test_which_frames_stream(fake, scene, streams, not_streams):
             fake.log()
             d.s.render_device(d.g.camera, st, SOME.value, SOME.value if aux else 0, 0, 0x7000)
             assert launches(fake.log(), form), (w, h, spp, depth, aux, form)
+
+
+def test_lock_step_renders_borrow_nothing_on_their_usual_streams(fake):
+    """A stream's lock-step renders count in that stream's own word, captured ones in another; with more streams than
+    words, and no memory to borrow, the render still runs."""
+    d = DeviceScene(SPHERES, 20)
+    fake.log()
+    counters = {}
+    for stream in [0x7000 + 16 * k for k in range(40)] * 2:
+        d.render(100, 60, 1, stream)
+        lines = fake.log()
+        (got,) = launches(lines, "megakernel")
+        borrowed = any(x.startswith("borrow") for x in lines)
+        if not borrowed:
+            assert counters.setdefault(stream, got[1]) == got[1]
+        assert borrowed == (stream not in counters)
+    fake.lib.fake_capture(0x7000)
+    d.render(100, 60, 1, 0x7000)
+    fake.lib.fake_capture(None)
+    (captured,) = launches(fake.log(), "megakernel")
+    assert len(counters) == len(set(counters.values())) == 31 and captured[1] not in counters.values()
+    with fake.failing_above(0):
+        d.render(100, 60, 1, 0x9000)
+    assert not any(x.startswith("bad") for x in fake.log())
