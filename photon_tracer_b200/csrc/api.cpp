@@ -309,6 +309,30 @@ bool pt::stream_gains(uint32_t kib, bool sky, int spp, int depth, uint64_t pixel
     return true;
 }
 
+// Streaming walks pay once lanes get several rays each; with fewer a walk's own
+// latency counts, and the lock-step kernels' steps are shorter. How many is a
+// matter of how long the walks are. (Times: streaming by lock-step.)
+bool pt_rays_stream(const PtSceneDev& S, size_t n, bool any, int sms) {
+    if (!S.words) return false;
+    const bool open = S.n_large > 0;  // a large sphere, tested before the trees, ends many rays
+    // A few nodes: at no size (24 spheres 1.04-1.20 to 1.2 million rays, the
+    // reference's field 1.1-1.2 to 2.5 million, its room's any hits of short
+    // segments 1.17).
+    if (S.tree_kib <= 8 || (open && S.tree_kib <= 40)) return false;
+    int per_lane = 2;  // rooms from 110 KiB on, 227,000 rays 0.83-0.98, 120,000 1.02-1.13
+    if (any && open) {
+        // 488 spheres 1.01-1.08 to 800,000 rays, 1.2 million 0.85-0.91; 2,000
+        // spheres 1.18 at 300,000, 0.88-0.93 at 650,000; 300 instances 1.10 at
+        // 400,000, 0.96 from 650,000; 10,000 instances 1.15 at 260,000, 0.80-0.92 above
+        per_lane = S.tree_kib <= 64 ? 9 : S.n_instances >= 1000 ? 3 : 6;
+    } else if (any && S.n_instances > 0) {
+        per_lane = 5;  // the textured room, six instances: 1.00-1.08 to 500,000, 0.85 at 1.2 million
+    } else if (open && (S.tree_kib <= 64 || (S.n_instances > 0 && S.n_instances < 128))) {
+        per_lane = 3;  // closest hits: 488 spheres 1.02 at 260,000, 0.97 from 300,000; 60 instances 1.09, 0.99 at 350,000
+    }
+    return n > size_t(sms) * 768 * size_t(per_lane);  // of the streaming kernel's resident lanes
+}
+
 void pt::set_wave_slots(pt_scene* s, uint32_t slots) { s->wave_slots = slots; }
 
 namespace {
@@ -657,7 +681,8 @@ pt_status pt_trace_closest_device(pt_scene* s, const float* d_rays, size_t n, fl
     clear_error();
     if (!s || (n && (!d_rays || !d_hits))) return fail(PT_ERR_INVALID_ARG, "pt_trace_closest_device: null pointer");
     if (pt_status e = use_device(s)) return e;
-    if (cudaError_t e = pt_launch_trace_closest(s->dev, d_rays, n, tmin, tmax, d_hits, static_cast<cudaStream_t>(stream)))
+    if (cudaError_t e = pt_launch_trace_closest(s->dev, d_rays, n, tmin, tmax, d_hits, s->sms,
+                                                static_cast<cudaStream_t>(stream)))
         return cuda_fail(e, "trace_closest launch");
     return PT_OK;
 }
@@ -667,7 +692,8 @@ pt_status pt_trace_any_device(pt_scene* s, const float* d_rays, size_t n, float 
     clear_error();
     if (!s || (n && (!d_rays || !d_occ))) return fail(PT_ERR_INVALID_ARG, "pt_trace_any_device: null pointer");
     if (pt_status e = use_device(s)) return e;
-    if (cudaError_t e = pt_launch_trace_any(s->dev, d_rays, n, tmin, tmax, d_occ, static_cast<cudaStream_t>(stream)))
+    if (cudaError_t e = pt_launch_trace_any(s->dev, d_rays, n, tmin, tmax, d_occ, s->sms,
+                                            static_cast<cudaStream_t>(stream)))
         return cuda_fail(e, "trace_any launch");
     return PT_OK;
 }
@@ -698,7 +724,7 @@ pt_status pt_trace_closest(pt_scene* s, const float* rays, size_t n, float tmin,
     if (cudaError_t e = cudaMemcpyAsync(s->in_rays.ptr, rays, n * 24, cudaMemcpyHostToDevice, stream))
         return cuda_fail(e, "pt_trace_closest: copy");
     if (cudaError_t e = pt_launch_trace_closest(s->dev, static_cast<const float*>(s->in_rays.ptr), n, tmin, tmax,
-                                                s->out_hits.ptr, stream))
+                                                s->out_hits.ptr, s->sms, stream))
         return cuda_fail(e, "trace_closest launch");
     if (cudaError_t e = cudaMemcpyAsync(hits, s->out_hits.ptr, n * sizeof(pt_hit), cudaMemcpyDeviceToHost, stream))
         return cuda_fail(e, "pt_trace_closest: copy back");
@@ -716,7 +742,7 @@ pt_status pt_trace_any(pt_scene* s, const float* rays, size_t n, float tmin, flo
     if (cudaError_t e = cudaMemcpyAsync(s->in_rays.ptr, rays, n * 24, cudaMemcpyHostToDevice, stream))
         return cuda_fail(e, "pt_trace_any: copy");
     if (cudaError_t e = pt_launch_trace_any(s->dev, static_cast<const float*>(s->in_rays.ptr), n, tmin, tmax,
-                                            static_cast<uint8_t*>(s->out_hits.ptr), stream))
+                                            static_cast<uint8_t*>(s->out_hits.ptr), s->sms, stream))
         return cuda_fail(e, "trace_any launch");
     if (cudaError_t e = cudaMemcpyAsync(occ, s->out_hits.ptr, n, cudaMemcpyDeviceToHost, stream))
         return cuda_fail(e, "pt_trace_any: copy back");

@@ -52,9 +52,11 @@ cudaError_t pt_launch_samples(const PtSceneDev& scene, const PtRenderParams& p, 
 // Ray queries: closest hit (pt_hit records), any hit (bytes), and traversal
 // work counters (5 x u64, added to).
 cudaError_t pt_launch_trace_closest(const PtSceneDev& scene, const float* rays, size_t n, float tmin, float tmax,
-                                    void* hits, cudaStream_t stream);
+                                    void* hits, int sms, cudaStream_t stream);
+// Whether n of a scene's ray queries are faster as streaming walks.
+bool pt_rays_stream(const PtSceneDev& scene, size_t n, bool any, int sms);
 cudaError_t pt_launch_trace_any(const PtSceneDev& scene, const float* rays, size_t n, float tmin, float tmax,
-                                uint8_t* occluded, cudaStream_t stream);
+                                uint8_t* occluded, int sms, cudaStream_t stream);
 cudaError_t pt_launch_trace_count(const PtSceneDev& scene, const float* rays, size_t n, float tmin, float tmax,
                                   unsigned long long* counts, cudaStream_t stream);
 

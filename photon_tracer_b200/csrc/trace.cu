@@ -211,23 +211,16 @@ int sm_count() {
     return sms;
 }
 
-int grid_for(size_t n, int threads) {
+int grid_for(size_t n, int threads, int sms) {
     const size_t want = (n + threads - 1) / threads;
-    const size_t cap = size_t(sm_count()) * 16;
+    const size_t cap = size_t(sms) * 16;
     return int(want < cap ? (want ? want : 1) : cap);
 }
 
-// Streaming pays once lanes get several rays each. Below two rays per
-// resident lane a walk's own latency is what counts, and the lock-step kernels
-// with their shorter steps are as fast or faster (room scene, closest hits:
-// 30,000 rays 76 against 87 us, 100,000 rays 95 against 106, 300,000 rays 137
-// against 130).
-bool stream_rays(const PtSceneDev& S, size_t n) { return S.words && n > size_t(sm_count()) * kStreamBlocks * 128 * 2; }
-
 template <bool ANY>
 cudaError_t launch_stream(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax, pt_hit* hits,
-                          uint8_t* occ, cudaStream_t stream) {
-    const int blocks = sm_count() * kStreamBlocks;
+                          uint8_t* occ, int sms, cudaStream_t stream) {
+    const int blocks = sms * kStreamBlocks;
     if (flat_scene(S))
         trace_stream_kernel<false, ANY><<<blocks, 128, 0, stream>>>(S, rays, n, tmin, tmax, hits, occ);
     else
@@ -238,31 +231,32 @@ cudaError_t launch_stream(const PtSceneDev& S, const float* rays, size_t n, floa
 }  // namespace
 
 cudaError_t pt_launch_trace_closest(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax,
-                                    void* hits, cudaStream_t stream) {
+                                    void* hits, int sms, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    if (stream_rays(S, n)) return launch_stream<false>(S, rays, n, tmin, tmax, static_cast<pt_hit*>(hits), nullptr, stream);
+    pt_hit* const out = static_cast<pt_hit*>(hits);
+    if (pt_rays_stream(S, n, false, sms)) return launch_stream<false>(S, rays, n, tmin, tmax, out, nullptr, sms, stream);
     if (flat_scene(S))
-        trace_closest_kernel<true><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, static_cast<pt_hit*>(hits));
+        trace_closest_kernel<true><<<grid_for(n, 128, sms), 128, 0, stream>>>(S, rays, n, tmin, tmax, out);
     else
-        trace_closest_kernel<false><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, static_cast<pt_hit*>(hits));
+        trace_closest_kernel<false><<<grid_for(n, 128, sms), 128, 0, stream>>>(S, rays, n, tmin, tmax, out);
     return cudaGetLastError();
 }
 
 cudaError_t pt_launch_trace_any(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax,
-                                uint8_t* occ, cudaStream_t stream) {
+                                uint8_t* occ, int sms, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    if (stream_rays(S, n)) return launch_stream<true>(S, rays, n, tmin, tmax, nullptr, occ, stream);
+    if (pt_rays_stream(S, n, true, sms)) return launch_stream<true>(S, rays, n, tmin, tmax, nullptr, occ, sms, stream);
     if (flat_scene(S))
-        trace_any_kernel<true><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, occ);
+        trace_any_kernel<true><<<grid_for(n, 128, sms), 128, 0, stream>>>(S, rays, n, tmin, tmax, occ);
     else
-        trace_any_kernel<false><<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, occ);
+        trace_any_kernel<false><<<grid_for(n, 128, sms), 128, 0, stream>>>(S, rays, n, tmin, tmax, occ);
     return cudaGetLastError();
 }
 
 cudaError_t pt_launch_trace_count(const PtSceneDev& S, const float* rays, size_t n, float tmin, float tmax,
                                   unsigned long long* counts, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    trace_count_kernel<<<grid_for(n, 128), 128, 0, stream>>>(S, rays, n, tmin, tmax, counts);
+    trace_count_kernel<<<grid_for(n, 128, sm_count()), 128, 0, stream>>>(S, rays, n, tmin, tmax, counts);
     return cudaGetLastError();
 }
 
@@ -270,6 +264,6 @@ cudaError_t pt_launch_primary_depth(const PtSceneDev& S, const PtCamDev& cam, in
                                     cudaStream_t stream) {
     const size_t n = size_t(width) * height;
     if (n == 0) return cudaSuccess;
-    primary_depth_kernel<<<grid_for(n, 128), 128, 0, stream>>>(S, cam, width, height, depth);
+    primary_depth_kernel<<<grid_for(n, 128, sm_count()), 128, 0, stream>>>(S, cam, width, height, depth);
     return cudaGetLastError();
 }

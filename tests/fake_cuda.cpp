@@ -194,11 +194,13 @@ cudaError_t pt_launch_samples(const PtSceneDev&, const PtRenderParams& p, int, i
     return launch("samples " + hex(st) + " work " + hex(p.work) + " buffer " + hex(buffer),
                   {{p.work, 4}, {buffer, pt_sample_bytes(p) * size_t(count)}});
 }
-cudaError_t pt_launch_trace_closest(const PtSceneDev&, const float*, size_t, float, float, void*, cudaStream_t) {
-    return kernel("closest");
+cudaError_t pt_launch_trace_closest(const PtSceneDev& S, const float*, size_t n, float, float, void*, int sms,
+                                    cudaStream_t) {
+    return kernel(pt_rays_stream(S, n, false, sms) ? "closest stream" : "closest lock-step");
 }
-cudaError_t pt_launch_trace_any(const PtSceneDev&, const float*, size_t, float, float, uint8_t*, cudaStream_t) {
-    return kernel("any");
+cudaError_t pt_launch_trace_any(const PtSceneDev& S, const float*, size_t n, float, float, uint8_t*, int sms,
+                                cudaStream_t) {
+    return kernel(pt_rays_stream(S, n, true, sms) ? "any stream" : "any lock-step");
 }
 cudaError_t pt_launch_trace_count(const PtSceneDev&, const float*, size_t, float, float, unsigned long long*,
                                   cudaStream_t) {

@@ -111,3 +111,32 @@ def test_streamed_batch(built, sizes):
         assert rays == total
     times = b.scene_times()
     assert np.all(times > 0) and np.all(np.isfinite(times))
+
+
+@pytest.mark.parametrize("kind,param,extent,n", [(10, 0, 6.0, 1023011), (12, 60, 60.0, 682017), (14, 0, 1.0, 568353)])
+def test_any_hit_ray_counts(built, kind, param, extent, n):
+    """Any hits of open and of instanced scenes stream from larger counts on."""
+    from oracle.oracle import Oracle
+    g = built.Generated(kind, seed=4, param=param)
+    rays = built.generate_rays(n, [-extent] * 3, [extent] * 3, n)
+    s, o = built.Scene(g), Oracle(g.desc)
+    assert np.array_equal(s.trace_any(rays, 0.001, extent), o.trace_any(rays, 0.001, extent))
+
+
+@pytest.mark.parametrize("copies", [8, 15, 16])
+def test_leaf_sizes_of_a_scene_that_streams(built, copies):
+    """As test_leaf_sizes, among enough other triangles for its trees to be walked as streams."""
+    from oracle.oracle import Oracle
+    from photon_tracer_b200 import abi
+    m = [abi.pt_material(type=0, albedo=abi.F3(0.5, 0.5, 0.5))]
+    tris = [tri(built, (-1, -1, 0), (1, -1, 0), (0, 1, 0)) for _ in range(copies)]
+    tris += [tri(built, (x, y, -1), (x + 0.1, y, -1), (x, y + 0.1, -1.2)) for x in np.linspace(-2, 2, 25)
+             for y in np.linspace(-2, 2, 20)]
+    d = scene_from(built, m, [abi.pt_sphere(center=abi.F3(0, 0, -2), radius=0.5)], tris)
+    s, o = built.Scene(d.desc_ptr), Oracle(d.desc)
+    assert 128 * s.info().n_nodes + 48 * s.info().n_slots > 16 << 10
+    rng, n = np.random.default_rng(copies), 240000
+    rays = np.concatenate([rng.uniform(-1, 1, (n, 2)), np.full((n, 1), 2.0), rng.normal(0, 0.3, (n, 2)),
+                           np.full((n, 1), -1.0)], 1).astype(np.float32)
+    assert_hits_equal(s.trace_closest(rays), o.trace_closest(rays, threads=8), rays)
+    assert np.array_equal(s.trace_any(rays), o.trace_any(rays))

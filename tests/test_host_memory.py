@@ -347,3 +347,20 @@ def test_lock_step_renders_borrow_nothing_on_their_usual_streams(fake):
     with fake.failing_above(0):
         d.render(100, 60, 1, 0x9000)
     assert not any(x.startswith("bad") for x in fake.log())
+
+
+@pytest.mark.parametrize("scene,closest,any_hit", [
+    # the ray counts up to which the lock-step kernels answer, in thousands; None: at any size
+    (SPHERES_24, None, None), (FIELD, None, None), (REF_ROOM, None, None), ((15, 0), None, None),
+    (SPHERES_488, 340, 1000), ((10, 2000), 227, 680), ((11, 2), 227, 227), (ROOM_1K, 227, 227), (ROOM_80K, 227, 227),
+    ((12, 60), 340, 680), (INSTANCES, 227, 680), ((12, 2000), 227, 340), ((14, 0), 227, 568)])
+def test_which_ray_queries_stream(fake, scene, closest, any_hit):
+    """Closest and any hits take the kernel that was measured faster for that many rays in scenes like these."""
+    d = DeviceScene(*scene)
+    fake.log()
+    for query, line in (("closest", closest), ("any", any_hit)):
+        fn = getattr(fake.lib, f"pt_trace_{query}_device")
+        for n in (1000, 120000, (line or 2500) * 1000 - 2000, (line or 2500) * 1000 + 25000, 16000000):
+            assert fn(d.s.handle, SOME, n, 0.001, 1000.0, SOME, None) == 0
+            form = "stream" if line and n > line * 1000 else "lock-step"
+            assert fake.log() == [f"{query} {form}"], n
