@@ -282,6 +282,28 @@ void plan_stream(pt_batch* b) {
     b->sample_bytes = size_t(most) * 12;
 }
 
+// Whether the batch renders faster as streams of samples: it does with enough
+// samples to fill the lanes (12 scenes of 256^2 and 512^2 pixels, 4 to 16
+// samples: 32.7 -> 26.2 ms; 3 scenes, 190,000 samples: 0.70 ms lock-step, 0.73
+// streaming) where some of its scenes gain (rooms 0.7-0.8 of the time with 4
+// samples), which outweighs what the others lose (a few spheres: 4 frames of
+// 512^2, 3 to 8 samples, 1.05-1.07). With one launch for all, a scene gains from
+// 3 samples per pixel on (8 frames of 128^2: 24 spheres 0.94, 2,000 spheres
+// 0.93), larger trees from 2 (0.78-0.97; spheres 1.02-1.10, textured rooms
+// 1.04-1.09), if a frame of the batch's pixels would.
+bool stream_gains(const pt_batch* b, const std::vector<uint32_t>& kib, const std::vector<char>& textured) {
+    uint64_t gaining = 0;
+    for (size_t i = 0; i < b->scenes.size(); ++i) {
+        const PtBatchScene& s = b->scenes[i];
+        if (int(s.depth) < 1 || int(s.depth) > PT_SAMPLES_MAX_DEPTH) return false;
+        const bool large = kib[i] > (s.sky ? 256u : 64u) && !textured[i];
+        if ((s.spp >= 3 || (s.spp == 2 && large)) &&
+            pt::stream_gains(kib[i], s.sky != 0, std::max(4, int(s.spp)), int(s.depth), b->total_pixels, false, b->sms))
+            gaining += uint64_t(s.width) * s.height * s.spp;
+    }
+    return 8 * gaining >= b->total_samples && b->total_samples >= 2 * b->total_pixels && b->total_samples >= (1u << 18);
+}
+
 // Plans the streaming launches and gets the memory they need; without it the
 // batch has none, and the lock-step form renders.
 pt_status make_stream(pt_batch* b) {
@@ -461,6 +483,8 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     uint64_t out_floats = 0;
     uint32_t items_total = 0;
     uint32_t stack_need = 0;
+    std::vector<uint32_t> kib;  // of each scene's trees
+    std::vector<char> textured;
     for (uint32_t i = 0; i < n; ++i) {
         const pt_batch_item& it = items[i];
         if (!it.desc) return fail(PT_ERR_INVALID_ARG, "pt_batch_create: item without a scene");
@@ -474,6 +498,8 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
             return fail(PT_ERR_OUT_OF_MEMORY, "pt_batch_create: out of host memory");
         }
         stack_need = std::max(stack_need, A.stack_entries);
+        kib.push_back(tree_kib(A.nodes, A.slots));
+        textured.push_back(A.has_textures != 0);
         PtBatchScene s = merge(all, A);
         const uint32_t tiles_x = uint32_t((it.width + 7) / 8), tiles_y = uint32_t((it.height + 3) / 4);
         s.width = uint32_t(it.width);
@@ -598,15 +624,7 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
         if (err) return cuda_fail(err, "pt_batch_create: scene views");
     }
     if (stack_need > PT_STACK_MAX) return fail(PT_ERR_STACK_OVERFLOW, "pt_batch_create: a scene's BVH is too deep");
-    // The streaming form needs stack words that fit and, to gain from samples
-    // in flight, several per pixel and enough of them to fill the lanes
-    // (12 scenes of 256^2 and 512^2 pixels, 4 to 16 samples: 32.7 -> 26.2 ms;
-    // 3 scenes, 190,000 samples: 0.70 ms lock-step, 0.73 streaming); without
-    // memory for its buffer the lock-step form renders.
-    bool depths = true;
-    for (const PtBatchScene& sc : b->scenes) depths &= int(sc.depth) > 0 && int(sc.depth) <= PT_SAMPLES_MAX_DEPTH;
-    const bool wants_stream =
-        D.words && depths && b->total_samples >= 2 * b->total_pixels && b->total_samples >= (1u << 18);
+    const bool wants_stream = D.words && stream_gains(b, kib, textured);
     // Per-scene scenes for the strategies that launch scene by scene. They come
     // before the buffer of samples, which the batch can do without.
     if (strategy != PT_BATCH_ONE_LAUNCH) {

@@ -364,3 +364,23 @@ def test_which_ray_queries_stream(fake, scene, closest, any_hit):
             assert fn(d.s.handle, SOME, n, 0.001, 1000.0, SOME, None) == 0
             form = "stream" if line and n > line * 1000 else "lock-step"
             assert fake.log() == [f"{query} {form}"], n
+
+
+@pytest.mark.parametrize("scenes,streams", [
+    # (scene, frame's width and height, samples, bounces), as often as given
+    ([(SPHERES_24, 256, 2, 10)] * 8, False), ([(SPHERES_24, 512, 8, 10)] * 4, False),
+    ([(SPHERES_24, 128, 3, 10)] * 8, True), ([((10, 2000), 256, 2, 10)] * 8, False),
+    ([((10, 2000), 256, 3, 10)] * 8, True), ([(ROOM_1K, 256, 2, 10)] * 8, True), ([(ROOM_1K, 512, 4, 2)] * 4, False),
+    ([((14, 0), 256, 2, 10)] * 8, False), ([((14, 0), 256, 4, 10)] * 8, True),
+    ([(SPHERES_24, 512, 8, 10)] * 3 + [(ROOM_1K, 512, 8, 10)], True), ([(ROOM_1K, 128, 4, 10)] * 3, False),
+    ([(ROOM_1K, 256, 2, 0)] * 8, False)])
+def test_which_batches_stream(fake, scenes, streams):
+    """Batches take the form that was measured faster for scenes like theirs."""
+    import photon_tracer_b200 as pt
+    items = []
+    for k, ((kind, param), side, spp, _) in enumerate(scenes):
+        g = pt.Generated(kind, seed=k + 1, param=param)
+        items.append((g, g.camera, side, side, spp, k))
+    b = pt.Batch(items, ONE_LAUNCH, max_bounces=scenes[0][3])
+    assert one_launch_lines(fake, b) == ["batch stream" if streams else "batch 128"]
+    b.close()
