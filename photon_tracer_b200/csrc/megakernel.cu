@@ -98,6 +98,11 @@ template <bool AUX, bool SNAP, int TREES, bool TEX, bool EXT>
 __global__ void __launch_bounds__(128, PT_MEGA_MIN_BLOCKS) megakernel(PtSceneDev S, PtRenderParams P, uint32_t tiles_x,
                                                   uint32_t total_items) {
     PT_FORM_STACK(stack, TREES, 128, PT_MEGA_SH_STACK, PT_MEGA_SH_STACK8);
+    // With the extended light sampling, SMALL but for the large flat scenes and
+    // textures (640x360, us, SMALL and FULL: room of 81,920 triangles, 8 samples
+    // 5,240, 4,960; textured room with guides, 1 sample 1,171, 1,086; but 488
+    // spheres, 8 samples 1,900, 2,550, the emissive meshes 4,700, 5,770).
+    constexpr int CODE = !EXT ? CODE_LOOP : TEX || TREES == PT_TREES_FLAT8 ? CODE_FULL : CODE_SMALL;
     // the traversal form the queries compile (PT_TREES_FLAT8 is the flat one
     // with the other stack)
     constexpr int QT = TREES == PT_TREES_FLAT8 ? int(PT_TREES_FLAT) : TREES;
@@ -207,7 +212,7 @@ __global__ void __launch_bounds__(128, PT_MEGA_MIN_BLOCKS) megakernel(PtSceneDev
         }
 
         if constexpr (ONE_QUERY) {
-            if (in_path && query_trip<AUX, TEX, EXT>(S, path, P.depth, smp, rng, first, pend, shadow_pending,
+            if (in_path && query_trip<AUX, TEX, EXT, CODE>(S, path, P.depth, smp, rng, first, pend, shadow_pending,
                                                 done_after_shadow, stack, rays, overflow)) {
                 acc = acc + path.rad;
                 if (AUX) {
@@ -236,7 +241,7 @@ __global__ void __launch_bounds__(128, PT_MEGA_MIN_BLOCKS) megakernel(PtSceneDev
             if (hit) fill<TEX, EXT>(S, h, path.o, path.d, t, rec);
             bool nee;
             Shadow sh;
-            const int step = shade<AUX, TEX, EXT>(S, path, hit, rec, P.depth, smp, rng, first, nee, sh, rays);
+            const int step = shade<AUX, TEX, EXT, CODE>(S, path, hit, rec, P.depth, smp, rng, first, nee, sh, rays);
             if (nee) {
                 bool ovf = false;
                 if (!occluded<false, QT>(S, sh.o, sh.d, 0.001f, sh.t_max, stack, cnt, &ovf))

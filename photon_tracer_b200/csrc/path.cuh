@@ -107,6 +107,8 @@ __device__ __forceinline__ uint32_t pick_light_ext(const PtSceneDev& S, float u)
 // cosine, the albedo applied by the caller); metal = true the rough-metal one
 // (the lobe density at the direction, weighted against the metal's own
 // scattered ray by the power heuristic). False when no shadow ray is needed.
+// ONE: one draw in the code for both kinds of light.
+template <bool ONE>
 __device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec& rec, bool metal, V mirror, float fuzz,
                                                  const Sampler& smp, Rng& rng, Shadow& sh,
                                                  unsigned long long& rays) {
@@ -125,8 +127,8 @@ __device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec&
         r2 = cr.w * cr.w;
         if (dist2 <= r2) return false;
     }
-    float s1, s2;  // one draw in the code for both kinds of light
-    smp.sample_2d(1, rng, s1, s2);
+    float s1, s2;
+    if (ONE) smp.sample_2d(1, rng, s1, s2);
     if (sphere) {
         const V center = xyz(cr);
         const float sin2_max = r2 / dist2;
@@ -135,6 +137,7 @@ __device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec&
         const V w = div(to_center, sqrtf(dist2));
         const V a = fabsf(w.x) > 0.9f ? mk(0, 1, 0) : mk(1, 0, 0);
         const V u = normalize(cross(w, a)), v = cross(w, u);
+        if (!ONE) smp.sample_2d(1, rng, s1, s2);
         const float cos_t = 1 - s1 * one_minus_cos_max;
         const float sin_t = sqrtf(fmaxf(0.0f, 1 - cos_t * cos_t));
         float sp, cp;
@@ -154,6 +157,7 @@ __device__ __forceinline__ bool direct_light_ext(const PtSceneDev& S, const Rec&
     } else {
         const PtTriLight* L = S.tri_lights + (k - S.n_lights);
         const float4 pa = __ldg(&L->p0_area), e1 = __ldg(&L->e1_er), e2 = __ldg(&L->e2_eg), fe = __ldg(&L->fn_eb);
+        if (!ONE) smp.sample_2d(1, rng, s1, s2);
         const float sq = sqrtf(s1);
         const V y = xyz(pa) + xyz(e1) * (1 - sq) + xyz(e2) * (s2 * sq);
         const V dv = y - rec.p;
@@ -229,21 +233,21 @@ enum : int { STEP_CONTINUE = 0, STEP_DONE = 1 };
 // record (or a miss). Sets *nee and sh when a shadow ray must be tested, with
 // sh.value already multiplied by throughput * attenuation; the caller adds it
 // to p.rad if the ray is not blocked. Returns STEP_DONE when the path ends.
-template <bool AUX, bool TEX = true, bool EXT = false>
+template <bool AUX, bool TEX = true, bool EXT = false, int CODE = EXT ? CODE_SMALL : CODE_LOOP>
 __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, const Rec& rec, int depth,
                                      const Sampler& smp, Rng& rng, First& first, bool& nee, Shadow& sh,
                                      unsigned long long& rays) {
-    // With the extended light sampling the code is large enough for
-    // instruction fetch to bound it, so the normalized incoming direction that
-    // the sky, metal and glass need has one copy there (77 -> 74 KB with the
-    // other SMALL forms: 640x360, 16 samples 8.6 -> 7.3 ms; without it they
-    // only cost registers: room frame +9%).
+    // CODE_SMALL's normalized incoming direction is what the sky, metal and glass
+    // need. In the extended light sampling's streaming kernel it and the single
+    // draws took 640x360, 16 samples from 8.6 to 7.1 ms; without that sampling
+    // they only cost registers: room frame +9%.
+    constexpr bool SMALL = CODE == CODE_SMALL;
     nee = false;
     V unit = p.d;
-    if (EXT && (hit ? fbits(__ldg(&S.mat[rec.mat].albedo_type.w)) != PT_MAT_LAMBERTIAN : S.sky != 0)) unit = normalize(p.d);
+    if (SMALL && (hit ? fbits(__ldg(&S.mat[rec.mat].albedo_type.w)) != PT_MAT_LAMBERTIAN : S.sky != 0)) unit = normalize(p.d);
     if (!hit) {
         if (AUX && p.bounce == 0) first = {mk(1, 1, 1), mk(0, 0, 0)};
-        p.rad = p.rad + p.tp * background<EXT>(S, unit);
+        p.rad = p.rad + p.tp * background<SMALL>(S, unit);
         return STEP_DONE;
     }
     const PtMaterial* m = S.mat + rec.mat;
@@ -264,7 +268,7 @@ __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, con
         }
     }
     V att, dir;
-    const bool scatters = scatter<EXT>(mat, type, unit, rec, smp, rng, att, dir);
+    const bool scatters = scatter<CODE>(mat, type, unit, rec, smp, rng, att, dir);
     if (TEX && S.has_textures && type == PT_MAT_LAMBERTIAN) {  // albedo * texture->sample(tex_u, tex_v) (:72)
         const uint32_t tex = fbits(mat.ior_flags.z);
         if (tex != PT_NONE) att = att * sample_texture(S, tex, rec.tex_u, rec.tex_v);
@@ -276,22 +280,37 @@ __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, con
         const float fuzz = mat.emission_fuzz.w;
         // Rough metal samples a light whether or not the scatter itself is
         // absorbed, so the light estimate does not depend on the scatter's
-        // outcome; a matte surface when it scatters. One copy of the sample
-        // for both (a second one made the kernel 15% larger, and it is
-        // instruction fetch that bounds it).
+        // outcome; a matte surface when it scatters.
         const bool metal = type == PT_MAT_METAL && fuzz > 1e-3f && can;
-        V mirror = mk(0, 0, 0);
         p.mis_pdf = 0;
-        if (metal) {
-            mirror = reflect(unit, rec.normal);
-            if (scatters) p.mis_pdf = metal_lobe_pdf(mirror, fuzz, normalize(dir));
+        if (CODE == CODE_FULL) {
+            if (metal) {
+                const V mirror = reflect(normalize(p.d), rec.normal);
+                if (direct_light_ext<false>(S, rec, true, mirror, fuzz, smp, rng, sh, rays)) {
+                    nee = true;
+                    sh.value = (p.tp * att) * sh.value;
+                }
+                if (scatters) p.mis_pdf = metal_lobe_pdf(mirror, fuzz, normalize(dir));
+            }
+            if (!scatters) return STEP_DONE;
+            p.sampled = (flags & PT_MF_DIFFUSE) && can;
+            if (p.sampled && direct_light_ext<false>(S, rec, false, mk(0, 0, 0), 0.0f, smp, rng, sh, rays)) {
+                nee = true;
+                sh.value = (p.tp * att) * sh.value;
+            }
+        } else {
+            V mirror = mk(0, 0, 0);
+            if (metal) {
+                mirror = reflect(SMALL ? unit : normalize(p.d), rec.normal);
+                if (scatters) p.mis_pdf = metal_lobe_pdf(mirror, fuzz, normalize(dir));
+            }
+            p.sampled = scatters && (flags & PT_MF_DIFFUSE) && can;
+            if ((metal || p.sampled) && direct_light_ext<true>(S, rec, metal, mirror, fuzz, smp, rng, sh, rays)) {
+                nee = true;
+                sh.value = (p.tp * att) * sh.value;
+            }
+            if (!scatters) return STEP_DONE;
         }
-        p.sampled = scatters && (flags & PT_MF_DIFFUSE) && can;
-        if ((metal || p.sampled) && direct_light_ext(S, rec, metal, mirror, fuzz, smp, rng, sh, rays)) {
-            nee = true;
-            sh.value = (p.tp * att) * sh.value;
-        }
-        if (!scatters) return STEP_DONE;
     } else {
         if (!scatters) return STEP_DONE;
         p.sampled = (flags & PT_MF_DIFFUSE) && S.sample_lights && S.n_lights > 0 && p.bounce + 1 < depth;
@@ -325,7 +344,7 @@ __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, con
 // results are those of the inline form. The pending shadow ray (origin,
 // direction, t_max, unblocked value) of each thread sits in shared memory,
 // column threadIdx.x of pend. Returns true when the path has ended.
-template <bool AUX, bool TEX, bool EXT, int N, class Stack>
+template <bool AUX, bool TEX, bool EXT, int CODE, int N, class Stack>
 __device__ __forceinline__ bool query_trip(const PtSceneDev& S, Path& path, int depth, Sampler& smp, Rng& rng,
                                            First& first, float (&pend)[10][N], bool& shadow_pending,
                                            bool& done_after_shadow, Stack& stack, unsigned long long& rays,
@@ -360,7 +379,7 @@ __device__ __forceinline__ bool query_trip(const PtSceneDev& S, Path& path, int 
     if (hit) fill<TEX, EXT>(S, h, path.o, path.d, tq, rec);
     bool nee;
     Shadow sh;
-    const bool done = shade<AUX, TEX, EXT>(S, path, hit, rec, depth, smp, rng, first, nee, sh, rays) == STEP_DONE;
+    const bool done = shade<AUX, TEX, EXT, CODE>(S, path, hit, rec, depth, smp, rng, first, nee, sh, rays) == STEP_DONE;
     if (!nee) return done;
     pend[0][t] = sh.o.x;
     pend[1][t] = sh.o.y;

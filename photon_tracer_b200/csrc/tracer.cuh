@@ -1214,6 +1214,16 @@ __device__ __forceinline__ V refract(V uv, V n, float ratio) {
     const V r_parallel = n * -sqrtf(fabsf(1 - dot(r_perp, r_perp)));
     return r_perp + r_parallel;
 }
+
+// How a kernel's shading code is written out. Instruction fetch bounds the
+// larger kernels, and which of these is fastest is a matter of the kernel:
+// CODE_FULL   the compiler unrolls the rejection loop, and the extended light
+//             sampling has a copy for matte surfaces and one for rough metal;
+// CODE_LOOP   one copy of the rejection loop's draw;
+// CODE_SMALL  also one copy of the extended light sampling and of its draws,
+//             and of the normalized incoming direction.
+enum : int { CODE_FULL = 0, CODE_LOOP = 1, CODE_SMALL = 2 };
+
 // random_in_unit_sphere (vec3.hpp:121-127). vec3::random(-1, 1) builds the
 // vector from three calls in one constructor argument list, which GCC on
 // x86-64 evaluates right to left: z is drawn first, x last. The rejection
@@ -1221,18 +1231,30 @@ __device__ __forceinline__ V refract(V uv, V n, float ratio) {
 // real stream, but an all-zero xoshiro state (which a caller could supply
 // as a snapshot) repeats (-1,-1,-1) forever; the bound turns that into a
 // zero offset instead of a hung kernel.
-template <bool SMALL = false>  // one copy of the draw in the code, in a loop
+__device__ __forceinline__ V random_vector(Rng& rng) {
+    V p;
+    p.z = -1.0f + 2.0f * rng.real();
+    p.y = -1.0f + 2.0f * rng.real();
+    p.x = -1.0f + 2.0f * rng.real();
+    return p;
+}
+template <int CODE = CODE_LOOP>
 __device__ __forceinline__ V random_in_unit_sphere(Rng& rng) {
+    if (CODE == CODE_FULL) {
+        for (int tries = 0; tries < 64; ++tries) {
+            const V p = random_vector(rng);
+            if (dot(p, p) < 1) return p;
+        }
+        return mk(0, 0, 0);
+    }
 #pragma unroll 1
     for (int tries = 0; tries < 64; ++tries) {
         V p = mk(0, 0, 0);
-        if (SMALL) {
+        if (CODE == CODE_SMALL) {
 #pragma unroll 1
             for (int k = 0; k < 3; ++k) p = mk(-1.0f + 2.0f * rng.real(), p.x, p.y);
         } else {
-            p.z = -1.0f + 2.0f * rng.real();
-            p.y = -1.0f + 2.0f * rng.real();
-            p.x = -1.0f + 2.0f * rng.real();
+            p = random_vector(rng);
         }
         if (dot(p, p) >= 1) continue;
         return p;
@@ -1241,9 +1263,9 @@ __device__ __forceinline__ V random_in_unit_sphere(Rng& rng) {
 }
 
 // material::scatter for the four kinds: lambertian :59-74, metal :85-91,
-// diffuse_light :97-102, dielectric :113-136. SMALL: d_in is normalized
-// already, and the code is kept small.
-template <bool SMALL = false>
+// diffuse_light :97-102, dielectric :113-136. CODE_SMALL: d_in is normalized
+// already.
+template <int CODE = CODE_LOOP>
 __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_in, const Rec& rec,
                                         const Sampler& smp, Rng& rng, V& attenuation, V& dir) {
     if (type == PT_MAT_LAMBERTIAN) {
@@ -1262,8 +1284,8 @@ __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_
         return true;
     }
     if (type == PT_MAT_METAL) {
-        const V reflected = reflect(SMALL ? d_in : normalize(d_in), rec.normal);
-        dir = reflected + random_in_unit_sphere<SMALL>(rng) * m.emission_fuzz.w;
+        const V reflected = reflect(CODE == CODE_SMALL ? d_in : normalize(d_in), rec.normal);
+        dir = reflected + random_in_unit_sphere<CODE>(rng) * m.emission_fuzz.w;
         attenuation = xyz(m.albedo_type);
         return dot(dir, rec.normal) > 0;
     }
@@ -1271,7 +1293,7 @@ __device__ __forceinline__ bool scatter(const PtMaterial& m, uint32_t type, V d_
         attenuation = mk(1, 1, 1);
         const float ior = m.ior_flags.x;
         const float ratio = rec.front_face ? (1 / ior) : ior;
-        const V unit = SMALL ? d_in : normalize(d_in);
+        const V unit = CODE == CODE_SMALL ? d_in : normalize(d_in);
         const float cos_theta = fminf(dot(-unit, rec.normal), 1.0f);
         const float sin_theta = sqrtf(1 - cos_theta * cos_theta);
         const bool cannot_refract = ratio * sin_theta > 1;
