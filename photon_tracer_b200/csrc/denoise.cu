@@ -147,6 +147,89 @@ __global__ void __launch_bounds__(kTX* kTY) atrous_pass(
     }
 }
 
+struct Pixel {
+    float4 lv;
+    float n0, n1, n2, a0, a1, a2, l;  // normal, albedo, luminance
+    bool sky;
+};
+template <bool ALIGNED>
+__device__ __forceinline__ Pixel load_pixel(const float* __restrict__ lv, const float* __restrict__ nrm,
+                                            const float* __restrict__ albedo, size_t q) {
+    Pixel p;
+    p.lv = load_lv<ALIGNED>(lv, q);
+    p.l = lum(p.lv.x, p.lv.y, p.lv.z);
+    p.n0 = nrm[3 * q];
+    p.n1 = nrm[3 * q + 1];
+    p.n2 = nrm[3 * q + 2];
+    p.a0 = albedo[3 * q];
+    p.a1 = albedo[3 * q + 1];
+    p.a2 = albedo[3 * q + 2];
+    p.sky = p.n0 == 0 && p.n1 == 0 && p.n2 == 0;
+    return p;
+}
+
+// The same pass with a thread per pixel in image order, reading its taps where
+// they are: for strips, which fill few of a tile's lattice columns or rows (the
+// filter in tiles throughout, then as launch_pass chooses: 16x20000 287 ->
+// 153 us, 20000x2 85 -> 46, 48x20000 503 -> 427).
+template <bool ALIGNED, bool LAST>
+__global__ void __launch_bounds__(128) atrous_direct(
+    int w, int h, int step, const float* __restrict__ albedo, const float* __restrict__ nrm,
+    const float* __restrict__ lv, float* __restrict__ lv_next, float* __restrict__ out) {
+    const unsigned p = blockIdx.x * 128u + threadIdx.x;
+    if (p >= unsigned(w) * unsigned(h)) return;
+    const int y = int(p / unsigned(w)), x = int(p - unsigned(y) * unsigned(w));
+    const Pixel c = load_pixel<ALIGNED>(lv, nrm, albedo, p);
+    float v = 0, vw = 0;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            const int qx = x + dx, qy = y + dy;
+            if (qx < 0 || qy < 0 || qx >= w || qy >= h) continue;
+            const float k = (dx ? 0.5f : 1) * (dy ? 0.5f : 1);
+            v += k * lv[4 * (size_t(qy) * w + qx) + 3];
+            vw += k;
+        }
+    const float scale = 1 / (4.0f * sqrtf(v / vw) + 1e-4f);
+    float s0 = 0, s1 = 0, s2 = 0, sum_w = 0, sum_var = 0;
+    const float kernel[3] = {3.0f / 8, 1.0f / 4, 1.0f / 16};
+#pragma unroll 1
+    for (int dy = -2; dy <= 2; ++dy) {
+        const long qy = y + long(dy) * step;
+        if (qy < 0 || qy >= h) continue;
+        const float ky = dy == 0 ? kernel[0] : dy * dy == 1 ? kernel[1] : kernel[2];
+#pragma unroll
+        for (int dx = -2; dx <= 2; ++dx) {
+            const long qx = x + long(dx) * step;
+            if (qx < 0 || qx >= w) continue;
+            const Pixel q = load_pixel<ALIGNED>(lv, nrm, albedo, size_t(qy) * w + qx);
+            if (q.sky != c.sky) continue;
+            float weight = kernel[dx < 0 ? -dx : dx] * ky;
+            if (!c.sky) {
+                float nd = fmaxf(c.n0 * q.n0 + c.n1 * q.n1 + c.n2 * q.n2, 0.0f);
+                for (int k = 0; k < 6; ++k) nd *= nd;
+                weight *= nd;
+            }
+            const float da0 = c.a0 - q.a0, da1 = c.a1 - q.a1, da2 = c.a2 - q.a2;
+            weight *= expf(-(da0 * da0 + da1 * da1 + da2 * da2) * (1 / 0.01f) - fabsf(c.l - q.l) * scale);
+            s0 += weight * q.lv.x;
+            s1 += weight * q.lv.y;
+            s2 += weight * q.lv.z;
+            sum_w += weight;
+            sum_var += weight * weight * q.lv.w;
+        }
+    }
+    const float4 r = make_float4(s0 / sum_w, s1 / sum_w, s2 / sum_w, sum_var / (sum_w * sum_w));
+    if (LAST) {
+        out[3 * size_t(p)] = r.x * fmaxf(c.a0, 0.01f);
+        out[3 * size_t(p) + 1] = r.y * fmaxf(c.a1, 0.01f);
+        out[3 * size_t(p) + 2] = r.z * fmaxf(c.a2, 0.01f);
+    } else {
+        store_lv<ALIGNED>(lv_next, p, r);
+    }
+}
+
 template <bool ALIGNED>
 __global__ void finish(int n, const float* __restrict__ lv, const float* albedo, float* out) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -163,9 +246,21 @@ template <int PH, bool ALIGNED, bool LAST>
 void launch_pass(int w, int h, int step, const float* albedo, const float* nrm, const float* lv, float* lv_next,
                  float* out, cudaStream_t stream) {
     const int lw = (w + step - 1) / step, lh = (h + step - 1) / step, columns = kTX / PH;
-    const int bx = (lw + columns - 1) / columns * (step / PH);
-    const unsigned blocks = unsigned(bx) * unsigned((lh + kTY - 1) / kTY * step);
-    atrous_pass<PH, ALIGNED, LAST><<<blocks, dim3(kTX, kTY), 0, stream>>>(w, h, step, bx, albedo, nrm, lv, lv_next, out);
+    const int tx = (lw + columns - 1) / columns, ty = (lh + kTY - 1) / kTY;
+    const int bx = tx * (step / PH);
+    const unsigned blocks = unsigned(bx) * unsigned(ty * step);
+    // Tiles cost two thirds of a direct pass when full (1920x1080: 138 us, 183),
+    // so they lose where less than two thirds of their pixels are in the image --
+    // unless they are too few to fill the GPU (eight to an SM), where a pass
+    // takes as long as one tile or one pixel, and the tile's loads go out at once
+    // (64x36, the filter: 54 us, 82).
+    const bool filled = 3 * (long(lw) * lh) >= 2 * (long(tx) * columns * ty * kTY);
+    if (!filled && blocks > 148u * 8u)
+        atrous_direct<ALIGNED, LAST><<<unsigned((long(w) * h + 127) / 128), 128, 0, stream>>>(w, h, step, albedo, nrm, lv,
+                                                                                              lv_next, out);
+    else
+        atrous_pass<PH, ALIGNED, LAST><<<blocks, dim3(kTX, kTY), 0, stream>>>(w, h, step, bx, albedo, nrm, lv, lv_next,
+                                                                              out);
 }
 
 template <bool ALIGNED>

@@ -52,3 +52,24 @@ def test_atrous_into_its_scratch(built, at):
     out = scratch[int(at * w * h):][:3 * w * h]
     run(out, scratch)
     assert torch.equal(out.view(h, w, 3), want)
+
+
+@pytest.mark.parametrize("w,h,shift", [(1, 21000, 0), (16, 5003, 1), (33, 20001, 0), (20001, 3, 0), (47, 9001, 2)])
+def test_atrous_strips(built, w, h, shift):
+    """Narrow and flat images, whose wider passes go pixel by pixel."""
+    import torch
+    from oracle.oracle import oracle_denoise
+    from photon_tracer_b200 import abi
+    rng = np.random.default_rng(w)
+    color = rng.gamma(1.0, 0.5, (h, w, 3)).astype(np.float32)
+    albedo = rng.uniform(0, 1, (h, w, 3)).astype(np.float32).round(1)
+    normal = rng.normal(0, 1, (h, w, 3)).astype(np.float32).round(0)
+    normal[rng.uniform(size=(h, w)) < 0.2] = 0
+    variance = rng.gamma(1.0, 0.1, (h, w)).astype(np.float32)
+    want = oracle_denoise(color, albedo, normal, variance)
+    d = [torch.from_numpy(a).cuda() for a in (color, albedo, normal, variance)]
+    scratch, out = torch.empty(11 * w * h + shift, device="cuda")[shift:], torch.empty((h, w, 3), device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    abi.check(built.load().pt_denoise_atrous_device(w, h, *[ptr(t) for t in d], ptr(out), ptr(scratch),
+                                                    C.c_void_p(torch.cuda.current_stream().cuda_stream)))
+    np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-3, atol=1e-5)  # as test_atrous_sizes
