@@ -180,19 +180,19 @@ unet::ConvOut to_cat(pt_unet* n, int l, int up) {
     return o;
 }
 
-// The forward pass from act[0] (the padded input) to act[15] (float, 16
-// channels). The encoder's second convolution at each level also writes
-// its 2x2-pooled output and its copy into the decoder's concatenation; each
-// decoder level's last convolution (and the bottleneck's) writes its
-// upsampled output into the next finer concatenation.
-// image: where to put the image_w x image_h radiance directly (inference with
-// tensor cores; *imaged tells whether that happened, else act[15] holds the
-// output).
+// Where inference wants the w x h radiance; imaged: it was written there.
 struct ImageOut {
     float* image;
     int w, h;
     bool imaged;
 };
+
+// The forward pass from act[0] (the padded input) to act[15] (float, 16
+// channels), or, with tensor cores and an image to write, to that image in
+// its place. The encoder's second convolution at each level also writes its
+// 2x2-pooled output and its copy into the decoder's concatenation; each decoder
+// level's last convolution (and the bottleneck's) writes its upsampled output
+// into the next finer concatenation.
 cudaError_t forward(pt_unet* n, cudaStream_t st, bool training, ImageOut* image = nullptr) {
     cudaError_t e;
     auto A = [&](int i) { return n->act[i].p; };
@@ -238,91 +238,79 @@ cudaError_t forward(pt_unet* n, cudaStream_t st, bool training, ImageOut* image 
     return cudaSuccess;
 }
 
-// Backward from gact[15] (d loss / d output): weight gradients into grads,
-// and d loss / d input into gact[0].
+// The bf16 weights of every layer, flip-transposed.
+cudaError_t transpose_weights(pt_unet* n, cudaStream_t st) {
+    unet::FlipLayers fl{};
+    fl.n = 15;
+    for (int l = 0; l < 15; ++l) {
+        fl.cin[l] = kLayers[l].cin;
+        fl.cout[l] = kLayers[l].cout;
+        fl.off[l] = long(n->w_off[l]);
+    }
+    return unet::flip_transpose_all(fl, n->params16.as<__nv_bfloat16>(), n->wt16.as<__nv_bfloat16>(), st);
+}
+
+// Backward from gact[15] (d loss / d output) on the CUDA cores: weight
+// gradients into grads, and d loss / d input into gact[0].
 cudaError_t backward(pt_unet* n, cudaStream_t st) {
     cudaError_t e;
     const int B = n->B, H = n->H, W = n->W;
     float* G = n->grads.as<float>();
-    // flip-transposed bf16 weights of every layer
-    for (int l = 0; l < 15; ++l)
-        TRY(unet::flip_transpose(kLayers[l].cin, kLayers[l].cout, w16(n, l), n->wt16.as<__nv_bfloat16>() + n->w_off[l],
-                                 st));
+    TRY(transpose_weights(n, st));
     for (int i = 0; i < 15; ++i) TRY(cudaMemsetAsync(n->gact[i].p, 0, n->gact[i].bytes, st));
     auto bf = [&](int i) { return n->act[i].as<__nv_bfloat16>(); };
     auto g = [&](int i) { return n->gact[i].as<float>(); };
-    // One convolution's backward: weight gradients from its input and output
-    // gradient, and the input gradient through the flip-transposed weights.
-    // With tensor cores on, a layer's output gradient is also rounded to bf16
-    // (the copy relu_back, or to_bf16 for the last layer, leaves in g16): its
-    // weight gradient is a tcgen05 GEMM over pixels of that copy and the
-    // layer input, and its input gradient the tcgen05 convolution of that
-    // copy with the flip-transposed weights. Tensor cores off: the float
-    // gradient on CUDA cores.
-    __nv_bfloat16* g16 = n->use_tc ? n->g16.as<__nv_bfloat16>() : nullptr;
-    auto conv_back = [&](int l, const __nv_bfloat16* in, const float* gout, bool gout16, float* gin) -> cudaError_t {
+    // One convolution's backward: weight and bias gradients from its input and
+    // output gradient, and the input gradient through the flip-transposed weights.
+    auto conv_back = [&](int l, const __nv_bfloat16* in, const float* gout, float* gin) -> cudaError_t {
         const LayerDef& L = kLayers[l];
         const unet::ConvShape s{B, H >> L.level, W >> L.level, L.cin, L.cout};
-        cudaError_t r = cudaErrorNotSupported;
-        if (gout16 && g16) {
-            r = unet::conv_wgrad_tc(s, in, g16, G + n->w_off[l], n->status.as<unsigned int>(), st);
-            if (!r) r = unet::bias_grad(pixels_at(n, L.level), L.cout, gout, G + n->b_off[l], st);
-        }
-        if (r == cudaErrorNotSupported) r = unet::conv_wgrad(s, in, gout, G + n->w_off[l], G + n->b_off[l], st);
-        if (r || !gin) return r;
+        if (const cudaError_t r = unet::conv_wgrad(s, in, gout, G + n->w_off[l], G + n->b_off[l], st)) return r;
         const unet::ConvShape t{B, H >> L.level, W >> L.level, L.cout, L.cin};
         const __nv_bfloat16* wt = n->wt16.as<__nv_bfloat16>() + n->w_off[l];
-        if (gout16 && g16) {
-            unet::ConvOut o;
-            o.out = gin;
-            o.stride = L.cin;
-            r = unet::conv_fwd_tc(t, g16, wt, nullptr, false, o, true, n->status.as<unsigned int>(), st);
-            if (r != cudaErrorNotSupported) return r;
-        }
         return unet::conv_fwd(t, gout, true, wt, nullptr, false, gin, true, L.cin, 0, st);
     };
     auto relu_back = [&](int i) {
-        return unet::relu_grad(pixels_at(n, act_level(i)) * act_channels(i), bf(i), g(i), g16, st);
+        return unet::relu_grad(pixels_at(n, act_level(i)) * act_channels(i), bf(i), g(i), st);
     };
-    if (g16) TRY(unet::to_bf16(pixels_at(n, 0) * kOutStride, g(15), g16, st));
-    TRY(conv_back(14, bf(14), g(15), true, g(14)));
+    TRY(conv_back(14, bf(14), g(15), g(14)));
     TRY(relu_back(14));
-    TRY(conv_back(13, bf(13), g(14), true, g(13)));
+    TRY(conv_back(13, bf(13), g(14), g(13)));
     TRY(relu_back(13));
-    TRY(conv_back(12, n->cat[0].as<__nv_bfloat16>(), g(13), true, n->gcat[0].as<float>()));
+    TRY(conv_back(12, n->cat[0].as<__nv_bfloat16>(), g(13), n->gcat[0].as<float>()));
     TRY(unet::up_bwd(B, H / 2, W / 2, 64, n->gcat[0].as<float>(), 96, 0, g(12), st));
     TRY(unet::add_channels(pixels_at(n, 0), 32, n->gcat[0].as<float>(), 96, 64, g(2), st));
     TRY(relu_back(12));
-    TRY(conv_back(11, bf(11), g(12), true, g(11)));
+    TRY(conv_back(11, bf(11), g(12), g(11)));
     TRY(relu_back(11));
-    TRY(conv_back(10, n->cat[1].as<__nv_bfloat16>(), g(11), true, n->gcat[1].as<float>()));
+    TRY(conv_back(10, n->cat[1].as<__nv_bfloat16>(), g(11), n->gcat[1].as<float>()));
     TRY(unet::up_bwd(B, H / 4, W / 4, 96, n->gcat[1].as<float>(), 160, 0, g(10), st));
     TRY(unet::add_channels(pixels_at(n, 1), 64, n->gcat[1].as<float>(), 160, 96, g(4), st));
     TRY(relu_back(10));
-    TRY(conv_back(9, bf(9), g(10), true, g(9)));
+    TRY(conv_back(9, bf(9), g(10), g(9)));
     TRY(relu_back(9));
-    TRY(conv_back(8, n->cat[2].as<__nv_bfloat16>(), g(9), true, n->gcat[2].as<float>()));
+    TRY(conv_back(8, n->cat[2].as<__nv_bfloat16>(), g(9), n->gcat[2].as<float>()));
     TRY(unet::up_bwd(B, H / 8, W / 8, 128, n->gcat[2].as<float>(), 224, 0, g(8), st));
     TRY(unet::add_channels(pixels_at(n, 2), 96, n->gcat[2].as<float>(), 224, 128, g(6), st));
     TRY(relu_back(8));
-    TRY(conv_back(7, bf(7), g(8), true, g(7)));
+    TRY(conv_back(7, bf(7), g(8), g(7)));
     TRY(relu_back(7));
-    TRY(conv_back(6, n->pool[2].as<__nv_bfloat16>(), g(7), true, n->gpool[2].as<float>()));
+    TRY(conv_back(6, n->pool[2].as<__nv_bfloat16>(), g(7), n->gpool[2].as<float>()));
     TRY(unet::pool_bwd(B, H / 4, W / 4, 96, bf(6), n->pool[2].as<__nv_bfloat16>(), n->gpool[2].as<float>(), g(6), st));
     TRY(relu_back(6));
-    TRY(conv_back(5, bf(5), g(6), true, g(5)));
+    TRY(conv_back(5, bf(5), g(6), g(5)));
     TRY(relu_back(5));
-    TRY(conv_back(4, n->pool[1].as<__nv_bfloat16>(), g(5), true, n->gpool[1].as<float>()));
+    TRY(conv_back(4, n->pool[1].as<__nv_bfloat16>(), g(5), n->gpool[1].as<float>()));
     TRY(unet::pool_bwd(B, H / 2, W / 2, 64, bf(4), n->pool[1].as<__nv_bfloat16>(), n->gpool[1].as<float>(), g(4), st));
     TRY(relu_back(4));
-    TRY(conv_back(3, bf(3), g(4), true, g(3)));
+    TRY(conv_back(3, bf(3), g(4), g(3)));
     TRY(relu_back(3));
-    TRY(conv_back(2, n->pool[0].as<__nv_bfloat16>(), g(3), true, n->gpool[0].as<float>()));
+    TRY(conv_back(2, n->pool[0].as<__nv_bfloat16>(), g(3), n->gpool[0].as<float>()));
     TRY(unet::pool_bwd(B, H, W, 32, bf(2), n->pool[0].as<__nv_bfloat16>(), n->gpool[0].as<float>(), g(2), st));
     TRY(relu_back(2));
-    TRY(conv_back(1, bf(1), g(2), true, g(1)));
+    TRY(conv_back(1, bf(1), g(2), g(1)));
     TRY(relu_back(1));
-    TRY(conv_back(0, bf(0), g(1), true, g(0)));
+    TRY(conv_back(0, bf(0), g(1), g(0)));
     return cudaSuccess;
 }
 
@@ -365,15 +353,8 @@ cudaError_t loss_backward_tc(pt_unet* n, const float* target, bool input_grad, c
         if (!fgrad) std::swap(cur, other);
         return r;
     };
-    unet::FlipLayers fl{};
-    fl.n = 15;
-    for (int l = 0; l < 15; ++l) {
-        fl.cin[l] = kLayers[l].cin;
-        fl.cout[l] = kLayers[l].cout;
-        fl.off[l] = long(n->w_off[l]);
-    }
     const int cat_c[3] = {96, 160, 224};
-    TRY(unet::flip_transpose_all(fl, n->params16.as<__nv_bfloat16>(), n->wt16.as<__nv_bfloat16>(), st));
+    TRY(transpose_weights(n, st));
     TRY(unet::l1_back(pixels_at(n, 0), n->act[15].as<float>(), target, n->g4.as<float4>(), cur, db(14),
                       n->loss.as<float>(), st));
     TRY(wgrad(14, bf(14)));

@@ -16,11 +16,8 @@ cudaError_t conv_fwd(const ConvShape& s, const void* in, bool in_f32, const __nv
 // dw += d loss / d w, db += d loss / d bias, from the layer input and the gradient of its output.
 cudaError_t conv_wgrad(const ConvShape& s, const __nv_bfloat16* in, const float* dout, float* dw, float* db,
                        cudaStream_t st);
-// db[c] += sum over pixels of g[p][c], g NHWC float with C <= 256 channels.
-cudaError_t bias_grad(long pixels, int C, const float* g, float* db, cudaStream_t st);
-cudaError_t flip_transpose(int Cin, int Cout, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t st);
-cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, __nv_bfloat16* g16, cudaStream_t st);
-cudaError_t to_bf16(long n, const float* g, __nv_bfloat16* g16, cudaStream_t st);
+// Gradient through a ReLU: g = 0 where its output y is not positive.
+cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, cudaStream_t st);
 cudaError_t pool_fwd(int B, int H, int W, int C, const __nv_bfloat16* in, __nv_bfloat16* out, cudaStream_t st);
 cudaError_t pool_bwd(int B, int H, int W, int C, const __nv_bfloat16* in, const __nv_bfloat16* out,
                      const float* gout, float* gin, cudaStream_t st);
@@ -58,7 +55,8 @@ cudaError_t up_back(int B, int h, int w, int C, const float* gcat, int stride, c
 // [offset, offset + C) of gcat and through its 2x2 max pool.
 cudaError_t skip_back(int B, int H, int W, int C, const float* gcat, int stride, int offset, const __nv_bfloat16* y,
                       const __nv_bfloat16* pooled, const float* gpool, __nv_bfloat16* g16, float* db, cudaStream_t st);
-// flip_transpose of every layer in one launch.
+// w_t[ci][tap][co] = w[co][8 - tap][ci] of every layer: the weights of the
+// transposed convolutions that carry gradients back to a layer's input.
 struct FlipLayers {
     int n, cin[16], cout[16];
     long off[16];

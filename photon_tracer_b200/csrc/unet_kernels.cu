@@ -136,52 +136,10 @@ __global__ void __launch_bounds__(256) conv_wgrad_kernel(int B, int H, int W, in
     if (db && tap == 0 && ci0 == 0 && t < kCoTile && co0 + t < Cout) atomicAdd(&db[co0 + t], bacc);
 }
 
-// db[c] += sum over pixels of g[p][c] (C <= 256): R = 256 / C rows of
-// threads per block stride over the block's pixels, then one row sums.
-__global__ void __launch_bounds__(256) bias_grad_kernel(long pixels, int C, const float* __restrict__ g,
-                                                        float* __restrict__ db, long px_per_block) {
-    __shared__ float part[256];
-    const int R = 256 / C;
-    const int t = threadIdx.x, c = t % C, r = t / C;
-    const long p0 = long(blockIdx.x) * px_per_block;
-    const long p1 = p0 + px_per_block < pixels ? p0 + px_per_block : pixels;
-    float acc = 0.0f;
-    if (r < R)
-        for (long p = p0 + r; p < p1; p += R) acc += g[p * C + c];
-    part[t] = acc;
-    __syncthreads();
-    if (r == 0) {
-        for (int k = 1; k < R; ++k) acc += part[k * C + c];
-        atomicAdd(db + c, acc);
-    }
-}
-
-// w_t[ci][tap][co] = w[co][8 - tap][ci]: the weights of the transposed
-// convolution that carries gradients back to a layer's input.
-__global__ void flip_transpose_kernel(int Cin, int Cout, const __nv_bfloat16* __restrict__ w,
-                                      __nv_bfloat16* __restrict__ wt) {
-    const long n = long(Cin) * 9 * Cout;
-    for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x) {
-        const int co = int(i % Cout);
-        const int tap = int((i / Cout) % 9);
-        const int ci = int(i / (long(Cout) * 9));
-        wt[i] = w[(size_t(co) * 9 + (8 - tap)) * Cin + ci];
-    }
-}
-
-// Gradient through ReLU: g *= (y > 0), converted to bf16 for the next conv.
-__global__ void relu_grad_kernel(long n, const __nv_bfloat16* __restrict__ y, float* __restrict__ g,
-                                 __nv_bfloat16* __restrict__ g16) {
-    for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x) {
-        const float v = __bfloat162float(y[i]) > 0.0f ? g[i] : 0.0f;
-        g[i] = v;
-        if (g16) g16[i] = __float2bfloat16_rn(v);
-    }
-}
-
-__global__ void to_bf16_kernel(long n, const float* __restrict__ g, __nv_bfloat16* __restrict__ g16) {
+// Gradient through ReLU: g *= (y > 0).
+__global__ void relu_grad_kernel(long n, const __nv_bfloat16* __restrict__ y, float* __restrict__ g) {
     for (long i = blockIdx.x * long(blockDim.x) + threadIdx.x; i < n; i += long(gridDim.x) * blockDim.x)
-        g16[i] = __float2bfloat16_rn(g[i]);
+        g[i] = __bfloat162float(y[i]) > 0.0f ? g[i] : 0.0f;
 }
 
 // 2x2 max pooling (H, W even).
@@ -652,27 +610,8 @@ cudaError_t conv_wgrad(const ConvShape& s, const __nv_bfloat16* in, const float*
     return cudaGetLastError();
 }
 
-cudaError_t bias_grad(long pixels, int C, const float* g, float* db, cudaStream_t st) {
-    if (C < 1 || C > 256) return cudaErrorInvalidValue;
-    const long per = 4096;
-    const long blocks = (pixels + per - 1) / per;
-    bias_grad_kernel<<<unsigned(blocks > 0 ? blocks : 1), 256, 0, st>>>(pixels, C, g, db, per);
-    return cudaGetLastError();
-}
-
-cudaError_t flip_transpose(int Cin, int Cout, const __nv_bfloat16* w, __nv_bfloat16* wt, cudaStream_t st) {
-    const long n = long(Cin) * 9 * Cout;
-    flip_transpose_kernel<<<grid1(n), 256, 0, st>>>(Cin, Cout, w, wt);
-    return cudaGetLastError();
-}
-
-cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, __nv_bfloat16* g16, cudaStream_t st) {
-    relu_grad_kernel<<<grid1(n), 256, 0, st>>>(n, y, g, g16);
-    return cudaGetLastError();
-}
-
-cudaError_t to_bf16(long n, const float* g, __nv_bfloat16* g16, cudaStream_t st) {
-    to_bf16_kernel<<<grid1(n), 256, 0, st>>>(n, g, g16);
+cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, cudaStream_t st) {
+    relu_grad_kernel<<<grid1(n), 256, 0, st>>>(n, y, g);
     return cudaGetLastError();
 }
 

@@ -117,7 +117,9 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 
 // UMMA descriptor of a K-major operand without swizzle: core matrices of
 // 8 rows x 16 bytes stored as 128 contiguous bytes, `lbo` bytes between the
-// two core matrices of a K = 16 step, `sbo` bytes between 8-row groups.
+// two core matrices of a K = 16 step, `sbo` bytes between 8-row groups. An
+// MN-major operand (the weight gradients') takes `lbo` between groups of 8 K
+// indices and `sbo` between groups of 8 rows of M or N.
 __device__ __forceinline__ uint64_t plain_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
     return uint64_t((addr >> 4) & 0x3fff) | (uint64_t((lbo >> 4) & 0x3fff) << 16) |
            (uint64_t((sbo >> 4) & 0x3fff) << 32) | (uint64_t(1) << 46);
@@ -605,12 +607,6 @@ constexpr uint32_t kWgPlane = kHaloTX * kHaloTY * 16;  // 2,048 bytes: 8 channel
 constexpr uint32_t kWgA = 16 * kWgPlane;               // what an M = 128 operand spans
 constexpr int kWgCols = 512;                           // 9 x 32 columns, a power of two
 
-// UMMA descriptor of an MN-major operand without swizzle: `lbo` bytes between
-// groups of 8 K indices, `sbo` bytes between groups of 8 rows of M or N.
-__device__ __forceinline__ uint64_t mn_plain_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return plain_desc(addr, lbo, sbo);
-}
-
 __device__ __forceinline__ void red_add4(float* p, float a, float b, float c, float d) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
@@ -701,11 +697,11 @@ __global__ void __launch_bounds__(kThreads) wgrad_tc_kernel(const __grid_constan
                 fence_after();
                 const uint32_t st = smem_u32(smem + s * stage_bytes), sx = st + dy_bytes;
                 for (int r = 0; r < kHaloTY; r += 2) {  // K = 16: two rows of 8 pixels
-                    const uint64_t ad = mn_plain_desc(st + r * (kHaloTX * 16), kHaloTX * 16, kWgPlane);
+                    const uint64_t ad = plain_desc(st + r * (kHaloTX * 16), kHaloTX * 16, kWgPlane);
 #pragma unroll
                     for (int tap = 0; tap < kWgTaps; ++tap)
                         mma_bf16(tmem + tap * kWgN, ad,
-                                 mn_plain_desc(sx + ((r + tap / 3) * kHaloW + tap % 3) * 16, kHaloW * 16, kPlane), idesc,
+                                 plain_desc(sx + ((r + tap / 3) * kHaloW + tap % 3) * 16, kHaloW * 16, kPlane), idesc,
                                  (it | r) != 0);
                 }
                 mma_commit(empty0 + 8 * s);

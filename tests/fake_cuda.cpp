@@ -247,16 +247,11 @@ cudaError_t conv_wgrad_tc(const ConvShape& s, const __nv_bfloat16* in, const __n
     if (!g_tensor_cores) return cudaErrorNotSupported;
     return launch("wgrad tc", {{in, px(s) * s.Cin * 2}, {g, px(s) * s.Cout * 2}});
 }
-cudaError_t bias_grad(long, int, const float*, float*, cudaStream_t) { return kernel("bias_grad"); }
-cudaError_t flip_transpose(int, int, const __nv_bfloat16*, __nv_bfloat16*, cudaStream_t) { return kernel("flip"); }
 cudaError_t flip_transpose_all(const FlipLayers&, const __nv_bfloat16*, __nv_bfloat16*, cudaStream_t) {
     return kernel("flip all");
 }
-cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, __nv_bfloat16*, cudaStream_t) {
+cudaError_t relu_grad(long n, const __nv_bfloat16* y, float* g, cudaStream_t) {
     return launch("relu_grad", {{y, size_t(n) * 2}, {g, size_t(n) * 4}});
-}
-cudaError_t to_bf16(long n, const float* g, __nv_bfloat16* g16, cudaStream_t) {
-    return launch("to_bf16", {{g, size_t(n) * 4}, {g16, size_t(n) * 2}});
 }
 cudaError_t pool_fwd(int B, int H, int W, int C, const __nv_bfloat16* in, __nv_bfloat16* out, cudaStream_t) {
     const size_t n = size_t(B) * H * W * C * 2;

@@ -384,3 +384,17 @@ def test_which_batches_stream(fake, scenes, streams):
     b = pt.Batch(items, ONE_LAUNCH, max_bounces=scenes[0][3])
     assert one_launch_lines(fake, b) == ["batch stream" if streams else "batch 128"]
     b.close()
+
+
+def test_gradients_that_the_tensor_cores_refuse_run_on_the_cuda_cores(fake):
+    from photon_tracer_b200 import abi
+    net = C.c_void_p()
+    abi.check(fake.lib.pt_unet_create(1, C.byref(net)))
+    fake.log()
+    fake.lib.fake_tensor_cores(0)
+    assert grads(fake, net, 1, 32, 48) == abi.PT_OK
+    fake.lib.fake_tensor_cores(1)
+    lines = fake.log()
+    fake.lib.pt_unet_destroy(net)
+    assert lines.count("wgrad") == 15 and lines.count("relu_grad") == 14
+    assert not [x for x in lines if x.startswith("bad") or x.endswith("tc")]
