@@ -284,9 +284,9 @@ pt_status pt_render(pt_scene* scene, const pt_camera* cam, const pt_settings* se
  * with the scene's other renders of those kinds by the caller. A frame of
  * several samples per pixel renders through a buffer of its samples (12 bytes
  * each, 36 with aux, at most 256 MB at a time or one sample per pixel), taken
- * from a memory pool of the device and given back in stream order; the pool
- * keeps up to 512 MB for later renders of any scene and goes with the device's
- * last scene. Without memory for the buffer, and under stream capture, frames
+ * from a pool of the device and given back in stream order. The pool keeps what
+ * the renders in flight at one time needed, at most 1.25 GB, for later renders
+ * of any scene, and frees it with the device's last scene. Without memory for the buffer, and under stream capture, frames
  * render without it, the same image more slowly. */
 pt_status pt_render_device(pt_scene* scene, const pt_camera* cam, const pt_settings* settings, float* d_out,
                            float* d_aux, uint64_t* d_rays, void* stream);

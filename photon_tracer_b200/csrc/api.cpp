@@ -74,7 +74,7 @@ struct pt_scene {
     int counters = 1;
     unsigned long long* rays = nullptr;
     cudaStream_t stream = nullptr;
-    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum;
+    Scratch out, aux, states, in_rays, out_hits, counts, wave, sum, small_samples;
     uint32_t* host_counts = nullptr;  // pinned, for the wavefront queue read-back
     int blocks_per_sm[2][6] = {};     // megakernel forms: lock-step, streaming; aux, snapshot, extended light sampling
     uint32_t wave_slots = 0;                   // wavefront path-queue capacity; 0: kMaxWaveSlots
@@ -188,14 +188,23 @@ int samples_per_launch(const PtRenderParams& p) {
 // borrowed from the device's pool for as long as its launches need it.
 constexpr size_t kCounterBytes = 256;
 
+// The scene's own stream is that of the host calls, which wait for their work:
+// their small renders (a scanline, a thumbnail) share a buffer that the scene
+// keeps: the pool's first block would cost a new scene's first scanline 350 us,
+// a buffer of its few KB 30.
+constexpr size_t kSmallSamples = size_t(1) << 20;
+
 struct RenderMemory {
-    void* ptr = nullptr;
+    int device = 0;
+    PoolBlock* block = nullptr;
     cudaStream_t stream = nullptr;
-    bool borrow(pt_scene* s, size_t bytes, cudaStream_t st) {  // false without memory for it
+    void* borrow(pt_scene* s, size_t bytes, cudaStream_t st) {  // null without memory for it
+        device = s->device;
         stream = st;
-        return pool_borrow(s->device, &ptr, bytes, st) == cudaSuccess;
+        block = pool_borrow(device, bytes, st);
+        return block ? block->ptr : nullptr;
     }
-    ~RenderMemory() { pool_return(ptr, stream); }
+    ~RenderMemory() { pool_return(device, block, stream); }
 };
 
 // The work counter of the scene's lock-step renders on a stream: renders in
@@ -242,18 +251,25 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
     RenderMemory memory;
     int count = 0;
     const bool captured = is_capturing(stream);
-    if (!captured) {
-        count = streams(s, p) ? samples_per_launch(p) : 0;
-        if (count > 0 && !memory.borrow(s, kCounterBytes + pt_sample_bytes(p) * size_t(count), stream)) count = 0;
+    void* samples = nullptr;  // and their counter in front
+    if (!captured && streams(s, p)) {
+        count = samples_per_launch(p);
+        const size_t bytes = kCounterBytes + pt_sample_bytes(p) * size_t(count);
+        if (count > 0 && stream == s->stream && bytes <= kSmallSamples) {
+            if (s->small_samples.ensure(bytes, "samples") == PT_OK) samples = s->small_samples.ptr;
+            else clear_error();
+        }
+        if (count > 0 && !samples) samples = memory.borrow(s, bytes, stream);
+        if (!samples) count = 0;
     }
     const int variant = p.nee_ext ? 4 + (p.aux ? 1 : 0) : (p.aux ? 1 : 0) + (p.rng_mode == PT_RNG_SNAPSHOT ? 2 : 0);
     if (count > 0) {
-        p.work = static_cast<unsigned int*>(memory.ptr);
-        float* samples = reinterpret_cast<float*>(static_cast<char*>(memory.ptr) + kCounterBytes);
+        p.work = static_cast<unsigned int*>(samples);
+        float* buffer = reinterpret_cast<float*>(static_cast<char*>(samples) + kCounterBytes);
         for (int first = 0; first < p.spp; first += count) {
             cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream);
             if (!e)
-                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first), samples, s->sms,
+                e = pt_launch_samples(s->dev, p, first, std::min(count, p.spp - first), buffer, s->sms,
                                       s->blocks_per_sm[1][variant], stream);
             if (e) return cuda_fail(e, "megakernel launch");
         }
@@ -262,8 +278,8 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
     p.work = s->work;
     if (!captured) {
         p.work = counter_of(s, stream);
-        if (!p.work)
-            p.work = memory.borrow(s, kCounterBytes, stream) ? static_cast<unsigned int*>(memory.ptr) : s->work;
+        if (!p.work) p.work = static_cast<unsigned int*>(memory.borrow(s, kCounterBytes, stream));
+        if (!p.work) p.work = s->work;
     }
     if (cudaError_t e = cudaMemsetAsync(p.work, 0, sizeof(unsigned int), stream)) return cuda_fail(e, "render");
     PtLaunchShape shape;
@@ -521,6 +537,7 @@ pt_status pt_scene_destroy(pt_scene* s) {
     s->out_hits.release();
     s->counts.release();
     s->wave.release();
+    s->small_samples.release();
     if (s->host_counts) cudaFreeHost(s->host_counts);
     if (s->stream) cudaStreamDestroy(s->stream);
     if (s->arena) cudaFree(s->arena);

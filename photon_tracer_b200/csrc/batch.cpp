@@ -30,7 +30,6 @@
 
 #include "batch.h"
 #include "kernels.h"
-#include "pool.h"
 #include "scene_host.hpp"
 
 namespace pt {
@@ -58,8 +57,8 @@ struct pt_batch {
     uint32_t total_items = 0;
     uint64_t total_pixels = 0, total_samples = 0, total_tris = 0;
     // Streaming form of the single launch: its launches' segments, and the
-    // buffer of samples with the segments behind it, borrowed from the device's
-    // pool for as long as the batch may run that launch.
+    // buffer of samples with the segments behind it, for as long as the batch may
+    // run that launch.
     struct Launch {
         uint32_t first, n, items, pixels;
     };
@@ -311,7 +310,8 @@ pt_status make_stream(pt_batch* b) {
     const size_t segment_bytes = b->segments.size() * sizeof(PtBatchSegment);
     const size_t at = align256(b->sample_bytes);
     void* memory = nullptr;
-    if (b->sample_bytes > 4 * 12 * kBatchSamples || pool_borrow(b->device, &memory, at + segment_bytes, b->stream)) {
+    if (b->sample_bytes > 4 * 12 * kBatchSamples || cudaMalloc(&memory, at + segment_bytes) != cudaSuccess) {
+        cudaGetLastError();
         b->launches.clear();
         return PT_OK;
     }
@@ -330,7 +330,7 @@ void drop_stream(pt_batch* b) {
         if (g) cudaGraphExecDestroy(g);
         g = nullptr;
     }
-    pool_return(b->d_samples, b->stream);
+    if (b->d_samples) cudaFree(b->d_samples);
     b->d_samples = nullptr;
     b->launches.clear();
     b->arena_bytes -= b->stream_bytes;
@@ -478,7 +478,6 @@ pt_status pt_batch_create(const pt_batch_item* items, uint32_t n, int32_t strate
     b->device = device;
     b->sms = sms;
     b->strategy = strategy;
-    pool_join(device);
     HostArena all;
     uint64_t out_floats = 0;
     uint32_t items_total = 0;
@@ -743,7 +742,6 @@ pt_status pt_batch_destroy(pt_batch* b) {
     if (b->done_event) cudaEventDestroy(b->done_event);
     if (b->stream) cudaStreamDestroy(b->stream);
     if (b->arena) cudaFree(b->arena);
-    pool_leave(b->device);
     delete b;
     return PT_OK;
 }

@@ -6,13 +6,22 @@
 
 namespace pt {
 
-// A scene or batch joins its device's pool when it is made and leaves it when
-// it is destroyed; the pool goes with the last one.
+// A scene joins its device's pool when it is made and leaves it when it is
+// destroyed, with none of its work in flight; the pool's memory goes with the
+// last one.
 void pool_join(int device);
 void pool_leave(int device);
-// Device memory from the stream's next work on, until pool_return in the
-// stream's order. Returns an error, and sets no error state, when there is none.
-cudaError_t pool_borrow(int device, void** ptr, size_t bytes, cudaStream_t stream);
-void pool_return(void* ptr, cudaStream_t stream);
+
+// Device memory for the stream's work from pool_borrow to pool_return, both of
+// which return at once. Null, with no error state set, when there is none.
+struct PoolBlock {
+    void* ptr = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t used = nullptr;     // the end of its last borrower's work
+    unsigned long long stream = 0;  // and the id of the stream of that work
+    bool lent = false;
+};
+PoolBlock* pool_borrow(int device, size_t bytes, cudaStream_t stream);
+void pool_return(int device, PoolBlock* block, cudaStream_t stream);
 
 }  // namespace pt

@@ -27,7 +27,8 @@ size_t g_fail_above = ~size_t(0), g_budget = ~size_t(0);
 bool g_falling_times = false;
 cudaStream_t g_capturing = nullptr;
 bool g_tensor_cores = true;
-long g_next = 0;
+long g_next = 0, g_finished = 0;
+std::map<cudaEvent_t, long> g_recorded;
 
 void log(const std::string& line) { g_log += line + "\n"; }
 std::string hex(const void* p) {
@@ -68,16 +69,13 @@ cudaError_t launch(const std::string& what, std::initializer_list<Use> uses) {
 
 }  // namespace
 
-struct CUmemPoolHandle_st {
-    int device;
-};
-
 extern "C" {
 
 // ---- the test's side ----
 void fake_clear() { g_log.clear(); }
 const char* fake_log() { return g_log.c_str(); }
 void fake_fail_after(long n) { g_fail_after = n; }
+void fake_finish() { ++g_finished; }  // all work so far is done
 void fake_fail_above(size_t bytes) { g_fail_above = bytes; }
 void fake_budget(size_t bytes) { g_budget = bytes; }
 void fake_falling_times(int on) { g_falling_times = on != 0; }
@@ -101,7 +99,7 @@ cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) { return s
 const char* cudaGetErrorString(cudaError_t) { return "a fake's error"; }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return log("wait device"), cudaSuccess; }
-cudaError_t cudaMalloc(void** p, size_t n) { return log("malloc"), allocate(p, n); }
+cudaError_t cudaMalloc(void** p, size_t n) { return log("malloc " + std::to_string(n)), allocate(p, n); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return *p = std::malloc(n), cudaSuccess; }
 cudaError_t cudaFreeHost(void* p) { return std::free(p), cudaSuccess; }
 cudaError_t cudaFree(void* p) {
@@ -110,20 +108,6 @@ cudaError_t cudaFree(void* p) {
     g_live.erase(static_cast<const char*>(p));
     std::free(p);
     return cudaSuccess;
-}
-cudaError_t cudaMemPoolCreate(cudaMemPool_t* pool, const cudaMemPoolProps*) {
-    return *pool = new CUmemPoolHandle_st{0}, log("pool create"), cudaSuccess;
-}
-cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, cudaMemPoolAttr, void* v) {
-    return log("pool keeps " + std::to_string(*static_cast<unsigned long long*>(v))), cudaSuccess;
-}
-cudaError_t cudaMemPoolDestroy(cudaMemPool_t pool) { return delete pool, log("pool destroy"), cudaSuccess; }
-cudaError_t cudaMallocFromPoolAsync(void** p, size_t n, cudaMemPool_t, cudaStream_t st) {
-    return log("borrow " + std::to_string(n) + " " + hex(st)), allocate(p, n);
-}
-cudaError_t cudaFreeAsync(void* p, cudaStream_t st) {  // its address is not used again: its stream may still be using it
-    g_live.erase(static_cast<const char*>(p));
-    return log("return " + hex(p) + " " + hex(st)), cudaSuccess;
 }
 cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { return std::memcpy(d, s, n), cudaSuccess; }
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
@@ -158,10 +142,20 @@ cudaError_t cudaGraphInstantiate(cudaGraphExec_t* e, cudaGraph_t, unsigned long 
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return log("graph destroy"), cudaSuccess; }
 cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return log("graph launch"), cudaSuccess; }
-cudaError_t cudaEventCreate(cudaEvent_t* e) { return *e = reinterpret_cast<cudaEvent_t>(1), cudaSuccess; }
+cudaError_t cudaEventCreate(cudaEvent_t* e) {
+    return *e = reinterpret_cast<cudaEvent_t>(0x100000 + 16 * ++g_next), cudaSuccess;
+}
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
-cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaEventDestroy(cudaEvent_t e) { return g_recorded.erase(e), cudaSuccess; }
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return g_recorded[e] = g_finished, cudaSuccess; }
+cudaError_t cudaEventQuery(cudaEvent_t e) {  // pending until the test lets the device finish
+    const auto it = g_recorded.find(e);
+    return it != g_recorded.end() && it->second == g_finished ? cudaErrorNotReady : cudaSuccess;
+}
+cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t, unsigned) {
+    return log("stream waits " + hex(s)), cudaSuccess;
+}
+cudaError_t cudaPeekAtLastError() { return cudaErrorNotReady; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
     *ms = g_falling_times ? 1.0f / float(++g_next) : 1.0f;

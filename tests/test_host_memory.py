@@ -104,30 +104,53 @@ def test_renders_on_two_streams_share_nothing(fake, kind, param, spp, form):
 
 
 def test_a_device_render_does_not_wait(fake):
-    """Neither the first frame nor larger ones after it, nor guides, allocate or free in a way that waits for the
-    device; what a frame borrows it gives back on its own stream after its last launch."""
+    """Neither the first frame nor larger ones after it, nor guides, free memory or wait for the device; a frame that
+    an earlier one's memory is large enough for allocates none."""
     d = DeviceScene(ROOM, 4)
     fake.log()
-    for w, h, spp, aux in ((64, 48, 4, False), (640, 360, 8, False), (1024, 1024, 24, True), (33, 17, 2, False)):
+    new = []
+    for w, h, spp, aux in ((64, 48, 4, False), (640, 360, 8, False), (1024, 1024, 24, True), (33, 17, 2, False),
+                           (1024, 1024, 24, True), (640, 360, 8, True)):
         d.render(w, h, spp, 0x7000, aux)
         lines = fake.log()
-        assert not [x for x in lines if x.split()[0] in ("malloc", "free", "wait", "bad")], lines
-        assert [x.split()[0] for x in lines if x.split()[0] in ("borrow", "return")] == ["borrow", "return"]
-        assert lines[-1].startswith("return") and lines[-1].endswith(" 0x7000")
+        assert not [x for x in lines if x.split()[0] in ("free", "wait", "stream", "bad")], lines
+        new.append(sum(x.startswith("malloc") for x in lines))
+    assert new == [1, 1, 1, 0, 0, 0]
 
 
 def test_scenes_hold_no_samples_between_renders(fake):
-    """Many scenes' renders leave only what the device's pool keeps, which is bounded and goes with the last scene."""
-    scenes = [DeviceScene(ROOM, 3) for _ in range(3)]
+    """Scenes that render one after another do so in the same memory, whichever streams they use once the work is
+    done, and the last of them frees it."""
+    before = fake.live_bytes()
+    scenes = [DeviceScene(ROOM, 3) for _ in range(4)]
     fake.log()
-    for d in scenes:
-        d.render(640, 360, 8, 0x7000)
-    lines = fake.log()
-    assert [x for x in lines if x.startswith("pool")] == ["pool create", f"pool keeps {512 << 20}"]
-    assert sum(x.startswith("borrow") for x in lines) == sum(x.startswith("return") for x in lines) == 3
     for k, d in enumerate(scenes):
+        if k == 3:
+            fake.lib.fake_finish()
+        d.render(640, 360, 8, 0x8000 if k == 3 else 0x7000)
+    lines = fake.log()
+    assert sum(x.startswith("malloc") for x in lines) == 1
+    for d in scenes:
+        assert fake.live_bytes() > before
         d.s.close()
-        assert ("pool destroy" in fake.log()) == (k == 2)
+    assert fake.live_bytes() == before
+
+
+def test_memory_of_frames_in_flight_is_bounded(fake):
+    """Large frames on many streams get memory of their own up to a bound; then a stream waits for another's, in
+    stream order, and no frame goes without."""
+    d = DeviceScene(ROOM, 3)
+    before = fake.live_bytes()
+    fake.log()
+    streams = [0x7000 + 16 * k for k in range(10)]
+    for stream in streams:
+        d.render(1024, 1024, 22, stream)
+    lines = fake.log()
+    assert len(launches(lines, "samples")) >= 10 and not launches(lines, "megakernel")
+    assert fake.live_bytes() - before <= 1280 << 20
+    waits = [x.split()[2] for x in lines if x.startswith("stream waits")]
+    assert waits and set(int(w, 16) for w in waits) <= set(streams[4:])
+    assert len({buffer for _, _, buffer in launches(lines, "samples")}) == 10 - len(waits)
 
 
 def test_captured_and_memoryless_renders_borrow_no_samples(fake):
@@ -137,7 +160,7 @@ def test_captured_and_memoryless_renders_borrow_no_samples(fake):
     d.render(400, 300, 4, 0x7000)
     fake.lib.fake_capture(None)
     lines = fake.log()
-    assert len(launches(lines, "megakernel")) == 1 and not any(x.startswith("borrow") for x in lines)
+    assert len(launches(lines, "megakernel")) == 1 and not any(x.startswith("malloc") for x in lines)
     with fake.failing_above(1 << 20):
         d.render(400, 300, 4, 0x7000)
     with fake.failing_above(0):
@@ -327,26 +350,26 @@ def test_which_frames_stream(fake, scene, streams, not_streams):
 
 def test_lock_step_renders_borrow_nothing_on_their_usual_streams(fake):
     """A stream's lock-step renders count in that stream's own word, captured ones in another; with more streams than
-    words, and no memory to borrow, the render still runs."""
+    words, or no memory to borrow, the render still runs."""
     d = DeviceScene(SPHERES, 20)
     fake.log()
-    counters = {}
-    for stream in [0x7000 + 16 * k for k in range(40)] * 2:
-        d.render(100, 60, 1, stream)
-        lines = fake.log()
-        (got,) = launches(lines, "megakernel")
-        borrowed = any(x.startswith("borrow") for x in lines)
-        if not borrowed:
-            assert counters.setdefault(stream, got[1]) == got[1]
-        assert borrowed == (stream not in counters)
+    work, streams = [{}, {}], [0x7000 + 16 * k for k in range(40)]
+    for seen in work:
+        for stream in streams:
+            d.render(100, 60, 1, stream)
+            lines = fake.log()
+            ((_, seen[stream], _),) = launches(lines, "megakernel")
+            assert ("malloc 1048576" in lines) == (stream >= streams[31] and seen is work[0])
+    assert work[0] == work[1] and len(set(work[0].values())) == 40
     fake.lib.fake_capture(0x7000)
     d.render(100, 60, 1, 0x7000)
     fake.lib.fake_capture(None)
     (captured,) = launches(fake.log(), "megakernel")
-    assert len(counters) == len(set(counters.values())) == 31 and captured[1] not in counters.values()
+    assert captured[1] not in work[0].values()
     with fake.failing_above(0):
         d.render(100, 60, 1, 0x9000)
-    assert not any(x.startswith("bad") for x in fake.log())
+    lines = fake.log()
+    assert launches(lines, "megakernel") and not any(x.startswith("bad") for x in lines)
 
 
 @pytest.mark.parametrize("scene,closest,any_hit", [
@@ -398,3 +421,24 @@ def test_gradients_that_the_tensor_cores_refuse_run_on_the_cuda_cores(fake):
     fake.lib.pt_unet_destroy(net)
     assert lines.count("wgrad") == 15 and lines.count("relu_grad") == 14
     assert not [x for x in lines if x.startswith("bad") or x.endswith("tc")]
+
+
+def test_small_host_renders_keep_a_buffer_of_their_scene(fake):
+    """A scanline's samples go through the scene's own buffer, which grows and goes with the scene; larger host frames
+    take the pool's memory, as every frame on a caller's stream does."""
+    import numpy as np
+    import photon_tracer_b200 as pt
+    before = fake.live_bytes()
+    d = DeviceScene(SPHERES, 20)
+    fake.log()
+    for width, spp in ((400, 16), (1920, 40), (64, 4)):
+        pt.render_row_linear(d.s, d.g.camera, 3, width, 200, spp, 10, np.empty((width, 3), np.float32), 1)
+        lines = fake.log()
+        assert len(launches(lines, "samples")) == 1 and not any(x.startswith("bad") for x in lines)
+        assert f"malloc {256 + 12 * width * spp}" in lines or width == 64
+    d.s.render(d.g.camera, 300, 200, 16)
+    assert f"malloc {16 << 20}" in fake.log()
+    d.render(64, 48, 4, 0x7000)
+    assert f"malloc {1 << 20}" in fake.log()
+    d.s.close()
+    assert fake.live_bytes() == before
