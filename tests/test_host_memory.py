@@ -442,3 +442,19 @@ def test_small_host_renders_keep_a_buffer_of_their_scene(fake):
     assert f"malloc {1 << 20}" in fake.log()
     d.s.close()
     assert fake.live_bytes() == before
+
+
+def test_gpu_comparisons_of_the_two_forms_have_both(fake):
+    """Every frame that the GPU tests compare between the streaming form and a capture's lock-step form streams when it
+    is not captured."""
+    import test_gpu_stream
+    import test_gpu_stream_forms
+    import photon_tracer_b200 as pt
+    (cases,) = [m.args[1] for m in test_gpu_stream.test_frames_equal_lock_step.pytestmark if m.name == "parametrize"]
+    for kind, param, width, height, spp, depth, aux, flags, snapshot in cases + test_gpu_stream_forms.FORMS:
+        g = pt.Generated(kind, seed=3, param=param)
+        s = pt.Scene(g)
+        st = s.settings(width, height, spp, depth, seed=9, flags=flags, rng=int(snapshot), states_ptr=64)
+        fake.log()
+        s.render_device(g.camera, st, SOME.value, SOME.value if aux else 0, 0, 0x7000)
+        assert launches(fake.log(), "samples"), (kind, param, width, height, spp)
