@@ -192,7 +192,7 @@ constexpr size_t kCounterBytes = 256;
 // their small renders (a scanline, a thumbnail) share a buffer that the scene
 // keeps: the pool's first block would cost a new scene's first scanline 350 us,
 // a buffer of its few KB 30.
-constexpr size_t kSmallSamples = size_t(1) << 20;
+constexpr size_t kSmallSamples = size_t(4) << 20;
 
 struct RenderMemory {
     int device = 0;
@@ -316,8 +316,12 @@ bool pt::stream_gains(uint32_t kib, bool sky, int spp, int depth, uint64_t pixel
     // room, 640x360, 8 samples, depth 1 163, 188; depth 2 736, 955; at 400x225, 4
     // samples 162, 195; the room of 81,920 triangles 0.54 and 0.74 of the time at
     // 640x360, 8 samples, but 1.33 at 1920x1080, 4, depth 1, and 1.06 at 320x180, 3.
-    if (depth <= (sky && kib <= 40 ? 3 : 2))
-        return spp > 3 && (pixels <= (kib > 64 ? lanes : lanes / 2) || (kib > 1024 && pixels <= 4 * lanes));
+    // Camera rays alone do in smaller scenes too (1,280 triangles, 640x360, 8
+    // samples 0.73, 2 samples 1.12; with a bounce 1.09).
+    if (depth <= (sky && kib <= 40 ? 3 : 2)) {
+        if (pixels <= (kib > 64 ? lanes : lanes / 2)) return spp > 3;
+        return pixels <= 4 * lanes && ((kib > 1024 && spp > 3) || (kib > 64 && depth == 1 && spp >= 8));
+    }
     // Small open scenes whose pixels fill the lanes several times over: 24
     // spheres, 1280x720, 8 samples 12% slower, the reference's field 4% (1920x1080:
     // 9%); 488 spheres 6% faster, with guides 2% slower at 1920x1080.

@@ -331,8 +331,8 @@ SPHERES_24, SPHERES_488, FIELD, REF_ROOM, ROOM_1K, ROOM_80K, INSTANCES = (
     (REF_ROOM, [(1920, 1080, 4, 3, 0), (640, 360, 4, 10, 1)], [(640, 360, 8, 1, 0), (640, 360, 8, 2, 1),
                                                             (1920, 1080, 4, 2, 0), (640, 360, 3, 10, 0),
                                                             (400, 225, 4, 2, 0)]),
-    (ROOM_1K, [(640, 360, 2, 10, 0), (256, 256, 16, 1, 0), (1920, 1080, 1, 10, 0)],
-     [(640, 360, 8, 2, 0), (1920, 1080, 4, 1, 0), (640, 360, 1, 10, 0)]),
+    (ROOM_1K, [(640, 360, 2, 10, 0), (256, 256, 16, 1, 0), (1920, 1080, 1, 10, 0), (640, 360, 8, 1, 0)],
+     [(640, 360, 8, 2, 0), (640, 360, 2, 1, 0), (1920, 1080, 4, 1, 0), (640, 360, 1, 10, 0)]),
     (ROOM_80K, [(1024, 1024, 64, 10, 0), (640, 360, 8, 1, 0), (640, 360, 8, 2, 0)],
      [(1920, 1080, 4, 1, 1), (1920, 1080, 4, 2, 0), (320, 180, 3, 2, 0)]),
     (INSTANCES, [(960, 540, 16, 10, 0), (640, 360, 2, 10, 0)], [(1920, 1080, 4, 1, 0)]),
@@ -436,8 +436,8 @@ def test_small_host_renders_keep_a_buffer_of_their_scene(fake):
         lines = fake.log()
         assert len(launches(lines, "samples")) == 1 and not any(x.startswith("bad") for x in lines)
         assert f"malloc {256 + 12 * width * spp}" in lines or width == 64
-    d.s.render(d.g.camera, 300, 200, 16)
-    assert f"malloc {16 << 20}" in fake.log()
+    d.s.render(d.g.camera, 400, 225, 16)
+    assert f"malloc {32 << 20}" in fake.log()
     d.render(64, 48, 4, 0x7000)
     assert f"malloc {1 << 20}" in fake.log()
     d.s.close()
