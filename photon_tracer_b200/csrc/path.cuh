@@ -239,7 +239,7 @@ __device__ __forceinline__ int shade(const PtSceneDev& S, Path& p, bool hit, con
                                      unsigned long long& rays) {
     // CODE_SMALL's normalized incoming direction is what the sky, metal and glass
     // need. In the extended light sampling's streaming kernel it and the single
-    // draws took 640x360, 16 samples from 8.6 to 7.1 ms; without that sampling
+    // draws took 640x360, 16 samples from 8.5 to 7.1 ms; without that sampling
     // they only cost registers: room frame +9%.
     constexpr bool SMALL = CODE == CODE_SMALL;
     nee = false;
