@@ -23,7 +23,8 @@ def build_fake(out_dir):
     with cf.ThreadPoolExecutor(8) as ex:
         list(ex.map(lambda so: run(["g++"] + flags + ["-c", so[0], "-o", so[1]]), zip(sources, objects)))
     path = os.path.join(out_dir, "libfake.so")
-    run(["g++", "-shared", "-o", path] + objects + ["-lpthread"])
+    # its own runtime, also where a process has the real one loaded
+    run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", path] + objects + ["-lpthread"])
     return path
 
 
