@@ -31,6 +31,7 @@ pt_status fail(pt_status code, const std::string& msg) {
 const char* error_text() { return g_error.c_str(); }
 
 pt_status cuda_fail(cudaError_t e, const char* what) {
+    cudaGetLastError();  // reported now, not by the next call's launch check
     return fail(e == cudaErrorMemoryAllocation ? PT_ERR_OUT_OF_MEMORY : PT_ERR_CUDA,
                 std::string(what) + ": " + cudaGetErrorString(e));
 }
@@ -195,16 +196,14 @@ constexpr size_t kCounterBytes = 256;
 constexpr size_t kSmallSamples = size_t(4) << 20;
 
 struct RenderMemory {
-    int device = 0;
     PoolBlock* block = nullptr;
     cudaStream_t stream = nullptr;
     void* borrow(pt_scene* s, size_t bytes, cudaStream_t st) {  // null without memory for it
-        device = s->device;
         stream = st;
-        block = pool_borrow(device, bytes, st);
+        block = pool_borrow(s->device, bytes, st);
         return block ? block->ptr : nullptr;
     }
-    ~RenderMemory() { pool_return(device, block, stream); }
+    ~RenderMemory() { pool_return(block, stream); }
 };
 
 // The work counter of the scene's lock-step renders on a stream: renders in
@@ -256,6 +255,7 @@ pt_status launch_render(pt_scene* s, PtRenderParams& p, int mode, cudaStream_t s
         count = samples_per_launch(p);
         const size_t bytes = kCounterBytes + pt_sample_bytes(p) * size_t(count);
         if (count > 0 && stream == s->stream && bytes <= kSmallSamples) {
+            RelaxedCapture relaxed;
             if (s->small_samples.ensure(bytes, "samples") == PT_OK) samples = s->small_samples.ptr;
             else clear_error();
         }

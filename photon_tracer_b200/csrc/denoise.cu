@@ -297,6 +297,7 @@ void run_atrous(int w, int h, const float* color, const float* albedo, const flo
 
 pt_status cuda_status(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return PT_OK;
+    cudaGetLastError();  // reported now, not by the next call's launch check
     return pt::fail(e == cudaErrorMemoryAllocation ? PT_ERR_OUT_OF_MEMORY : PT_ERR_CUDA,
                     std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -42,13 +42,6 @@ size_t block_size(size_t bytes) {
     return b;
 }
 
-// The pool's own calls must not disturb a capture on another stream.
-struct Relaxed {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
-
 void clear_last_error() { cudaGetLastError(); }
 
 PoolBlock* new_block(DevicePool& d, size_t bytes) {
@@ -88,7 +81,7 @@ void pool_leave(int device) {
 }
 
 PoolBlock* pool_borrow(int device, size_t bytes, cudaStream_t stream) {
-    Relaxed relaxed;
+    RelaxedCapture relaxed;
     std::lock_guard<std::mutex> lock(g_lock);
     DevicePool& d = g_pools[device];
     unsigned long long id = 0;
@@ -121,9 +114,9 @@ PoolBlock* pool_borrow(int device, size_t bytes, cudaStream_t stream) {
     return best;
 }
 
-void pool_return(int device, PoolBlock* block, cudaStream_t stream) {
+void pool_return(PoolBlock* block, cudaStream_t stream) {
     if (!block) return;
-    Relaxed relaxed;
+    RelaxedCapture relaxed;
     std::lock_guard<std::mutex> lock(g_lock);
     block->stream = 0;
     if (cudaStreamGetId(stream, &block->stream) != cudaSuccess || cudaEventRecord(block->used, stream) != cudaSuccess) {

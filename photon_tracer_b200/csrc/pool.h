@@ -22,6 +22,14 @@ struct PoolBlock {
     bool lent = false;
 };
 PoolBlock* pool_borrow(int device, size_t bytes, cudaStream_t stream);
-void pool_return(int device, PoolBlock* block, cudaStream_t stream);
+void pool_return(PoolBlock* block, cudaStream_t stream);
+
+// Allocations and event queries while this lives do not disturb a capture on
+// another stream.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 
 }  // namespace pt

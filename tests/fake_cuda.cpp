@@ -11,6 +11,7 @@
 #include <initializer_list>
 #include <map>
 #include <string>
+#include <utility>
 
 #include "../include/photon_cuda.h"
 #include "../photon_tracer_b200/csrc/batch.h"
@@ -28,6 +29,7 @@ bool g_falling_times = false;
 cudaStream_t g_capturing = nullptr;
 bool g_tensor_cores = true;
 long g_next = 0, g_finished = 0;
+cudaError_t g_last = cudaSuccess;  // what cudaGetLastError has not been asked for yet
 std::map<cudaEvent_t, long> g_recorded;
 
 void log(const std::string& line) { g_log += line + "\n"; }
@@ -40,7 +42,8 @@ cudaError_t allocate(void** p, size_t bytes) {
     *p = nullptr;
     size_t used = 0;
     for (const auto& a : g_live) used += a.second;
-    if (g_fail_after == 0 || bytes > g_fail_above || used + bytes > g_budget) return cudaErrorMemoryAllocation;
+    if (g_fail_after == 0 || bytes > g_fail_above || used + bytes > g_budget)
+        return g_last = cudaErrorMemoryAllocation;
     if (g_fail_after > 0) --g_fail_after;
     *p = std::malloc(bytes ? bytes : 1);
     g_live[static_cast<const char*>(*p)] = bytes;
@@ -57,7 +60,9 @@ struct Use {
     const void* p;
     size_t bytes;
 };
+// Reports, as the library's launches do, whatever error is pending.
 cudaError_t launch(const std::string& what, std::initializer_list<Use> uses) {
+    if (g_last != cudaSuccess) return std::exchange(g_last, cudaSuccess);
     for (const Use& u : uses)
         if (u.bytes && !live(u.p, u.bytes)) {
             log("bad " + what);
@@ -97,7 +102,7 @@ cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
 }
 cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void*) { return std::memset(a, 0, sizeof *a), cudaSuccess; }
 const char* cudaGetErrorString(cudaError_t) { return "a fake's error"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return std::exchange(g_last, cudaSuccess); }
 cudaError_t cudaDeviceSynchronize() { return log("wait device"), cudaSuccess; }
 cudaError_t cudaMalloc(void** p, size_t n) { return log("malloc " + std::to_string(n)), allocate(p, n); }
 cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return *p = std::malloc(n), cudaSuccess; }
@@ -150,12 +155,12 @@ cudaError_t cudaEventDestroy(cudaEvent_t e) { return g_recorded.erase(e), cudaSu
 cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t) { return g_recorded[e] = g_finished, cudaSuccess; }
 cudaError_t cudaEventQuery(cudaEvent_t e) {  // pending until the test lets the device finish
     const auto it = g_recorded.find(e);
-    return it != g_recorded.end() && it->second == g_finished ? cudaErrorNotReady : cudaSuccess;
+    return it != g_recorded.end() && it->second == g_finished ? g_last = cudaErrorNotReady : cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t, unsigned) {
     return log("stream waits " + hex(s)), cudaSuccess;
 }
-cudaError_t cudaPeekAtLastError() { return cudaErrorNotReady; }
+cudaError_t cudaPeekAtLastError() { return g_last; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) {
     *ms = g_falling_times ? 1.0f / float(++g_next) : 1.0f;

@@ -154,6 +154,8 @@ def test_memory_of_frames_in_flight_is_bounded(fake):
 
 
 def test_captured_and_memoryless_renders_borrow_no_samples(fake):
+    import numpy as np
+    import photon_tracer_b200 as pt
     d = DeviceScene(ROOM, 4)
     fake.lib.fake_capture(0x7000)
     fake.log()
@@ -165,8 +167,11 @@ def test_captured_and_memoryless_renders_borrow_no_samples(fake):
         d.render(400, 300, 4, 0x7000)
     with fake.failing_above(0):
         d.render(400, 300, 4, 0x7000)
+    with fake.failing_above(3 * 4 * 400):  # a scanline's pixels, not its samples
+        row = np.empty((400, 3), np.float32)
+        pt.render_row_linear(d.s, d.g.camera, 3, 400, 300, 16, 10, row, 1)
     lines = fake.log()
-    assert len(launches(lines, "megakernel")) == 2 and not launches(lines, "samples")
+    assert len(launches(lines, "megakernel")) == 3 and not launches(lines, "samples")
     assert not any(x.startswith("bad") for x in lines)
 
 
